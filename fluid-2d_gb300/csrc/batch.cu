@@ -156,8 +156,7 @@ int build_plan(fs_batch* b, float diff, float visc, float dt) {
             for (int g : L.grids)
                 for (int q = 0; q < 3; ++q) {
                     StencilField f{};
-                    field_geometry(f, b->rows[g], b->cols[g], b->pitch[g], b->tile_rows, dplan[pass]);
-                    realign_columns(f);
+                    field_tiling(f, b->rows[g], b->cols[g], b->pitch[g], b->tile_rows, dplan[pass]);
                     field_diffusion(f, b->rows[g], b->cols[g], rates[q], dt);
                     f.s_lr = bnd_sign_lr(modes[q]);
                     f.s_tb = bnd_sign_tb(modes[q]);
@@ -185,9 +184,8 @@ int build_plan(fs_batch* b, float diff, float visc, float dt) {
                 std::vector<StencilField> fl;
                 for (int g : L.grids) {
                     StencilField f{};
-                    field_geometry(f, b->rows[g], b->cols[g], b->pitch[g], b->tile_rows,
+                    field_tiling(f, b->rows[g], b->cols[g], b->pitch[g], b->tile_rows,
                                    pplan[pass] + (last && !split ? 1 : 0));
-                    realign_columns(f);
                     const float h = grid_spacing(b->rows[g], b->cols[g]);
                     f.s_lr = f.s_tb = 1.f;
                     f.sweeps = pplan[pass];

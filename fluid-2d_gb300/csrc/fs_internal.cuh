@@ -29,8 +29,7 @@ enum PassKind : int {
     PASS_PRESSURE = 3,       // reads p, div
 };
 
-// Region width of the stencil kernels: 128 columns, one per thread of a CTA row in the
-// load and store phases, four per lane of a warp in the sweeps.
+// Region width of the stencil kernels: 128 columns, four per lane of a warp.
 constexpr int kRegionW = 128;
 
 struct StencilField {
@@ -47,7 +46,7 @@ struct StencilField {
     float* u_out;
     float* v_out;
     // constants
-    float a, dh, dl, rf;  // diffuse: a and the FP32 pair for 1/(1+4a) (see stencil.cu)
+    float a, rh, rl;      // diffuse: a and the FP32 pair for 1/(1+4a) (see stencil.cu)
     float dt;             // add_sources
     float cdiv;           // divergence factor -0.5f*h
     float h;              // gradient divisor
@@ -55,10 +54,11 @@ struct StencilField {
     int kind;             // PassKind
     int sweeps;           // Jacobi sweeps in this pass
     int epilogue;         // 1: gradient subtract + velocity fills after the sweeps
-    int halo;             // H: region = tile grown by H on each side
+    int halo;             // H: a region's margin around its output tile (field_tiling)
     int rows, cols, pitch;
-    int tile_w, tile_h, tiles_x, tiles_y, shift_x, shift_y;
-    int realign;          // 1: start each region on a multiple of four columns (see realign_columns)
+    int tile_w, tile_h, tiles_x, tiles_y;
+    int gx_last, gy_last; // first column and row of the last regions
+    int caller_rows;      // 1: u_out, v_out are a caller's buffers, their row padding is not written
     int tile_begin;       // first block index of this field in the launch
     int* nonfinite;       // optional flag (epilogue outputs)
 };
@@ -126,30 +126,26 @@ struct AdvectJob {
     int smooth;
 };
 
-// Tile geometry: tiles partition [0, n) starting at -shift, and never put a domain
-// edge cell (index 0 or n-1) in a different tile from its inner neighbour, so the
-// boundary fill of a tile only ever depends on cells of the same tile.
-inline void tile_split(int n, int tile, int* count, int* shift) {
-    int s = ((n - 1) % tile == 0) ? 1 : 0;
-    *shift = s;
-    *count = (n + s + tile - 1) / tile;
-}
-
-// Column tiling for passes whose interior tiles can take the stencil's direct path,
-// which loads and stores a region's rows 16 bytes at a time and so needs each region to
-// start on a multiple of four columns. With tile width 128 - 2H and halo H that holds
-// for every tile when the width is a multiple of four and H + shift is too. Otherwise
-// the width shrinks by three and the kernel moves each region's start down to the
-// multiple of four below it (by a = 0..3 columns): the left margin becomes H + a and the
-// right one H + 3 - a, both at least H.
-inline void realign_columns(StencilField& f) {
-    f.realign = 0;
-    const int w = kRegionW - 2 * f.halo;
-    if (w % 4 == 0 && (f.halo + f.shift_x) % 4 == 0) return;
-    if (w - 3 < 1) return;
-    f.tile_w = w - 3;
-    tile_split(f.cols, f.tile_w, &f.tiles_x, &f.shift_x);
-    f.realign = 1;
+// Tiling of a grid into regions of region_rows x 128 cells with a margin of at least
+// `halo` rows and `halo` rounded up to whole groups of four columns. Region t starts at
+// min(t * tile, last), the last region ends at the grid's last row (column group), and its
+// output runs from t * tile + margin (0 for the first) to the next region's (the grid's
+// end for the last). So every region lies inside a grid at least as large as it, region
+// columns and output columns start at multiples of four, and an edge cell's inner
+// neighbour is always in the same tile (the last tile keeps more than `halo` rows and
+// columns of the grid).
+inline void field_tiling(StencilField& f, int rows, int cols, int pitch, int region_rows, int halo) {
+    f.rows = rows;
+    f.cols = cols;
+    f.pitch = pitch;
+    f.halo = halo;
+    f.tile_w = kRegionW - 2 * ((halo + 3) / 4 * 4);
+    f.tile_h = region_rows - 2 * halo;
+    const int end = (cols + 3) / 4 * 4;  // the last column group's end
+    f.gx_last = end > kRegionW ? end - kRegionW : 0;
+    f.gy_last = rows > region_rows ? rows - region_rows : 0;
+    f.tiles_x = 1 + (f.gx_last + f.tile_w - 1) / f.tile_w;
+    f.tiles_y = 1 + (f.gy_last + f.tile_h - 1) / f.tile_h;
 }
 
 // Sets the calling thread's fs_last_error() message and returns code (solver.cu).

@@ -1,5 +1,4 @@
-// Host-side helpers shared by the single-grid and batched drivers: pass planning,
-// tile geometry, the reference's step constants, and CUDA error reporting.
+// Host-side helpers shared by the single-grid and batched drivers: pass planning, the reference's step constants, and CUDA error reporting.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -48,26 +47,14 @@ inline std::vector<int> plan_passes(int total, int k) {
     return out;
 }
 
-inline void field_geometry(StencilField& f, int rows, int cols, int pitch, int tile_rows, int halo) {
-    f.rows = rows;
-    f.cols = cols;
-    f.pitch = pitch;
-    f.halo = halo;
-    f.tile_w = kRegionW - 2 * halo;
-    f.tile_h = tile_rows - 2 * halo;
-    tile_split(cols, f.tile_w, &f.tiles_x, &f.shift_x);
-    tile_split(rows, f.tile_h, &f.tiles_y, &f.shift_y);
-}
-
-// a = dt * float(rows*cols) * rate (fluid_solver_gpu.cu:79) and the FP32 pair for
-// dividing by the reference's double divisor 1 + 4a.
+// a = dt * float(rows*cols) * rate (fluid_solver_gpu.cu:79) and the FP32 pair whose sum is
+// the reciprocal of the reference's double divisor 1 + 4a.
 inline void field_diffusion(StencilField& f, int rows, int cols, float rate, float dt) {
     const float a = dt * (float)((size_t)rows * (size_t)cols) * rate;
     const double D = 1.0 + 4.0 * (double)a;
     f.a = a;
-    f.dh = (float)D;
-    f.dl = (float)(D - (double)f.dh);
-    f.rf = (float)(1.0 / D);
+    f.rh = (float)(1.0 / D);
+    f.rl = (float)(1.0 / D - (double)f.rh);
 }
 
 // dt0 = sqrt(rows*cols)*dt evaluated in double (fluid_solver_gpu.cu:334).

@@ -119,15 +119,7 @@ extern "C" int fs_project_noalloc(const float* u, const float* v, float* u_out, 
         L.nfields = 1;
         StencilField& f = L.f[0];
         const int halo = plan[pass] + (last ? 1 : 0);
-        f.rows = rows;
-        f.cols = cols;
-        f.pitch = pitch;
-        f.halo = halo;
-        f.tile_w = kRegionW - 2 * halo;
-        f.tile_h = tile_rows - 2 * halo;
-        tile_split(cols, f.tile_w, &f.tiles_x, &f.shift_x);
-        tile_split(rows, f.tile_h, &f.tiles_y, &f.shift_y);
-        if (pass > 0 && !last) realign_columns(f);  // as for a handle's fixed-count projection
+        field_tiling(f, rows, cols, pitch, tile_rows, halo);
         f.s_lr = f.s_tb = 1.f;
         f.sweeps = plan[pass];
         f.cdiv = -0.5f * h;
@@ -146,6 +138,7 @@ extern "C" int fs_project_noalloc(const float* u, const float* v, float* u_out, 
         f.y = last ? nullptr : pbuf[pass & 1];
         if (last) {
             f.epilogue = 1;
+            f.caller_rows = 1;
             f.u_in = u;
             f.v_in = v;
             f.u_out = u_out;

@@ -32,6 +32,7 @@
 
 #include "../../include/fluid2d_gb300.h"
 #include "fs_internal.cuh"
+#include "host_common.h"
 
 #define FS_VERSION "0.1.0"
 
@@ -237,24 +238,7 @@ std::vector<int> split_sweeps(int total, int k) {
 }
 
 void set_geometry(StencilField& f, const fs_solver* s, int halo) {
-    f.rows = s->rows;
-    f.cols = s->cols;
-    f.pitch = s->pitch;
-    f.halo = halo;
-    f.tile_w = kRegionW - 2 * halo;
-    f.tile_h = s->tile_rows - 2 * halo;
-    tile_split(s->cols, f.tile_w, &f.tiles_x, &f.shift_x);
-    tile_split(s->rows, f.tile_h, &f.tiles_y, &f.shift_y);
-}
-
-void diffuse_constants(StencilField& f, int rows, int cols, float rate, float dt) {
-    // a = dt * T(rows*cols) * rate in float (fluid_solver_gpu.cu:79)
-    const float a = dt * (float)((size_t)rows * (size_t)cols) * rate;
-    const double D = 1.0 + 4.0 * (double)a;
-    f.a = a;
-    f.dh = (float)D;
-    f.dl = (float)(D - (double)f.dh);
-    f.rf = (float)(1.0 / D);
+    field_tiling(f, s->rows, s->cols, s->pitch, s->tile_rows, halo);
 }
 
 AdvectArgs advect_args(const fs_solver* s, float dt) {
@@ -334,8 +318,7 @@ int enqueue_diffuse(fs_solver* s, const int* fields, int nf, const float* rates,
             const int fid = fields[q];
             StencilField& f = L.f[q];
             set_geometry(f, s, plan[pass]);
-            realign_columns(f);
-            diffuse_constants(f, s->rows, s->cols, rates[q], dt);
+            field_diffusion(f, s->rows, s->cols, rates[q], dt);
             const int mode = fid == F_D ? BND_CONT : (fid == F_U ? BND_OPP_H : BND_OPP_V);
             f.s_lr = bnd_sign_lr(mode);
             f.s_tb = bnd_sign_tb(mode);
@@ -582,7 +565,6 @@ int enqueue_project_learned_cycles(fs_solver* s, const float* u_in, const float*
     CK(cudaMemsetAsync(s->ctrl + slot, 0, sizeof(SolveCtrl), s->stream));
     PressureSolve P{};
     set_geometry(P.mid, s, K + 1);
-    realign_columns(P.mid);  // interior tiles take the direct path (P.first copies the tiling)
     P.mid.s_lr = P.mid.s_tb = 1.f;
     P.mid.sweeps = K;
     P.mid.h = grid_h(s->rows, s->cols);
@@ -646,7 +628,6 @@ int enqueue_project_learned_defect(fs_solver* s, const float* u_in, const float*
     double* hsums = reinterpret_cast<double*>(s->host_ctrl + 1);
     PressureSolve P{};
     set_geometry(P.mid, s, K + 1);
-    realign_columns(P.mid);  // interior tiles take the direct path (P.first copies the tiling)
     P.mid.s_lr = P.mid.s_tb = 1.f;
     P.mid.sweeps = K;
     P.mid.h = grid_h(s->rows, s->cols);
@@ -726,7 +707,6 @@ int enqueue_project_to_residual(fs_solver* s, const float* u_in, const float* v_
     PressureSolve P{};
     for (StencilField* f : {&P.first, &P.mid}) {
         set_geometry(*f, s, K + 1);
-        realign_columns(*f);  // one tiling for both; the middle passes' interior tiles go direct
         f->s_lr = f->s_tb = 1.f;
         f->sweeps = K;
         f->cdiv = -0.5f * h;
@@ -789,7 +769,6 @@ int enqueue_project(fs_solver* s, const float* u_in, const float* v_in, float* u
         L.nfields = 1;
         StencilField& f = L.f[0];
         set_geometry(f, s, plan[pass] + (fused ? 1 : 0));
-        if (pass > 0) realign_columns(f);  // the first pass's tiling is aligned at depth 8
         f.s_lr = f.s_tb = 1.f;
         f.sweeps = plan[pass];
         f.cdiv = -0.5f * h;
