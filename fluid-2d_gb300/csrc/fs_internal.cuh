@@ -246,17 +246,24 @@ cudaError_t launch_advect_velocity(const float* u0, const float* v0, float* u, f
                                    cudaStream_t st);
 
 // Gauss-Seidel compatibility step (gs.cu): the host solver's method, bit for bit, on a
-// square n x n grid of pitched fields; four scratch fields of the same shape.
+// square n x n grid of pitched fields (d, u, v).
 struct GsFields {
-    float *d, *u, *v;
-    const float *ds, *us, *vs;
-    float* scratch[5];
-    float* aux;                 // two floats of device scratch
-    SolveCtrl* ctrl;            // grid-barrier state of the tiled solves (larger grids)
-    const unsigned* poll_limit; // device word: polls before a grid barrier gives up (0 = default)
+    float* state[3];
+    const float* src[3];
+    // scratch, each of a field's size; big[0..2] are two fields each and contiguous
+    float* big[3];
+    float* dif[3];
+    float* vel[2];
+    float* p;
+    int *head, *next;
+    void* words;
+    SolveCtrl* ctrl;            // error flag of the waits between SMs
+    const unsigned* poll_limit; // device word: polls before such a wait gives up (0 = default)
+    cudaStream_t side;          // the splat's stream, forked and joined by the events
+    cudaEvent_t fork, join;
 };
-int gs_max_size();                 // largest n of the one-CTA form on the current device (larger: tiled)
-int gs_tiled_max_size();           // largest n the method accepts
+int gs_one_cta_size();            // largest n without waits between CTAs
+int gs_tiled_max_size();           // largest n the method accepts (0: no device)
 cudaError_t gs_prepare();          // shared-memory opt-in on the current device, outside capture
 cudaError_t gs_step(const GsFields& F, int n, int pitch, int kd, int kp, float diff, float visc, float dt,
                     cudaStream_t st, int* launches);

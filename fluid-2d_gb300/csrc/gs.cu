@@ -1,32 +1,45 @@
 // Exact reproduction of the reference's host solver (fluid_solver_cpu, src/
-// fluid_solver_cpu.cpp:6-215) on the GPU, for square grids whose field fits in one
-// SM's shared memory (n <= gs_max_size(), 234 on a 227 KB part).
+// fluid_solver_cpu.cpp:6-215) on the GPU, for square grids up to gs_tiled_max_size().
 //
 // The host solver differs from the CUDA one in method, not just rounding: its
 // diffusion and pressure sweeps update in place in row-major order (lexicographic
 // Gauss-Seidel), every boundary fill also averages the four corners, the diffusion
 // divisor is float, there is no smoothing, and the forward splat adds in raster order.
-// Here each in-place solve runs in one CTA with the field in shared memory as an
-// anti-diagonal wavefront: cell (i, j) of sweep s is updated at time (i-1)+(j-1)+2s, so
-// every sweep sees its up/left neighbours already updated and its down/right
-// neighbours not yet, exactly as the sequential loop does, and all sweeps are in
-// flight at once. An edge cell is read only by its inner neighbour, so the thread that
-// updates that neighbour also rewrites the edge (the fill the host solver does after
-// every sweep); corners are never read by a sweep and are averaged once at the end.
-// The splat keeps the host solver's order of additions to every cell: a cell receives
-// its contributions in the raster order of their source cells. When no source moves
-// more than kGatherMaxD cells, each target cell gathers them itself, scanning the
-// sources around it in raster order (many CTAs); otherwise the whole CTA computes the
-// targets and weights of a chunk of source cells and one thread applies them in order.
 //
-// A step is four launches on the solver's pitched fields (element (i, j) at i*P + j):
-//   1. 3 CTAs: add sources + diffuse d | copy u, add sources, diffuse u, largest
-//      displacement | same for v
-//   2. project u, v (CTA 0) | splat d by the step's initial velocity into a scratch
-//      field: one CTA in order (CTA 1) or one CTA per 1024 target cells (CTAs 2..)
-//   3. copy u, v and advect both by the copies (CTA 0) | the splat result and the
-//      host solver's fill into d (CTA 1)
-//   4. 1 CTA : project u, v
+// Solves (gs_solve_kernel). Cell (i, j) of sweep s needs the new values above and to its
+// left and the previous sweep's to its right and below, so a sweep is a chain of
+// dependences through the grid, but sweeps can follow one another closely. The grid is cut
+// into bands of 32 rows, one CTA per band and one warp per sweep: a lane owns a row and
+// walks along the columns, lane l one column behind lane l - 1, so that
+//   left:  the lane's value of the step before (a register);
+//   above: the previous lane's value of the step before (a shuffle);
+//   right, below: the previous sweep's values, from the band's array, which every sweep
+//          updates in place; the value below comes from the next lane's load (a shuffle).
+// Sweep s runs `lag` columns behind sweep s - 1 on the next warp, all warps in step: chunks
+// of kChunk columns, a block barrier between them, a chunk's loads one chunk ahead of their
+// use. The row above a band and the row below it come from the neighbouring bands' CTAs
+// through global memory: each exported value is an 8-byte word {value, tag of the sweep},
+// read until the tag is the expected one, so that no fence and no separate flag is needed; a
+// word is overwritten only by a sweep that depends on its reader. Words are loaded two
+// chunks before their use (a load of another SM's store takes longer than a chunk).
+// Waits are bounded: a warp that gives up sets ctrl->error and the solve ends
+// (FS_ERR_TIMEOUT on the host). All CTAs are co-resident (cooperative launch); a CTA with
+// several bands takes every gridDim.x-th in turn, which cannot deadlock because a band's
+// sweeps reach at most as many bands ahead as a launch has sweeps.
+//
+// Grids whose bands all fit one SM's shared memory (up to 141 x 141) run in one CTA per
+// field instead, bands side by side, so that nothing leaves the SM.
+//
+// What bounds it: the latency of a chunk's instructions on the chain of bands, columns and
+// sweeps, and the trips between SMs (2-3 us per band with a CTA per band). At 20/20 sweeps a
+// step takes 0.43 ms at 130 x 130 (1.12 ms with a block barrier per anti-diagonal of one CTA)
+// and 1.61 ms at 800 x 800 (21.0 ms with a grid barrier per diagonal of 64 x 64 tiles).
+//
+// The splat keeps the host solver's order of additions to every cell: a cell receives
+// its contributions in the raster order of their source cells. Source cells are linked
+// into one list per target, and each cell sorts the few it receives; cells that receive
+// very many fall back to one thread that applies all sources in order.
+//
 // Every operation uses explicitly rounded single-precision intrinsics so that no
 // contraction changes a result; the outputs are bit-identical to the host solver's.
 
@@ -40,767 +53,803 @@
 namespace fs {
 namespace {
 
-constexpr int kGsThreads = 1024;
-constexpr int kGsStage = 512;   // source cells per splat chunk (in-order path)
-constexpr int kGatherMaxD = 16; // largest displacement (cells) for the gathering splat
+constexpr int kMaxWarps = 24;    // warps of a CTA; sweeps of one launch with a CTA per band
+constexpr int kLine = 33;        // floats per line of a band's array: 32 lanes and a pad
+constexpr int kChunk = 8;        // columns a warp advances between barriers
+constexpr unsigned kGsPolls = 1u << 21;  // default bound of a wait, about 2 s
 
-struct GsStageEntry {
-    int i0, j0;
-    float w[4];  // contributions to (i0,j0), (i0+1,j0), (i0,j0+1), (i0+1,j0+1)
+// One field of a solve. Diffusion: x + dt*src is both the start and the constant term;
+// pressure: the constant term is the divergence of (u, v), the start zero. A later launch
+// of the same solve (more than kMaxSweeps sweeps) starts from `start`.
+struct GsField {
+    const float* x;
+    const float* src;
+    const float* u;
+    const float* v;
+    const float* start;  // null: the first launch
+    float* out;
+    float* big;  // global memory for the band arrays that shared memory does not hold
+    int mode;
+    float a, den, rden;
 };
 
-// set_boundary_* of the host solver (fluid_solver_cpu.cpp:33-83) on an n x n field of
-// row stride `ld`: edges from their inner neighbours with the mode's signs, then the
-// corners averaged from their two edge neighbours. Ends with a block barrier.
-__device__ void cpu_fill(float* g, int n, int ld, int mode) {
-    const int tid = threadIdx.x, nt = blockDim.x;
-    const float s_lr = mode == BND_OPP_H ? -1.f : 1.f, s_tb = mode == BND_OPP_V ? -1.f : 1.f;
-    for (int k = 1 + tid; k < n - 1; k += nt) {
-        g[k * ld] = s_lr * g[k * ld + 1];
-        g[k * ld + n - 1] = s_lr * g[k * ld + n - 2];
-        g[k] = s_tb * g[ld + k];
-        g[(n - 1) * ld + k] = s_tb * g[(n - 2) * ld + k];
-    }
-    __syncthreads();
-    if (tid == 0) {
-        const int b = (n - 1) * ld, c = n - 1;
-        g[0] = __fmul_rn(0.5f, __fadd_rn(g[1], g[ld]));
-        g[c] = __fmul_rn(0.5f, __fadd_rn(g[c - 1], g[ld + c]));
-        g[b] = __fmul_rn(0.5f, __fadd_rn(g[b + 1], g[b - ld]));
-        g[b + c] = __fmul_rn(0.5f, __fadd_rn(g[b + c - 1], g[b - ld + c]));
-    }
-    __syncthreads();
-}
-
-// Pipelined lexicographic Gauss-Seidel on x (shared, n x n dense, in place):
-//   DIFF: x = (c + a*(U + D + L + R)) / den          (fluid_solver_cpu.cpp:105-110)
-//   else: x = (c + R + L + D + U) / 4                (fluid_solver_cpu.cpp:197-202)
-// with c read from `cst` (global, row stride P): x0 for diffusion, div for pressure.
-template <bool DIFF>
-__device__ void gs_wavefront(float* x, const float* cst, int n, int P, int iters, int mode, float a, float den) {
-    const int tid = threadIdx.x, nt = blockDim.x;
-    const float s_lr = mode == BND_OPP_H ? -1.f : 1.f, s_tb = mode == BND_OPP_V ? -1.f : 1.f;
-    const int m = n - 2, dmax = 2 * m - 2;
-    const int last_t = dmax + 2 * (iters - 1);
-    for (int t = 0; t <= last_t; ++t) {
-        // sweeps with a diagonal d = t - 2s in [0, dmax]
-        const int s_lo = t > dmax ? (t - dmax + 1) / 2 : 0;
-        const int s_hi = min(iters - 1, t / 2);
-        const int work = (s_hi - s_lo + 1) * m;
-        for (int e = tid; e < work; e += nt) {
-            const int s = s_lo + e / m, q = e % m, d = t - 2 * s;
-            if (q < d - (m - 1) || q > d) continue;
-            const int i = 1 + q, j = 1 + d - q;
-            const int o = i * n + j;
-            float val;
-            if (DIFF) {
-                float sum = __fadd_rn(x[o - n], x[o + n]);
-                sum = __fadd_rn(sum, x[o - 1]);
-                sum = __fadd_rn(sum, x[o + 1]);
-                val = __fdiv_rn(__fadd_rn(cst[i * P + j], __fmul_rn(a, sum)), den);
-            } else {
-                float sum = __fadd_rn(cst[i * P + j], x[o + 1]);
-                sum = __fadd_rn(sum, x[o - 1]);
-                sum = __fadd_rn(sum, x[o + n]);
-                sum = __fadd_rn(sum, x[o - n]);
-                val = __fdiv_rn(sum, 4.0f);
-            }
-            x[o] = val;
-            // the host solver's fill after this sweep, for the edges next to (i, j)
-            if (j == 1) x[o - 1] = s_lr * val;
-            if (j == n - 2) x[o + 1] = s_lr * val;
-            if (i == 1) x[o - n] = s_tb * val;
-            if (i == n - 2) x[o + n] = s_tb * val;
-        }
-        __syncthreads();
-    }
-}
-
-struct GsArgs {
-    float* f[3];         // d, u, v (state)
-    const float* src[3]; // ds, us, vs
-    float* su;           // scratch: copy of u
-    float* sv;           // scratch: copy of v
-    float* dv;           // scratch: divergence
-    float* acc;          // scratch: splat result (interior)
-    float* dmax;         // scratch: largest |dt0 u| and |dt0 v| of the step's initial velocity
-    int n, P, kd, kp;
-    float a[3], den[3];  // diffusion constants per field
-    float dt, dt0, h;
-};
-
-__device__ void copy_field(float* dst, const float* src, int n, int P) {
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) dst[(e / n) * P + e % n] = src[(e / n) * P + e % n];
-}
-
-// add_source then diffuse (fluid_solver_cpu.cpp:85-114) of field k.
-__device__ void gs_diffuse(const GsArgs& A, int k, float* x) {
-    const int n = A.n, P = A.P;
-    const int mode = k == 0 ? BND_CONT : (k == 1 ? BND_OPP_H : BND_OPP_V);
-    float* g = A.f[k];
-    const float* s = A.src[k];
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
-        const int i = e / n, j = e % n, o = i * P + j;
-        float val = g[o];
-        if (i > 0 && i < n - 1 && j > 0 && j < n - 1) {
-            val = __fadd_rn(val, __fmul_rn(A.dt, s[o]));
-            g[o] = val;  // the diffusion's x0
-        }
-        x[e] = val;
-    }
-    __syncthreads();
-    if (A.kd > 0) {
-        gs_wavefront<true>(x, g, n, P, A.kd, mode, A.a[k], A.den[k]);
-        cpu_fill(x, n, n, mode);
-    }
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) g[(e / n) * P + e % n] = x[e];
-}
-
-// advect(trace=true) (fluid_solver_cpu.cpp:127-152) of d by (su, sv), accumulating in
-// shared memory, then the host solver's continuous fill.
-__device__ void gs_splat(const GsArgs& A, float* acc, GsStageEntry* stage) {
-    const int n = A.n, P = A.P, m = n - 2;
-    const float* d0 = A.f[0];
-    const float hi = (float)n - 1.5f;
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) acc[e] = 0.f;
-    for (int base = 0; base < m * m; base += kGsStage) {
-        const int cnt = min(kGsStage, m * m - base);
-        __syncthreads();
-        for (int k = threadIdx.x; k < cnt; k += blockDim.x) {
-            const int c = base + k, i = 1 + c / m, j = 1 + c % m, o = i * P + j;
-            const float x = __fadd_rn((float)j, __fmul_rn(A.dt0, A.su[o]));
-            const float y = __fadd_rn((float)i, __fmul_rn(A.dt0, A.sv[o]));
-            GsStageEntry en;
-            if (!(x >= 0.5f && x <= hi && y >= 0.5f && y <= hi)) {  // NaN-safe form of the skip test
-                en.i0 = -1;
-                en.j0 = 0;
-                en.w[0] = en.w[1] = en.w[2] = en.w[3] = 0.f;
-            } else {
-                const int j0 = (int)x, i0 = (int)y;
-                const float s0 = __fsub_rn(x, (float)j0), s1 = __fsub_rn(1.f, s0);
-                const float s2 = __fsub_rn(y, (float)i0), s3 = __fsub_rn(1.f, s2);
-                const float w = d0[o];
-                en.i0 = i0;
-                en.j0 = j0;
-                en.w[0] = __fmul_rn(__fmul_rn(s1, s3), w);
-                en.w[1] = __fmul_rn(__fmul_rn(s1, s2), w);
-                en.w[2] = __fmul_rn(__fmul_rn(s0, s3), w);
-                en.w[3] = __fmul_rn(__fmul_rn(s0, s2), w);
-            }
-            stage[k] = en;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            for (int k = 0; k < cnt; ++k) {
-                const GsStageEntry en = stage[k];
-                if (en.i0 < 0) continue;
-                const int t = en.i0 * n + en.j0;
-                acc[t] = __fadd_rn(acc[t], en.w[0]);
-                acc[t + n] = __fadd_rn(acc[t + n], en.w[1]);
-                acc[t + 1] = __fadd_rn(acc[t + 1], en.w[2]);
-                acc[t + n + 1] = __fadd_rn(acc[t + n + 1], en.w[3]);
-            }
-        }
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < m * m; e += blockDim.x) {
-        const int i = 1 + e / m, j = 1 + e % m;
-        A.acc[i * P + j] = acc[i * n + j];
-    }
-}
-
-// The same splat gathered by target: thread t of target block b owns interior cell
-// T = b*blockDim + t and adds, in the raster order of the sources, the contribution of
-// every source within W = D + 2 cells (D = the largest displacement, so every source
-// that can reach T is scanned); each source reaches T through at most one corner.
-__device__ void gs_splat_gather(const GsArgs& A, int b, int D) {
-    const int n = A.n, P = A.P, m = n - 2;
-    const int e = b * blockDim.x + threadIdx.x;
-    if (e >= m * m) return;
-    const int ti = 1 + e / m, tj = 1 + e % m;
-    const float hi = (float)n - 1.5f;
-    const float* d0 = A.f[0];
-    const int W = D + 2;
-    const int i_lo = max(1, ti - W), i_hi = min(n - 2, ti + W), j_lo = max(1, tj - W), j_hi = min(n - 2, tj + W);
-    float acc = 0.f;
-    for (int i = i_lo; i <= i_hi; ++i)
-        for (int j = j_lo; j <= j_hi; ++j) {
-            const int o = i * P + j;
-            const float x = __fadd_rn((float)j, __fmul_rn(A.dt0, A.su[o]));
-            const float y = __fadd_rn((float)i, __fmul_rn(A.dt0, A.sv[o]));
-            if (!(x >= 0.5f && x <= hi && y >= 0.5f && y <= hi)) continue;
-            const int j0 = (int)x, i0 = (int)y;
-            const int di = ti - i0, dj = tj - j0;  // which corner of the source's cell T is
-            if ((unsigned)di > 1u || (unsigned)dj > 1u) continue;
-            const float s0 = __fsub_rn(x, (float)j0), s1 = __fsub_rn(1.f, s0);
-            const float s2 = __fsub_rn(y, (float)i0), s3 = __fsub_rn(1.f, s2);
-            const float wy = di ? s2 : s3, wx = dj ? s0 : s1;
-            acc = __fadd_rn(acc, __fmul_rn(__fmul_rn(wx, wy), d0[o]));
-        }
-    A.acc[ti * P + tj] = acc;
-}
-
-// project (fluid_solver_cpu.cpp:179-215) of (u, v), pressure from zero in shared memory.
-__device__ void gs_project(const GsArgs& A, float* p) {
-    const int n = A.n, P = A.P, m = n - 2;
-    float* u = A.f[1];
-    float* v = A.f[2];
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) p[e] = 0.f;
-    for (int e = threadIdx.x; e < m * m; e += blockDim.x) {
-        const int o = (1 + e / m) * P + 1 + e % m;
-        float s = __fsub_rn(u[o + 1], u[o - 1]);
-        s = __fadd_rn(s, v[o + P]);
-        s = __fsub_rn(s, v[o - P]);
-        A.dv[o] = __fmul_rn(__fmul_rn(-0.5f, A.h), s);
-    }
-    __syncthreads();
-    if (A.kp > 0) {
-        gs_wavefront<false>(p, A.dv, n, P, A.kp, BND_CONT, 0.f, 0.f);
-        cpu_fill(p, n, n, BND_CONT);
-    }
-    for (int e = threadIdx.x; e < m * m; e += blockDim.x) {
-        const int i = 1 + e / m, j = 1 + e % m, o = i * P + j, q = i * n + j;
-        u[o] = __fsub_rn(u[o], __fdiv_rn(__fmul_rn(0.5f, __fsub_rn(p[q + 1], p[q - 1])), A.h));
-        v[o] = __fsub_rn(v[o], __fdiv_rn(__fmul_rn(0.5f, __fsub_rn(p[q + n], p[q - n])), A.h));
-    }
-    __syncthreads();
-    cpu_fill(u, n, P, BND_OPP_H);
-    cpu_fill(v, n, P, BND_OPP_V);
-}
-
-// advect(trace=false) (fluid_solver_cpu.cpp:154-173) of u and v by the copies (su, sv).
-__device__ void gs_gather(const GsArgs& A) {
-    const int n = A.n, P = A.P, m = n - 2;
-    copy_field(A.su, A.f[1], n, P);
-    copy_field(A.sv, A.f[2], n, P);
-    __syncthreads();
-    const float hi = (float)n - 1.5f;
-    for (int e = threadIdx.x; e < m * m; e += blockDim.x) {
-        const int i = 1 + e / m, j = 1 + e % m, o = i * P + j;
-        float x = __fsub_rn((float)j, __fmul_rn(A.dt0, A.su[o]));
-        float y = __fsub_rn((float)i, __fmul_rn(A.dt0, A.sv[o]));
-        x = (x < hi) ? x : hi;
-        x = (1.5f < x) ? x : 1.5f;
-        y = (y < hi) ? y : hi;
-        y = (1.5f < y) ? y : 1.5f;
-        const int j0 = (int)x, i0 = (int)y;
-        const float s0 = __fsub_rn(x, (float)j0), s1 = __fsub_rn(1.f, s0);
-        const float s2 = __fsub_rn(y, (float)i0), s3 = __fsub_rn(1.f, s2);
-        const int a = i0 * P + j0;
-        for (int k = 0; k < 2; ++k) {
-            const float* g0 = k == 0 ? A.su : A.sv;
-            const float top = __fadd_rn(__fmul_rn(s1, g0[a]), __fmul_rn(s0, g0[a + 1]));
-            const float bot = __fadd_rn(__fmul_rn(s1, g0[a + P]), __fmul_rn(s0, g0[a + P + 1]));
-            A.f[1 + k][o] = __fadd_rn(__fmul_rn(s3, top), __fmul_rn(s2, bot));
-        }
-    }
-    __syncthreads();
-    cpu_fill(A.f[1], n, P, BND_OPP_H);
-    cpu_fill(A.f[2], n, P, BND_OPP_V);
-}
-
-__global__ void __launch_bounds__(kGsThreads) gs_diffuse_kernel(const __grid_constant__ GsArgs A) {
-    extern __shared__ float4 gs_smem[];
-    float* x = reinterpret_cast<float*>(gs_smem);
-    const int k = blockIdx.x;
-    if (k > 0) {  // keep the step's initial velocity for the density splat
-        float* dst = k == 1 ? A.su : A.sv;
-        const float* src = A.f[k];
-        const int n = A.n, P = A.P, m = n - 2;
-        copy_field(dst, src, n, P);
-        // largest interior displacement |dt0 * velocity| (non-finite counts as huge)
-        float dm = 0.f;
-        for (int e = threadIdx.x; e < m * m; e += blockDim.x) {
-            float a = fabsf(__fmul_rn(A.dt0, src[(1 + e / m) * P + 1 + e % m]));
-            if (!(a <= 1e30f)) a = 1e30f;
-            dm = fmaxf(dm, a);
-        }
-        __shared__ float red[32];
-        for (int o = 16; o > 0; o >>= 1) dm = fmaxf(dm, __shfl_xor_sync(0xffffffffu, dm, o));
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = dm;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            float t = 0.f;
-            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t = fmaxf(t, red[w]);
-            A.dmax[k - 1] = t;
-        }
-        __syncthreads();
-    }
-    gs_diffuse(A, k, x);
-}
-
-__global__ void __launch_bounds__(kGsThreads) gs_splat_project_kernel(const __grid_constant__ GsArgs A) {
-    extern __shared__ float4 gs_smem[];
-    float* f = reinterpret_cast<float*>(gs_smem);
-    // every CTA reads the same two values (written by the previous launch)
-    const float dm = fmaxf(__ldcg(A.dmax), __ldcg(A.dmax + 1));
-    const bool gather = dm <= (float)kGatherMaxD;
-    if (blockIdx.x == 0)
-        gs_project(A, f);
-    else if (blockIdx.x == 1) {
-        if (!gather) gs_splat(A, f, reinterpret_cast<GsStageEntry*>(f + A.n * A.n));
-    } else if (gather) {
-        gs_splat_gather(A, blockIdx.x - 2, (int)ceilf(dm));
-    }
-}
-
-// CTA 0: advect u, v; CTA 1: density = the splat result with the host solver's fill.
-__global__ void __launch_bounds__(kGsThreads) gs_gather_kernel(const __grid_constant__ GsArgs A) {
-    if (blockIdx.x == 0) {
-        gs_gather(A);
-        return;
-    }
-    const int n = A.n, P = A.P, m = n - 2;
-    float* d = A.f[0];
-    for (int e = threadIdx.x; e < m * m; e += blockDim.x) {
-        const int o = (1 + e / m) * P + 1 + e % m;
-        d[o] = A.acc[o];
-    }
-    __syncthreads();
-    cpu_fill(d, n, P, BND_CONT);
-}
-
-__global__ void __launch_bounds__(kGsThreads) gs_project_kernel(const __grid_constant__ GsArgs A) {
-    extern __shared__ float4 gs_smem[];
-    gs_project(A, reinterpret_cast<float*>(gs_smem));
-}
-
-size_t gs_smem_bytes(int n) {
-    return ((size_t)n * n * sizeof(float) + 15) / 16 * 16 + kGsStage * sizeof(GsStageEntry);
-}
-
-// ---------------------------------------------------------------------------
-// Tiled form for grids larger than one SM's shared memory.
-//
-// Each in-place solve runs as one cooperative launch over kTile x kTile tiles of the
-// interior, with the field in global memory. Tile (I, J) of sweep s is processed at
-// wavefront time t = I + J + 2s, all tiles of one time in parallel, a grid barrier
-// between times. This keeps every dependency of the sequential loop: the tiles above
-// and to the left finished sweep s at time t - 1 (their new values), the tiles below
-// and to the right finished sweep s - 1 at t - 1 and start sweep s only at t + 1 (their
-// old values), and no two tiles of one time are neighbours. Inside a tile the cells are
-// updated by the same anti-diagonal wavefront as the one-CTA form, from a shared copy
-// of the tile and its one-cell halo, and an update next to a domain edge rewrites that
-// edge cell (the host solver's fill after each sweep, which only that cell reads).
-// Grid barriers wait a bounded number of polls; a CTA that gives up sets ctrl->error
-// and the solve ends early (FS_ERR_TIMEOUT on the host).
-constexpr int kTile = 64;
-constexpr int kTileThreads = 64;
-constexpr unsigned kGsBarrierPolls = 1u << 24;
-
-struct GsTiled {
-    float* x;        // field, in place (row stride P)
-    const float* c;  // constant term: x0 (diffusion) or div (pressure)
-    int n, P, iters, mode;
-    float a, den;    // diffusion
+struct GsSolve {
+    GsField f[3];
+    int nf;
+    int n, P, sweeps;
+    int lag, band_lag;
+    int bands;
+    float dt, cdiv;
+    unsigned epoch;                // distinguishes the tags of a step's launches
+    unsigned long long* words;     // exported rows: [field][band][top, bottom][column]
     SolveCtrl* ctrl;
     const unsigned* poll_limit;
 };
 
-__device__ bool gs_grid_barrier(SolveCtrl* ctrl, unsigned nblocks, unsigned limit) {
-    __shared__ int s_ok;
+__device__ __forceinline__ unsigned long long ld_word(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_word(unsigned long long* p, float v, unsigned tag) {
+    const unsigned long long w = ((unsigned long long)tag << 32) | __float_as_uint(v);
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(w) : "memory");
+}
+
+// x / b correctly rounded, y = RN(1/b): Markstein's correction step (P. Markstein, IBM J.
+// Res. Dev. 34(1), 1990), exact for normal quotients and remainders; other x, and divisors
+// outside (2^-20, 2^20) (y passed as zero), take the IEEE division.
+__device__ __forceinline__ float gs_div(float x, float b, float y) {
+    const float ax = fabsf(x);
+    const float q0 = __fmul_rn(x, y);
+    const float r = __fmaf_rn(-q0, b, x);
+    const float q = ax == 0.f ? x : __fmaf_rn(r, y, q0);
+    if (((ax <= 0x1p-100f || !(ax < 0x1p100f)) && ax != 0.f) || y == 0.f) return __fdiv_rn(x, b);
+    return q;
+}
+
+// x + dt*s on an interior cell (fluid_solver_cpu.cpp:85-92).
+__device__ __forceinline__ float gs_source(float x, float s, float dt) { return __fadd_rn(x, __fmul_rn(dt, s)); }
+
+// Lines of a band's arrays: the columns, the lanes' skew, whole chunks.
+__host__ __device__ inline int gs_lines(int m) { return (m + 31 + kChunk - 1) / kChunk * kChunk; }
+
+// Where a band's arrays are: both in shared memory, the constant terms in global memory,
+// both there. Value of row (lane) l in column j of either: line j + l, place l.
+enum GsPlace { GS_SHARED = 0, GS_CONST_GLOBAL = 1, GS_GLOBAL = 2 };
+
+template <bool DIFF, int PLACE>
+struct GsBand {
+    const GsSolve& S;
+    const GsField& F;
+    int xo, co;          // offsets of the arrays in shared memory
+    float *xg, *cg;      // the arrays in global memory
+    int band, m, lane, lm;  // lm: lane of the grid's last interior row (the last band), else 32
+    bool top, bot;
+    float s_lr, s_tb;
+
+    __device__ __forceinline__ float& x(int line, int l) const {
+        extern __shared__ float4 gs_smem[];
+        const int k = line * kLine + l;
+        return PLACE == GS_GLOBAL ? xg[k] : reinterpret_cast<float*>(gs_smem)[xo + k];
+    }
+    __device__ __forceinline__ float& c(int line, int l) const {
+        extern __shared__ float4 gs_smem[];
+        const int k = line * kLine + l;
+        return PLACE == GS_SHARED ? reinterpret_cast<float*>(gs_smem)[co + k] : cg[k];
+    }
+
+    // The value a sweep 0 finds in grid cell (i, j).
+    __device__ __forceinline__ float initial(int i, int j) const {
+        const size_t o = (size_t)i * S.P + j;
+        if (F.start) return __ldcg(F.start + o);
+        if (!DIFF) return 0.f;
+        const float v = __ldg(F.x + o);
+        const bool in = i > 0 && i < S.n - 1 && j > 0 && j < S.n - 1;
+        return in ? gs_source(v, __ldg(F.src + o), S.dt) : v;
+    }
+
+    // a value of the neighbouring band's last or first row (arrays of one CTA)
+    __device__ __forceinline__ float x_above(int line) const { return x(line - (gs_lines(m) + 1), 31); }
+    __device__ __forceinline__ float x_below(int line) const { return x(line + (gs_lines(m) + 1), 0); }
+
+    // Load and store of the band by `parts` warps, this one the part-th.
+    __device__ void load(int part, int parts) const {
+        const int rows = min(32, m - band * 32);
+        // one more row than the band's own: the edge row, where it has a lane to live in
+        const int extra = bot && rows < 32 ? 1 : 0;
+        for (int l = part; l < rows + extra; l += parts) {
+            const int i = 1 + band * 32 + l;
+            const size_t row = (size_t)i * S.P + 1;
+#pragma unroll 4
+            for (int j = lane; j < m; j += 32) {
+                const float v = initial(i, 1 + j);
+                x(j + l, l) = v;
+                if (l >= rows) continue;
+                const size_t o = row + j;
+                if (DIFF) {
+                    c(j + l, l) = F.start ? gs_source(__ldg(F.x + o), __ldg(F.src + o), S.dt) : v;
+                } else {
+                    // (-0.5*h) * (uR - uL + vD - vU), fluid_solver_cpu.cpp:186-191
+                    float d = __fsub_rn(__ldg(F.u + o + 1), __ldg(F.u + o - 1));
+                    d = __fadd_rn(d, __ldg(F.v + o + S.P));
+                    d = __fsub_rn(d, __ldg(F.v + o - S.P));
+                    c(j + l, l) = __fmul_rn(S.cdiv, d);
+                }
+            }
+        }
+    }
+
+    // The band's final values with the host solver's fill (fluid_solver_cpu.cpp:33-83):
+    // edges from their inner neighbours, corners the mean of their two edge neighbours.
+    __device__ void store(int part, int parts) const {
+        const int rows = min(32, m - band * 32), P = S.P, n = S.n;
+        float* __restrict__ g = F.out;
+        for (int l = part; l < rows; l += parts) {
+            const int i = 1 + band * 32 + l;
+            const bool it = i == 1, ib = i == n - 2;
+#pragma unroll 4
+            for (int j = lane; j < m; j += 32) {
+                const float v = x(j + l, l);
+                const size_t o = (size_t)i * P + 1 + j;
+                g[o] = v;
+                const float ex = __fmul_rn(s_lr, v), ey = __fmul_rn(s_tb, v);
+                const bool jl = j == 0, jr = j == m - 1;
+                if (jl) g[o - 1] = ex;
+                if (jr) g[o + 1] = ex;
+                if (it) g[o - P] = ey;
+                if (ib) g[o + P] = ey;
+                if ((it || ib) && (jl || jr)) {
+                    const float q = __fmul_rn(0.5f, __fadd_rn(ey, ex));
+                    if (it && jl) g[o - P - 1] = q;
+                    if (it && jr) g[o - P + 1] = q;
+                    if (ib && jl) g[o + P - 1] = q;
+                    if (ib && jr) g[o + P + 1] = q;
+                }
+            }
+        }
+    }
+
+    // The previous sweep's values one column to the right, and the constant terms, of lines
+    // t0 .. t0 + kChunk - 1.
+    __device__ __forceinline__ void lines_of(int t0, float (&xr)[kChunk], float (&cc)[kChunk]) const {
+#pragma unroll
+        for (int k = 0; k < kChunk; ++k) {
+            xr[k] = x(t0 + k + 1, lane);
+            cc[k] = c(t0 + k, lane);
+        }
+    }
+};
+
+// One chunk of one sweep: lines t0 .. t0 + kChunk - 1. xr: the previous sweep's values one
+// column to the right; old: the one in line t0 before this sweep. inj: for lane 0 the values
+// above its row, for lane 31 those below its row. RAMP: some lane is outside the columns or
+// at an edge column. The fills of the domain's edges are known before the sweep's chain
+// starts (sign x a value of the previous sweep), so they go into its inputs.
+template <bool DIFF, int PLACE, bool RAMP>
+__device__ __forceinline__ void gs_chunk(const GsBand<DIFF, PLACE>& B, bool first, int t0, float (&xr)[kChunk],
+                                         const float (&cc)[kChunk], float (&inj)[kChunk], float& val, float& old,
+                                         float l_edge, float r_edge, float a, float den, float rden) {
+    constexpr unsigned FULL = 0xffffffffu;
+    const int lane = B.lane, m = B.m;
+    const float next_old = xr[kChunk - 1];
+    float below[kChunk], left[kChunk];
+#pragma unroll
+    for (int k = 0; k < kChunk; ++k) {
+        below[k] = __shfl_down_sync(FULL, xr[k], 1);
+        if (lane == 31) below[k] = inj[k];
+    }
+    if (!first) {
+        if (B.top && lane == 0) {
+#pragma unroll
+            for (int k = 0; k < kChunk; ++k) inj[k] = __fmul_rn(B.s_tb, k > 0 ? xr[k > 0 ? k - 1 : 0] : old);
+        }
+        if (B.bot && lane == B.lm) {
+#pragma unroll
+            for (int k = 0; k < kChunk; ++k) below[k] = __fmul_rn(B.s_tb, k > 0 ? xr[k > 0 ? k - 1 : 0] : old);
+        }
+    }
+    if (RAMP) {
+#pragma unroll
+        for (int k = kChunk - 1; k >= 0; --k) {
+            const float e = __fmul_rn(B.s_lr, k > 0 ? xr[k > 0 ? k - 1 : 0] : old);
+            left[k] = first ? l_edge : e;
+            if (t0 + k - lane == m - 1) xr[k] = first ? r_edge : e;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kChunk; ++k) {
+        const int j = t0 + k - lane;
+        float U = __shfl_up_sync(FULL, val, 1);
+        if (lane == 0) U = inj[k];
+        float L = val;
+        if (RAMP && j == 0) L = left[k];
+        float v;
+        if (DIFF) {  // (x0 + a*(U + D + L + R)) / (1 + 4a), fluid_solver_cpu.cpp:107-108
+            float sum = __fadd_rn(U, below[k]);
+            sum = __fadd_rn(sum, L);
+            sum = __fadd_rn(sum, xr[k]);
+            v = gs_div(__fadd_rn(cc[k], __fmul_rn(a, sum)), den, rden);
+            // cells outside the columns write places no valid cell reads; zero keeps them
+            // from decaying into the slow division
+            if (RAMP && (unsigned)j >= (unsigned)m) v = 0.f;
+        } else {  // (div + R + L + D + U) / 4, fluid_solver_cpu.cpp:199-200
+            float sum = __fadd_rn(cc[k], xr[k]);
+            sum = __fadd_rn(sum, L);
+            sum = __fadd_rn(sum, below[k]);
+            sum = __fadd_rn(sum, U);
+            v = __fmul_rn(sum, 0.25f);
+        }
+        val = v;
+        B.x(t0 + k, lane) = v;
+    }
+    old = next_old;
+}
+
+// ONE: a CTA holds all bands of a field, blockDim / 32 / bands sweeps of each in flight (a
+// warp takes every such sweep in turn), and neighbouring bands read each other's arrays.
+// Otherwise a CTA holds one band and a warp per sweep. Lags: columns between sweeps, and
+// (ONE) between bands.
+template <bool DIFF, int PLACE, bool ONE>
+__global__ void __launch_bounds__(32 * kMaxWarps) gs_solve_kernel(const __grid_constant__ GsSolve S) {
+    __shared__ int s_stop;
+    __shared__ __align__(16) float s_mail[kMaxWarps][2 * kChunk];
+    const int m = S.n - 2, lines = gs_lines(m);
+    const int array = (lines + 1) * kLine;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int in_flight = ONE ? (int)(blockDim.x >> 5) / S.bands : S.sweeps;
+    const unsigned lim_set = S.poll_limit ? __ldcg(S.poll_limit) : 0u;
+    const unsigned limit = lim_set ? lim_set : kGsPolls;
+    if (threadIdx.x == 0) s_stop = 0;
+    for (int item = blockIdx.x; item < (ONE ? S.nf : S.nf * S.bands); item += gridDim.x) {
+        const int fi = ONE ? item : item / S.bands;
+        const GsField& F = S.f[fi];
+        const int band = ONE ? w % S.bands : item - fi * S.bands;
+        int s = ONE ? w / S.bands : w;
+        GsBand<DIFF, PLACE> B{S, F};
+        B.xo = ONE ? band * array : 0;
+        B.co = ONE ? (S.bands + band) * array : array;
+        B.xg = F.big + (size_t)band * array * (PLACE == GS_GLOBAL ? 2 : 1);
+        B.cg = B.xg + (PLACE == GS_GLOBAL ? array : 0);
+        B.band = band;
+        B.m = m;
+        B.lane = lane;
+        B.top = band == 0;
+        B.bot = band == S.bands - 1;
+        B.lm = B.bot ? m - 1 - band * 32 : 32;
+        B.s_lr = F.mode == BND_OPP_H ? -1.f : 1.f;
+        B.s_tb = F.mode == BND_OPP_V ? -1.f : 1.f;
+        // lanes behind the grid's last row stay zero (their constant terms are)
+        const float a = lane > B.lm ? 0.f : F.a, den = F.den, rden = F.rden;
+        // the warps that load and store a band: all of the CTA, or (ONE) the band's own
+        const int part = ONE ? s : w, parts = ONE ? in_flight : (int)(blockDim.x >> 5);
+        __syncthreads();  // the previous band's store has read the arrays
+        // places outside the columns and rows stay finite: nothing reads them, but a NaN
+        // would send its lane through the slow division
+        for (int k = part * 32 + lane; k < array; k += parts * 32) B.x(0, k) = B.c(0, k) = 0.f;
+        __syncthreads();
+        B.load(part, parts);
+        __syncthreads();
+        // edge values a first sweep reads
+        float l_edge = 0.f, r_edge = 0.f;
+        if (s == 0 && 1 + band * 32 + lane < S.n - 1) {
+            l_edge = B.initial(1 + band * 32 + lane, 0);
+            r_edge = B.initial(1 + band * 32 + lane, S.n - 1);
+        }
+        // Imported rows, one value per lane and chunk: lanes 0 .. kChunk-1 the last row of the
+        // band above, this sweep's values; lanes 16 .. 16+kChunk-1 the first row of the band
+        // below, the sweep before. Exported rows: the same lanes the band's first and last row.
+        unsigned long long* const W = S.words + ((size_t)fi * S.bands + band) * 2 * m;
+        const unsigned tag = S.epoch * 64u + s + 1u;
+        const bool role_u = lane < kChunk, role_d = lane >= 16 && lane < 16 + kChunk;
+        const int k_role = lane & 15, shift = role_d ? k_role - 31 : k_role;  // column = t0 + shift
+        const unsigned long long* imp = nullptr;
+        unsigned want = tag;
+        if (!ONE && role_u && !B.top) imp = W - m;
+        if (!ONE && role_d && !B.bot && s > 0) {
+            imp = W + 2 * m;
+            want = tag - 1u;
+        }
+        unsigned long long* exp = nullptr;
+        if (!ONE && role_u && !B.top) exp = W;
+        if (!ONE && role_d && !B.bot) exp = W + m;
+        const int direct_row = role_u ? 0 : 1 + (band + 1) * 32;
+        float* const mail = s_mail[w] + (role_d ? kChunk : 0) + k_role;
+        const float4* const box = reinterpret_cast<const float4*>(s_mail[w] + (lane == 31 ? kChunk : 0));
+        auto fetch = [&](int t0) {
+            const int j = t0 + shift;
+            return imp != nullptr && (unsigned)j < (unsigned)m ? ld_word(imp + j) : 0ull;
+        };
+        float val = 0.f, old = 0.f;
+        float xa[kChunk], ca[kChunk], xb[kChunk], cb[kChunk];
+#pragma unroll
+        for (int k = 0; k < kChunk; ++k) xa[k] = ca[k] = xb[k] = cb[k] = 0.f;
+        const int start = ONE ? band * S.band_lag : 0;
+        const int total = lines + S.lag * (S.sweeps - 1) + (ONE ? S.band_lag * (S.bands - 1) : 0);
+        // chunk q; word, xr, cc: its import, loaded two chunks before, and its lines, loaded one
+        // before; next, xn, cn: the next chunk's
+        auto chunk = [&](int q, unsigned long long& word, unsigned long long& next, float (&xr)[kChunk],
+                         float (&cc)[kChunk], float (&xn)[kChunk], float (&cn)[kChunk]) {
+            if (ONE && q * kChunk - s * S.lag - start >= lines) s += in_flight;
+            const int t0 = q * kChunk - s * S.lag - start;
+            const bool first = s == 0;
+            if (t0 >= 0 && t0 < lines && s < S.sweeps) {  // t0 is a multiple of kChunk
+                if (t0 == 0) {
+                    word = fetch(t0);
+                    next = fetch(t0 + kChunk);
+                    old = B.x(0, lane);
+                    val = 0.f;
+                    B.lines_of(t0, xr, cc);
+                }
+                const int jr = t0 + shift;
+                const bool in_row = (unsigned)jr < (unsigned)m;
+                float in = 0.f;
+                if (ONE) {
+                    // completed by the barrier: the band above is 31 columns and a chunk ahead
+                    if (in_row && role_u && !B.top) in = B.x_above(t0 + k_role + 31);
+                    if (in_row && role_d && !B.bot && !first) in = B.x_below(jr);
+                } else {
+                    const bool needs = imp != nullptr && in_row;
+                    unsigned polls = 0;
+                    while (!__all_sync(0xffffffffu, !needs || (unsigned)(word >> 32) == want)) {
+                        if (++polls > limit || ((polls & 63u) == 0 && *(volatile int*)&S.ctrl->error != 0)) {
+                            if (lane == 0) {
+                                atomicExch(&S.ctrl->error, 1);
+                                *(volatile int*)&s_stop = 1;
+                            }
+                            break;
+                        }
+                        word = fetch(t0);
+                    }
+                    in = __uint_as_float((unsigned)word);
+                }
+                // a first sweep's values of rows outside the band that no import carries
+                if (first && ((role_u && B.top) || role_d))
+                    in = in_row && direct_row < S.n ? B.initial(direct_row, 1 + jr) : 0.f;
+                if (role_u || role_d) *mail = in;
+                __syncwarp();
+                float inj[kChunk];
+#pragma unroll
+                for (int k = 0; k < kChunk; k += 4) {
+                    const float4 v = box[k / 4];
+                    inj[k] = v.x;
+                    inj[k + 1] = v.y;
+                    inj[k + 2] = v.z;
+                    inj[k + 3] = v.w;
+                }
+                if (!ONE) word = fetch(t0 + 2 * kChunk);
+                // the next chunk's lines: the previous sweep is past them (lag > 2 chunks)
+                if (t0 + kChunk < lines) B.lines_of(t0 + kChunk, xn, cn);
+                if (t0 < 32 || t0 + kChunk >= m)
+                    gs_chunk<DIFF, PLACE, true>(B, first, t0, xr, cc, inj, val, old, l_edge, r_edge, a, den, rden);
+                else
+                    gs_chunk<DIFF, PLACE, false>(B, first, t0, xr, cc, inj, val, old, l_edge, r_edge, a, den, rden);
+                if (!ONE) {
+                    __syncwarp();
+                    if (exp != nullptr && in_row) st_word(exp + jr, B.x(t0 + k_role, role_d ? 31 : 0), tag);
+                }
+            }
+            __syncthreads();
+            return ONE || *(volatile int*)&s_stop == 0;  // the same for every thread after the barrier
+        };
+        unsigned long long wa = 0, wb = 0;
+#pragma unroll 1
+        for (int q = 0; q * kChunk < total; q += 2) {
+            if (!chunk(q, wa, wb, xa, ca, xb, cb)) return;
+            if (!chunk(q + 1, wb, wa, xb, cb, xa, ca)) return;
+        }
+        B.store(part, parts);
+    }
+}
+
+// The fields a solve of no sweeps leaves: x + dt*s, edges as given.
+__global__ void gs_add_kernel(const GsSolve S) {
+    const GsField& F = S.f[blockIdx.y];
+    for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < (long)S.n * S.n; e += (long)gridDim.x * blockDim.x) {
+        const int i = (int)(e / S.n), j = (int)(e % S.n);
+        const size_t o = (size_t)i * S.P + j;
+        const bool in = i > 0 && i < S.n - 1 && j > 0 && j < S.n - 1;
+        F.out[o] = in ? gs_source(F.x[o], F.src[o], S.dt) : F.x[o];
+    }
+}
+
+struct GsVel {
+    const float *u, *v;  // in
+    const float* p;      // remove_p only
+    float *uo, *vo;
+    int n, P;
+    float h, dt0;
+};
+
+// Writes (un, vn) of inner cell (i, j) to cell (gi, gj) = itself or an edge or corner cell
+// next to it, with the host solver's reflecting fills.
+__device__ __forceinline__ void gs_put(const GsVel& A, int gi, int gj, int i, int j, float un, float vn) {
+    const size_t o = (size_t)gi * A.P + gj;
+    const bool ei = gi != i, ej = gj != j;
+    float a = un, b = vn;
+    if (ei && ej) {  // the mean of the corner's two edge neighbours
+        a = __fmul_rn(0.5f, __fadd_rn(un, -un));
+        b = __fmul_rn(0.5f, __fadd_rn(-vn, vn));
+    } else if (ej) {
+        a = -un;
+    } else if (ei) {
+        b = -vn;
+    }
+    A.uo[o] = a;
+    A.vo[o] = b;
+}
+
+// remove_p (fluid_solver_cpu.cpp:205-210) and the reflecting fills, one thread per cell.
+__global__ void __launch_bounds__(256) gs_remove_p_kernel(const GsVel A) {
+    const int gj = blockIdx.x * 32 + threadIdx.x, gi = blockIdx.y * 8 + threadIdx.y;
+    if (gi >= A.n || gj >= A.n) return;
+    const int i = min(max(gi, 1), A.n - 2), j = min(max(gj, 1), A.n - 2);
+    const size_t o = (size_t)i * A.P + j;
+    const float* __restrict__ p = A.p;
+    const float un = __fsub_rn(A.u[o], __fdiv_rn(__fmul_rn(0.5f, __fsub_rn(p[o + 1], p[o - 1])), A.h));
+    const float vn = __fsub_rn(A.v[o], __fdiv_rn(__fmul_rn(0.5f, __fsub_rn(p[o + A.P], p[o - A.P])), A.h));
+    gs_put(A, gi, gj, i, j, un, vn);
+}
+
+// advect(trace=false) (fluid_solver_cpu.cpp:154-173) of u and v by themselves and the
+// reflecting fills, one thread per cell.
+__global__ void __launch_bounds__(256) gs_gather_kernel(const GsVel A) {
+    const int gj = blockIdx.x * 32 + threadIdx.x, gi = blockIdx.y * 8 + threadIdx.y;
+    if (gi >= A.n || gj >= A.n) return;
+    const int i = min(max(gi, 1), A.n - 2), j = min(max(gj, 1), A.n - 2), P = A.P;
+    const size_t o = (size_t)i * P + j;
+    const float hi = (float)A.n - 1.5f;
+    float x = __fsub_rn((float)j, __fmul_rn(A.dt0, A.u[o]));
+    float y = __fsub_rn((float)i, __fmul_rn(A.dt0, A.v[o]));
+    x = (x < hi) ? x : hi;
+    x = (1.5f < x) ? x : 1.5f;
+    y = (y < hi) ? y : hi;
+    y = (1.5f < y) ? y : 1.5f;
+    const int j0 = (int)x, i0 = (int)y;
+    const float s0 = __fsub_rn(x, (float)j0), s1 = __fsub_rn(1.f, s0);
+    const float s2 = __fsub_rn(y, (float)i0), s3 = __fsub_rn(1.f, s2);
+    const size_t a = (size_t)i0 * P + j0;
+    auto mix = [&](const float* __restrict__ g) {
+        const float t = __fadd_rn(__fmul_rn(s1, g[a]), __fmul_rn(s0, g[a + 1]));
+        const float b = __fadd_rn(__fmul_rn(s1, g[a + P]), __fmul_rn(s0, g[a + P + 1]));
+        return __fadd_rn(__fmul_rn(s3, t), __fmul_rn(s2, b));
+    };
+    gs_put(A, gi, gj, i, j, mix(A.u), mix(A.v));
+}
+
+// ------------------------------------------------------------------- splat
+struct GsSplat {
+    const float *d, *u, *v;  // diffused density, the step's initial velocity
+    float* out;
+    int* head;  // per target cell: the last source linked to it (-1: none)
+    int* next;  // per source cell: the source linked before it
+    int* many;  // set when a cell receives more sources than kGsMost
+    int n, P;
+    float dt0;
+};
+constexpr int kGsSorted = 24;  // sources a thread sorts in its own array
+constexpr int kGsMost = 256;   // more go to the in-order form
+
+// Target cell and offsets of source (i, j) (fluid_solver_cpu.cpp:132-139); false when the
+// source leaves the grid (a NaN position too).
+__device__ __forceinline__ bool gs_target(const GsSplat& A, int i, int j, int& i0, int& j0, float& s0, float& s2) {
+    const size_t o = (size_t)i * A.P + j;
+    const float hi = (float)A.n - 1.5f;
+    const float x = __fadd_rn((float)j, __fmul_rn(A.dt0, __ldg(A.u + o)));
+    const float y = __fadd_rn((float)i, __fmul_rn(A.dt0, __ldg(A.v + o)));
+    if (!(x >= 0.5f && x <= hi && y >= 0.5f && y <= hi)) return false;
+    j0 = (int)x;
+    i0 = (int)y;
+    s0 = __fsub_rn(x, (float)j0);
+    s2 = __fsub_rn(y, (float)i0);
+    return true;
+}
+
+__global__ void __launch_bounds__(256) gs_link_kernel(const GsSplat A) {
+    const int j = 1 + blockIdx.x * 32 + threadIdx.x, i = 1 + blockIdx.y * 8 + threadIdx.y;
+    if (i > A.n - 2 || j > A.n - 2) return;
+    int i0, j0;
+    float s0, s2;
+    if (!gs_target(A, i, j, i0, j0, s0, s2)) return;
+    const int o = i * A.P + j;
+    A.next[o] = atomicExch(A.head + (i0 * A.P + j0), o);
+}
+
+// Contribution of source o to the cell at offset (di, dj) from its target.
+__device__ __forceinline__ float gs_share(const GsSplat& A, int o, int di, int dj) {
+    const int i = o / A.P, j = o - i * A.P;
+    int i0, j0;
+    float s0, s2;
+    gs_target(A, i, j, i0, j0, s0, s2);
+    const float wx = dj ? s0 : __fsub_rn(1.f, s0), wy = di ? s2 : __fsub_rn(1.f, s2);
+    return __fmul_rn(__fmul_rn(wx, wy), __ldg(A.d + o));
+}
+
+// Sum of the contributions to interior cell (i, j) in the raster order of their sources
+// (advect(trace=true), fluid_solver_cpu.cpp:127-152).
+__device__ float gs_collect(const GsSplat& A, int i, int j) {
+    int src[kGsSorted];  // source * 4 + corner; a source reaches a cell through one corner
+    int cnt = 0;
+    for (int c = 0; c < 4; ++c) {
+        const int di = c >> 1, dj = c & 1;
+        for (int o = __ldcg(A.head + ((i - di) * A.P + j - dj)); o >= 0; o = __ldcg(A.next + o)) {
+            if (cnt < kGsSorted) {
+                int k = cnt;
+                for (; k > 0 && (src[k - 1] >> 2) > o; --k) src[k] = src[k - 1];
+                src[k] = o * 4 + c;
+            }
+            if (++cnt > kGsMost) {
+                atomicExch(A.many, 1);
+                return 0.f;
+            }
+        }
+    }
+    float acc = 0.f;
+    if (cnt <= kGsSorted) {
+        for (int k = 0; k < cnt; ++k) acc = __fadd_rn(acc, gs_share(A, src[k] >> 2, (src[k] >> 1) & 1, src[k] & 1));
+        return acc;
+    }
+    // more than the array holds: the lists once per contribution, next larger source each time
+    int last = -1;
+    for (int k = 0; k < cnt; ++k) {
+        int best = 0x7fffffff, bc = 0;
+        for (int c = 0; c < 4; ++c)
+            for (int o = __ldcg(A.head + ((i - (c >> 1)) * A.P + j - (c & 1))); o >= 0; o = __ldcg(A.next + o))
+                if (o > last && o < best) {
+                    best = o;
+                    bc = c;
+                }
+        acc = __fadd_rn(acc, gs_share(A, best, bc >> 1, bc & 1));
+        last = best;
+    }
+    return acc;
+}
+
+// One thread per cell; edges and corners repeat or average (their two edge neighbours hold
+// the same value) the inner cell's sum.
+__global__ void __launch_bounds__(256) gs_splat_kernel(const GsSplat A) {
+    const int gj = blockIdx.x * 32 + threadIdx.x, gi = blockIdx.y * 8 + threadIdx.y;
+    if (gi >= A.n || gj >= A.n) return;
+    const int i = min(max(gi, 1), A.n - 2), j = min(max(gj, 1), A.n - 2);
+    const float x = gs_collect(A, i, j);
+    A.out[(size_t)gi * A.P + gj] = gi != i && gj != j ? __fmul_rn(0.5f, __fadd_rn(x, x)) : x;
+}
+
+// Every source in order by one thread, when some cell received more than kGsMost.
+__global__ void __launch_bounds__(1024) gs_splat_in_order_kernel(const GsSplat A) {
+    if (*A.many == 0) return;
+    const int n = A.n, P = A.P;
+    float* g = A.out;
+    for (int e = threadIdx.x; e < n * n; e += blockDim.x) g[(size_t)(e / n) * P + e % n] = 0.f;
     __syncthreads();
     if (threadIdx.x == 0) {
-        volatile unsigned* gen = &ctrl->bar_gen;
-        volatile int* err = &ctrl->error;
-        const unsigned g = *gen;
-        __threadfence();
-        if (atomicAdd(&ctrl->bar_count, 1u) == nblocks - 1) {
-            atomicExch(&ctrl->bar_count, 0u);
-            __threadfence();
-            atomicAdd(&ctrl->bar_gen, 1u);
-        } else {
-            unsigned spins = 0;
-            while (*gen == g && *err == 0) {
-                if (++spins > limit) {
-                    atomicExch(&ctrl->error, 1);
-                    break;
-                }
-                __nanosleep(64);
+        for (int i = 1; i < n - 1; ++i)
+            for (int j = 1; j < n - 1; ++j) {
+                int i0, j0;
+                float s0, s2;
+                if (!gs_target(A, i, j, i0, j0, s0, s2)) continue;
+                const float s1 = __fsub_rn(1.f, s0), s3 = __fsub_rn(1.f, s2);
+                const float w = A.d[(size_t)i * P + j];
+                // edge cells that this adds to are filled below
+                float* t = g + (size_t)i0 * P + j0;
+                t[0] = __fadd_rn(t[0], __fmul_rn(__fmul_rn(s1, s3), w));
+                t[P] = __fadd_rn(t[P], __fmul_rn(__fmul_rn(s1, s2), w));
+                t[1] = __fadd_rn(t[1], __fmul_rn(__fmul_rn(s0, s3), w));
+                t[P + 1] = __fadd_rn(t[P + 1], __fmul_rn(__fmul_rn(s0, s2), w));
             }
-        }
-        __threadfence();
-        s_ok = (*err == 0);
     }
     __syncthreads();
-    return s_ok != 0;
-}
-
-template <bool DIFF>
-__device__ void gs_tile(const GsTiled& S, int I, int J, float* xs, float* cs) {
-    constexpr int LD = kTile + 2;
-    const int n = S.n, P = S.P, tid = threadIdx.x, nt = blockDim.x;
-    const float s_lr = S.mode == BND_OPP_H ? -1.f : 1.f, s_tb = S.mode == BND_OPP_V ? -1.f : 1.f;
-    const int i0 = 1 + I * kTile, j0 = 1 + J * kTile;
-    const int th = min(kTile, n - 1 - i0), tw = min(kTile, n - 1 - j0);
-    for (int e = tid; e < (th + 2) * (tw + 2); e += nt) {
-        const int r = e / (tw + 2), q = e - r * (tw + 2);
-        xs[r * LD + q] = __ldcg(S.x + (size_t)(i0 - 1 + r) * P + (j0 - 1 + q));
-    }
-    for (int e = tid; e < th * tw; e += nt) {
-        const int r = e / tw, q = e - r * tw;
-        cs[r * kTile + q] = __ldcg(S.c + (size_t)(i0 + r) * P + (j0 + q));
-    }
-    __syncthreads();
-    for (int dg = 0; dg < th + tw - 1; ++dg) {
-        for (int r = tid; r < th; r += nt) {
-            const int q = dg - r;
-            if (q < 0 || q >= tw) continue;
-            const int o = (r + 1) * LD + q + 1;
-            float val;
-            if (DIFF) {  // (x0 + a*(U + D + L + R)) / (1 + 4a), fluid_solver_cpu.cpp:107-108
-                float sum = __fadd_rn(xs[o - LD], xs[o + LD]);
-                sum = __fadd_rn(sum, xs[o - 1]);
-                sum = __fadd_rn(sum, xs[o + 1]);
-                val = __fdiv_rn(__fadd_rn(cs[r * kTile + q], __fmul_rn(S.a, sum)), S.den);
-            } else {     // (div + R + L + D + U) / 4, fluid_solver_cpu.cpp:199-200
-                float sum = __fadd_rn(cs[r * kTile + q], xs[o + 1]);
-                sum = __fadd_rn(sum, xs[o - 1]);
-                sum = __fadd_rn(sum, xs[o + LD]);
-                sum = __fadd_rn(sum, xs[o - LD]);
-                val = __fdiv_rn(sum, 4.0f);
-            }
-            xs[o] = val;
-            const int gi = i0 + r, gj = j0 + q;
-            if (gj == 1) xs[o - 1] = s_lr * val;
-            if (gj == n - 2) xs[o + 1] = s_lr * val;
-            if (gi == 1) xs[o - LD] = s_tb * val;
-            if (gi == n - 2) xs[o + LD] = s_tb * val;
-        }
-        __syncthreads();
-    }
-    // the tile, and the domain-edge cells next to it (the other halo cells belong to
-    // other tiles)
-    for (int e = tid; e < th * tw; e += nt) {
-        const int r = e / tw, q = e - r * tw;
-        S.x[(size_t)(i0 + r) * P + (j0 + q)] = xs[(r + 1) * LD + q + 1];
-    }
-    for (int q = tid; q < tw; q += nt) {
-        if (i0 == 1) S.x[j0 + q] = xs[q + 1];
-        if (i0 + th == n - 1) S.x[(size_t)(n - 1) * P + j0 + q] = xs[(th + 1) * LD + q + 1];
-    }
-    for (int r = tid; r < th; r += nt) {
-        if (j0 == 1) S.x[(size_t)(i0 + r) * P] = xs[(r + 1) * LD];
-        if (j0 + tw == n - 1) S.x[(size_t)(i0 + r) * P + n - 1] = xs[(r + 1) * LD + tw + 1];
-    }
-    __syncthreads();  // xs is reused by this CTA's next tile
-}
-
-template <bool DIFF>
-__global__ void __launch_bounds__(kTileThreads) gs_tiled_kernel(const __grid_constant__ GsTiled S) {
-    __shared__ float xs[(kTile + 2) * (kTile + 2)];
-    __shared__ float cs[kTile * kTile];
-    const int m = S.n - 2, NT = (m + kTile - 1) / kTile, K = S.iters;
-    const unsigned G = gridDim.x;
-    const unsigned lim_set = S.poll_limit ? __ldcg(S.poll_limit) : 0u;
-    const unsigned limit = lim_set ? lim_set : kGsBarrierPolls;
-    const int last_t = 2 * (NT - 1) + 2 * (K - 1);
-    for (int t = 0; t <= last_t; ++t) {
-        int base = 0;
-        for (int s = max(0, (t - 2 * (NT - 1) + 1) / 2); s <= min(K - 1, t / 2); ++s) {
-            const int d = t - 2 * s;
-            const int ilo = max(0, d - NT + 1), ihi = min(NT - 1, d);
-            for (int k = 0; k <= ihi - ilo; ++k)
-                if ((unsigned)(base + k) % G == blockIdx.x) gs_tile<DIFF>(S, ilo + k, d - ilo - k, xs, cs);
-            base += max(0, ihi - ilo + 1);
-        }
-        if (t < last_t && !gs_grid_barrier(S.ctrl, G, limit)) return;
-    }
-}
-
-// The host solver's fill (cpu_fill) on a field in global memory, one CTA.
-__global__ void __launch_bounds__(kGsThreads) gs_fill_kernel(float* g, int n, int P, int mode) { cpu_fill(g, n, P, mode); }
-
-// x += dt*s on the interior and x0 = x (the diffusion's constant term).
-__global__ void gs_add_copy_kernel(float* x, const float* __restrict__ src, float* __restrict__ x0, int n, int P,
-                                   float dt) {
-    for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < (long)n * n; e += (long)gridDim.x * blockDim.x) {
-        const int i = (int)(e / n), j = (int)(e % n);
-        const size_t o = (size_t)i * P + j;
-        float val = x[o];
-        if (i > 0 && i < n - 1 && j > 0 && j < n - 1) {
-            val = __fadd_rn(val, __fmul_rn(dt, src[o]));
-            x[o] = val;
-        }
-        x0[o] = val;
-    }
-}
-
-// su = u, sv = v and the largest interior displacement |dt0 * velocity| into dmax[0..1]
-// (float bits, non-negative, so an integer maximum orders them; zeroed before).
-__global__ void gs_copy_vel_kernel(const GsArgs A) {
-    const int n = A.n, P = A.P;
-    float dm = 0.f;
-    for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < (long)n * n; e += (long)gridDim.x * blockDim.x) {
-        const int i = (int)(e / n), j = (int)(e % n);
-        const size_t o = (size_t)i * P + j;
-        const float u = A.f[1][o], v = A.f[2][o];
-        A.su[o] = u;
-        A.sv[o] = v;
-        if (i > 0 && i < n - 1 && j > 0 && j < n - 1) {
-            float a = fmaxf(fabsf(__fmul_rn(A.dt0, u)), fabsf(__fmul_rn(A.dt0, v)));
-            if (!(a <= 1e30f)) a = 1e30f;
-            dm = fmaxf(dm, a);
-        }
-    }
-    for (int o = 16; o > 0; o >>= 1) dm = fmaxf(dm, __shfl_xor_sync(0xffffffffu, dm, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<int*>(A.dmax), __float_as_int(dm));
-}
-
-// Divergence (fluid_solver_cpu.cpp:186-191) into dv and p = 0.
-__global__ void gs_div_kernel(const GsArgs A, float* p) {
-    const int n = A.n, P = A.P;
-    for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < (long)n * n; e += (long)gridDim.x * blockDim.x) {
-        const int i = (int)(e / n), j = (int)(e % n);
-        const size_t o = (size_t)i * P + j;
-        p[o] = 0.f;
-        if (i > 0 && i < n - 1 && j > 0 && j < n - 1) {
-            const float* u = A.f[1];
-            const float* v = A.f[2];
-            float s = __fsub_rn(u[o + 1], u[o - 1]);
-            s = __fadd_rn(s, v[o + P]);
-            s = __fsub_rn(s, v[o - P]);
-            A.dv[o] = __fmul_rn(__fmul_rn(-0.5f, A.h), s);
+    for (int k = threadIdx.x; k < n; k += blockDim.x) {
+        const int c = min(max(k, 1), n - 2);
+        const float w = g[(size_t)c * P + 1], e = g[(size_t)c * P + n - 2], t = g[P + c], b = g[(size_t)(n - 2) * P + c];
+        if (k == c) {
+            g[(size_t)k * P] = w;
+            g[(size_t)k * P + n - 1] = e;
+            g[k] = t;
+            g[(size_t)(n - 1) * P + k] = b;
+        } else {  // corners: (0, 0) and (0, n-1), or (n-1, 0) and (n-1, n-1)
+            g[(size_t)k * P] = __fmul_rn(0.5f, __fadd_rn(w, w));
+            g[(size_t)k * P + n - 1] = __fmul_rn(0.5f, __fadd_rn(e, e));
         }
     }
 }
 
-// remove_p (fluid_solver_cpu.cpp:205-210) on the interior.
-__global__ void gs_remove_p_kernel(const GsArgs A, const float* __restrict__ p) {
-    const int n = A.n, P = A.P, m = n - 2;
-    for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < (long)m * m; e += (long)gridDim.x * blockDim.x) {
-        const size_t o = (size_t)(1 + e / m) * P + 1 + e % m;
-        float* u = A.f[1];
-        float* v = A.f[2];
-        u[o] = __fsub_rn(u[o], __fdiv_rn(__fmul_rn(0.5f, __fsub_rn(p[o + 1], p[o - 1])), A.h));
-        v[o] = __fsub_rn(v[o], __fdiv_rn(__fmul_rn(0.5f, __fsub_rn(p[o + P], p[o - P])), A.h));
-    }
+// ------------------------------------------------------------------- host
+size_t array_bytes(int n) { return (size_t)(gs_lines(n - 2) + 1) * kLine * sizeof(float); }
+
+int smem_limit() {
+    int dev = 0, smem = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    if (cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 0;
+    return smem - 2048;  // the kernel's static shared memory
 }
 
-// advect(trace=false) of u and v by the copies (su, sv) on the interior
-// (fluid_solver_cpu.cpp:154-173).
-__global__ void gs_gather_grid_kernel(const GsArgs A) {
-    const int n = A.n, P = A.P, m = n - 2;
-    const float hi = (float)n - 1.5f;
-    for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < (long)m * m; e += (long)gridDim.x * blockDim.x) {
-        const int i = 1 + (int)(e / m), j = 1 + (int)(e % m);
-        const size_t o = (size_t)i * P + j;
-        float x = __fsub_rn((float)j, __fmul_rn(A.dt0, A.su[o]));
-        float y = __fsub_rn((float)i, __fmul_rn(A.dt0, A.sv[o]));
-        x = (x < hi) ? x : hi;
-        x = (1.5f < x) ? x : 1.5f;
-        y = (y < hi) ? y : hi;
-        y = (1.5f < y) ? y : 1.5f;
-        const int j0 = (int)x, i0 = (int)y;
-        const float s0 = __fsub_rn(x, (float)j0), s1 = __fsub_rn(1.f, s0);
-        const float s2 = __fsub_rn(y, (float)i0), s3 = __fsub_rn(1.f, s2);
-        const size_t a = (size_t)i0 * P + j0;
-        for (int k = 0; k < 2; ++k) {
-            const float* g0 = k == 0 ? A.su : A.sv;
-            const float top = __fadd_rn(__fmul_rn(s1, g0[a]), __fmul_rn(s0, g0[a + 1]));
-            const float bot = __fadd_rn(__fmul_rn(s1, g0[a + P]), __fmul_rn(s0, g0[a + P + 1]));
-            A.f[1 + k][o] = __fadd_rn(__fmul_rn(s3, top), __fmul_rn(s2, bot));
-        }
-    }
+// Columns between a sweep and the next, in whole chunks: the next chunk's loads need two
+// chunks and one column.
+// With a CTA per band the previous sweep must also have come back from the band below, two
+// trips between SMs away. Between bands of one CTA: the band above must be a chunk past the
+// column above.
+constexpr int kLagOne = 3 * kChunk;
+constexpr int kLagMany = 5 * kChunk;
+constexpr int kBandLag = 32 + kChunk;
+
+// Bands of one CTA: the grids whose arrays all fit its shared memory.
+bool one_cta(int n) {
+    const int bands = (n - 2 + 31) / 32;
+    return bands <= 6 && 2 * bands * array_bytes(n) <= (size_t)smem_limit();
 }
 
-// The splat by target (gs_splat_gather) over every target block; when some source
-// moves more than kGatherMaxDTiled cells, one CTA applies the contributions in the raster
-// order of their sources into the global accumulator instead.
-constexpr int kGatherMaxDTiled = 40;
-__global__ void __launch_bounds__(kGsThreads) gs_splat_grid_kernel(const GsArgs A) {
-    const float dm = fmaxf(__ldcg(A.dmax), __ldcg(A.dmax + 1));
-    if (dm <= (float)kGatherMaxDTiled) {
-        gs_splat_gather(A, blockIdx.x, (int)ceilf(dm));
-        return;
-    }
-    if (blockIdx.x != 0) return;
-    const int n = A.n, P = A.P, m = n - 2;
-    for (int e = threadIdx.x; e < m * m; e += blockDim.x) A.acc[(size_t)(1 + e / m) * P + 1 + e % m] = 0.f;
-    __syncthreads();
-    if (threadIdx.x != 0) return;
-    const float hi = (float)n - 1.5f;
-    for (int i = 1; i < n - 1; ++i)
-        for (int j = 1; j < n - 1; ++j) {
-            const size_t o = (size_t)i * P + j;
-            const float x = __fadd_rn((float)j, __fmul_rn(A.dt0, A.su[o]));
-            const float y = __fadd_rn((float)i, __fmul_rn(A.dt0, A.sv[o]));
-            if (!(x >= 0.5f && x <= hi && y >= 0.5f && y <= hi)) continue;
-            const int j0 = (int)x, i0 = (int)y;
-            const float s0 = __fsub_rn(x, (float)j0), s1 = __fsub_rn(1.f, s0);
-            const float s2 = __fsub_rn(y, (float)i0), s3 = __fsub_rn(1.f, s2);
-            const float w = A.f[0][o];
-            float* t = A.acc + (size_t)i0 * P + j0;
-            // the accumulator's edge cells are never read back (the density takes its
-            // interior, then the fill), so every target can be added to
-            t[0] = __fadd_rn(t[0], __fmul_rn(__fmul_rn(s1, s3), w));
-            t[P] = __fadd_rn(t[P], __fmul_rn(__fmul_rn(s1, s2), w));
-            t[1] = __fadd_rn(t[1], __fmul_rn(__fmul_rn(s0, s3), w));
-            t[P + 1] = __fadd_rn(t[P + 1], __fmul_rn(__fmul_rn(s0, s2), w));
-        }
-}
-
-// d = the splat result on the interior (the fill follows).
-__global__ void gs_take_acc_kernel(const GsArgs A) {
-    const int n = A.n, P = A.P, m = n - 2;
-    for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < (long)m * m; e += (long)gridDim.x * blockDim.x) {
-        const size_t o = (size_t)(1 + e / m) * P + 1 + e % m;
-        A.f[0][o] = A.acc[o];
-    }
-}
-
-int g_tiled_blocks[64] = {};  // co-resident CTAs of gs_tiled_kernel per device (set-up)
-
-cudaError_t gs_solve_tiled(const GsTiled& S, bool diff, cudaStream_t st) {
-    if (S.iters <= 0) return cudaSuccess;
-    int dev = 0;
+template <bool DIFF, int PLACE, bool ONE>
+cudaError_t launch_solve(GsSolve& S, cudaStream_t st) {
+    S.bands = (S.n - 2 + 31) / 32;
+    S.band_lag = kBandLag;
+    const int in_flight = std::min(S.sweeps, kMaxWarps / S.bands);
+    const int warps = ONE ? S.bands * in_flight : S.sweeps;
+    // ONE: a warp's next sweep begins when its last one is done
+    const int per_warp = (gs_lines(S.n - 2) / kChunk + in_flight - 1) / in_flight * kChunk;
+    S.lag = ONE ? std::max(kLagOne, per_warp) : kLagMany;
+    const size_t smem = (PLACE == GS_GLOBAL ? 0 : (PLACE == GS_SHARED ? 2 : 1) * array_bytes(S.n)) * (ONE ? S.bands : 1);
+    int dev = 0, sms = 0, per = 0;
     cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess)
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, gs_solve_kernel<DIFF, PLACE, ONE>, 32 * warps, smem);
     if (e != cudaSuccess) return e;
-    const int m = S.n - 2, NT = (m + kTile - 1) / kTile;
-    const int want = NT * std::min(NT, S.iters);  // most tiles of one wavefront time
-    const int blocks = std::max(1, std::min(g_tiled_blocks[dev & 63], want));
-    e = cudaMemsetAsync(S.ctrl, 0, sizeof(SolveCtrl), st);
-    if (e != cudaSuccess) return e;
+    if (per * sms <= 0) return cudaErrorInvalidConfiguration;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(kTileThreads);
+    cfg.gridDim = dim3(std::min(per * sms, ONE ? S.nf : S.nf * S.bands));
+    cfg.blockDim = dim3(32 * warps);
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return diff ? cudaLaunchKernelEx(&cfg, gs_tiled_kernel<true>, S) : cudaLaunchKernelEx(&cfg, gs_tiled_kernel<false>, S);
+    cfg.numAttrs = ONE ? 0 : 1;  // only CTAs that wait for one another must be co-resident
+    return cudaLaunchKernelEx(&cfg, gs_solve_kernel<DIFF, PLACE, ONE>, S);
 }
 
-int grid_blocks(long work, int threads) { return (int)std::max<long>(1, std::min<long>((work + threads - 1) / threads, 4096)); }
+template <bool DIFF>
+cudaError_t launch_placed(GsSolve& S, cudaStream_t st) {
+    const size_t limit = (size_t)smem_limit(), one = array_bytes(S.n);
+    if (one_cta(S.n)) return launch_solve<DIFF, GS_SHARED, true>(S, st);
+    if (2 * one <= limit) return launch_solve<DIFF, GS_SHARED, false>(S, st);
+    if (one <= limit) return launch_solve<DIFF, GS_CONST_GLOBAL, false>(S, st);
+    return launch_solve<DIFF, GS_GLOBAL, false>(S, st);
+}
 
-// A step of the host solver's method on a grid too large for the one-CTA form: the
-// same order of operations (fluid_solver_cpu.cpp:6-31), each solve a tiled cooperative
-// launch, the rest grid-wide kernels.
-cudaError_t gs_step_tiled(const GsFields& F, const GsArgs& A, cudaStream_t st) {
-    const int n = A.n, P = A.P;
-    const long cells = (long)n * n;
-    const int B = grid_blocks(cells, 256);
-    const int modes[3] = {BND_CONT, BND_OPP_H, BND_OPP_V};
-    float* x0 = F.scratch[2];  // the divergence's buffer doubles as the diffusion's x0
-    float* p = F.scratch[4];
-    cudaError_t e = cudaMemsetAsync(A.dmax, 0, 2 * sizeof(float), st);
-    if (e != cudaSuccess) return e;
-    gs_copy_vel_kernel<<<B, 256, 0, st>>>(A);
-    auto diffuse = [&](int k) -> cudaError_t {
-        gs_add_copy_kernel<<<B, 256, 0, st>>>(A.f[k], A.src[k], x0, n, P, A.dt);
-        GsTiled S{A.f[k], x0, n, P, A.kd, modes[k], A.a[k], A.den[k], F.ctrl, F.poll_limit};
-        cudaError_t r = gs_solve_tiled(S, true, st);
-        if (r == cudaSuccess && A.kd > 0) gs_fill_kernel<<<1, kGsThreads, 0, st>>>(A.f[k], n, P, modes[k]);
-        return r == cudaSuccess ? cudaGetLastError() : r;
-    };
-    auto project = [&]() -> cudaError_t {
-        gs_div_kernel<<<B, 256, 0, st>>>(A, p);
-        GsTiled S{p, A.dv, n, P, A.kp, BND_CONT, 0.f, 0.f, F.ctrl, F.poll_limit};
-        cudaError_t r = gs_solve_tiled(S, false, st);
-        if (r != cudaSuccess) return r;
-        if (A.kp > 0) gs_fill_kernel<<<1, kGsThreads, 0, st>>>(p, n, P, BND_CONT);
-        gs_remove_p_kernel<<<B, 256, 0, st>>>(A, p);
-        gs_fill_kernel<<<1, kGsThreads, 0, st>>>(A.f[1], n, P, BND_OPP_H);
-        gs_fill_kernel<<<1, kGsThreads, 0, st>>>(A.f[2], n, P, BND_OPP_V);
-        return cudaGetLastError();
-    };
-    if ((e = diffuse(0)) != cudaSuccess) return e;
-    const int target_blocks = (int)(((long)(n - 2) * (n - 2) + kGsThreads - 1) / kGsThreads);
-    gs_splat_grid_kernel<<<target_blocks, kGsThreads, 0, st>>>(A);
-    gs_take_acc_kernel<<<B, 256, 0, st>>>(A);
-    gs_fill_kernel<<<1, kGsThreads, 0, st>>>(A.f[0], n, P, BND_CONT);
-    if ((e = diffuse(1)) != cudaSuccess) return e;
-    if ((e = diffuse(2)) != cudaSuccess) return e;
-    if ((e = project()) != cudaSuccess) return e;
-    gs_copy_vel_kernel<<<B, 256, 0, st>>>(A);  // copies for the velocity advection
-    gs_gather_grid_kernel<<<B, 256, 0, st>>>(A);
-    gs_fill_kernel<<<1, kGsThreads, 0, st>>>(A.f[1], n, P, BND_OPP_H);
-    gs_fill_kernel<<<1, kGsThreads, 0, st>>>(A.f[2], n, P, BND_OPP_V);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    return project();
+// All sweeps of a solve, kMaxWarps to a launch where a warp runs one sweep.
+cudaError_t solve(GsSolve S, bool diff, int sweeps, unsigned& epoch, cudaStream_t st, int* launches) {
+    const int most = one_cta(S.n) ? sweeps : kMaxWarps;
+    for (int done = 0; done < sweeps;) {
+        S.sweeps = std::min(most, sweeps - done);
+        S.epoch = ++epoch;
+        for (int k = 0; k < S.nf; ++k) S.f[k].start = done > 0 ? S.f[k].out : nullptr;
+        const cudaError_t e = diff ? launch_placed<true>(S, st) : launch_placed<false>(S, st);
+        if (e != cudaSuccess) return e;
+        ++*launches;
+        done += S.sweeps;
+    }
+    return cudaSuccess;
 }
 
 }  // namespace
 
-int gs_max_size() {
-    int dev = 0, smem = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-    if (cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return 0;
+int gs_one_cta_size() {
     int n = 3;
-    while (gs_smem_bytes(n + 1) <= (size_t)smem) ++n;
+    while (one_cta(n + 1)) ++n;
     return n;
 }
 
-int gs_tiled_max_size() { return 16384; }
+int gs_tiled_max_size() { return smem_limit() > 0 ? 16384 : 0; }
 
 cudaError_t gs_prepare() {
-    // the largest size, so that handles of different sizes share one setting
-    const int n = gs_max_size();
-    if (n < 3) return cudaErrorNoDevice;
-    {
-        int dev = 0, sms = 0, per = 0;
-        cudaError_t r = cudaGetDevice(&dev);
-        if (r == cudaSuccess) r = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (r == cudaSuccess)
-            r = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, gs_tiled_kernel<true>, kTileThreads, 0);
-        int per2 = 0;
-        if (r == cudaSuccess)
-            r = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per2, gs_tiled_kernel<false>, kTileThreads, 0);
-        if (r != cudaSuccess) return r;
-        g_tiled_blocks[dev & 63] = std::min(per, per2) * sms;
-    }
-    const int bytes = (int)gs_smem_bytes(n);
-    cudaError_t e = cudaFuncSetAttribute(gs_diffuse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(gs_splat_project_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(gs_project_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    const int bytes = smem_limit();
+    if (bytes <= 0) return cudaErrorNoDevice;
+    constexpr auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(gs_solve_kernel<true, GS_SHARED, false>, attr, bytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gs_solve_kernel<false, GS_SHARED, false>, attr, bytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gs_solve_kernel<true, GS_SHARED, true>, attr, bytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gs_solve_kernel<false, GS_SHARED, true>, attr, bytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gs_solve_kernel<true, GS_CONST_GLOBAL, false>, attr, bytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(gs_solve_kernel<false, GS_CONST_GLOBAL, false>, attr, bytes);
     return e;
 }
 
-cudaError_t gs_step(const GsFields& F, int n, int pitch, int kd, int kp, float diff, float visc, float dt,
+// A step in the host solver's order (fluid_solver_cpu.cpp:6-31). The state keeps the step's
+// initial velocity until the last launch, so the density's splat runs on the side stream
+// beside the projections.
+cudaError_t gs_step(const GsFields& G, int n, int pitch, int kd, int kp, float diff, float visc, float dt,
                     cudaStream_t st, int* launches) {
-    GsArgs A;
-    A.f[0] = F.d;
-    A.f[1] = F.u;
-    A.f[2] = F.v;
-    A.src[0] = F.ds;
-    A.src[1] = F.us;
-    A.src[2] = F.vs;
-    A.su = F.scratch[0];
-    A.sv = F.scratch[1];
-    A.dv = F.scratch[2];
-    A.acc = F.scratch[3];
-    A.dmax = F.aux;
-    A.n = n;
-    A.P = pitch;
-    A.kd = kd;
-    A.kp = kp;
+    *launches = 0;
     // constants as the host solver computes them, in float (fluid_solver_cpu.cpp:97-98,
     // 119, 181): a = dt * (rows*cols) * rate, den = 1 + 4a, dt0 = sqrt(rows*cols) * dt
     const float cells = (float)((size_t)n * (size_t)n);
+    const float h = 1.0f / sqrtf(cells), dt0 = sqrtf(cells) * dt;
+    cudaError_t e;
+#define GS_CK(call) \
+    if ((e = (call)) != cudaSuccess) return e
+    GsSolve S{};
+    S.n = n;
+    S.P = pitch;
+    S.dt = dt;
+    S.cdiv = -0.5f * h;
+    S.ctrl = G.ctrl;
+    S.poll_limit = G.poll_limit;
+    // the words' tags and the splat's overflow flag start at zero, the lists empty
+    int* many = reinterpret_cast<int*>(G.words);
+    S.words = reinterpret_cast<unsigned long long*>(G.words) + 32;
+    const int max_bands = (n - 2 + 31) / 32;
+    GS_CK(cudaMemsetAsync(G.words, 0, 256 + (size_t)3 * max_bands * 2 * (n - 2) * 8, st));
+    GS_CK(cudaMemsetAsync(G.ctrl, 0, sizeof(SolveCtrl), st));
+    const int modes[3] = {BND_CONT, BND_OPP_H, BND_OPP_V};
     const float rates[3] = {diff, visc, visc};
     for (int k = 0; k < 3; ++k) {
-        A.a[k] = dt * cells * rates[k];
-        A.den[k] = 1.f + 4.f * A.a[k];  // 4a is exact, so a fused form rounds the same
+        GsField& F = S.f[k];
+        F.x = G.state[k];
+        F.src = G.src[k];
+        F.out = G.dif[k];
+        F.big = G.big[k];
+        F.mode = modes[k];
+        F.a = dt * cells * rates[k];
+        F.den = 1.f + 4.f * F.a;  // 4a is exact, so a fused form rounds the same
+        F.rden = F.den > 0x1p-20f && F.den < 0x1p20f ? 1.f / F.den : 0.f;
     }
-    A.dt = dt;
-    A.dt0 = sqrtf(cells) * dt;
-    A.h = 1.0f / sqrtf(cells);
-    if (n > gs_max_size()) {
-        *launches = 29;
-        return gs_step_tiled(F, A, st);
+    unsigned epoch = 0;
+    S.nf = 3;
+    if (kd == 0) {
+        gs_add_kernel<<<dim3(std::min(4096, (n * n + 255) / 256), 3), 256, 0, st>>>(S);
+        GS_CK(cudaGetLastError());
+        ++*launches;
+    } else if (array_bytes(n) <= (size_t)smem_limit()) {
+        GS_CK(solve(S, true, kd, epoch, st, launches));
+    } else {
+        // both band arrays in global memory: one field at a time in all of the scratch
+        for (int k = 0; k < 3; ++k) {
+            GsSolve one = S;
+            one.nf = 1;
+            one.f[0] = S.f[k];
+            one.f[0].big = G.big[0];
+            GS_CK(solve(one, true, kd, epoch, st, launches));
+        }
     }
-    *launches = 4;
-    const size_t smem = gs_smem_bytes(n);
-    gs_diffuse_kernel<<<3, kGsThreads, smem, st>>>(A);
-    const int target_blocks = ((n - 2) * (n - 2) + kGsThreads - 1) / kGsThreads;
-    gs_splat_project_kernel<<<2 + target_blocks, kGsThreads, smem, st>>>(A);
-    gs_gather_kernel<<<2, kGsThreads, 0, st>>>(A);
-    gs_project_kernel<<<1, kGsThreads, smem, st>>>(A);
-    return cudaGetLastError();
+    const dim3 cells2((n + 31) / 32, (n + 7) / 8), threads(32, 8);
+    // density on the side stream
+    GS_CK(cudaEventRecord(G.fork, st));
+    GS_CK(cudaStreamWaitEvent(G.side, G.fork, 0));
+    const GsSplat A{G.dif[0], G.state[1], G.state[2], G.state[0], G.head, G.next, many, n, pitch, dt0};
+    GS_CK(cudaMemsetAsync(G.head, 0xff, (size_t)n * pitch * sizeof(int), G.side));
+    gs_link_kernel<<<cells2, threads, 0, G.side>>>(A);
+    gs_splat_kernel<<<cells2, threads, 0, G.side>>>(A);
+    gs_splat_in_order_kernel<<<1, 1024, 0, G.side>>>(A);
+    GS_CK(cudaGetLastError());
+    *launches += 3;
+    GS_CK(cudaEventRecord(G.join, G.side));
+    // velocity
+    auto project = [&](const float* u, const float* v, float* uo, float* vo) -> cudaError_t {
+        GsSolve Q = S;
+        Q.nf = 1;
+        Q.f[0] = GsField{};
+        Q.f[0].u = u;
+        Q.f[0].v = v;
+        Q.f[0].out = G.p;
+        Q.f[0].big = G.big[0];
+        Q.f[0].mode = BND_CONT;
+        if (kp == 0) {
+            GS_CK(cudaMemsetAsync(G.p, 0, (size_t)n * pitch * sizeof(float), st));
+        } else {
+            GS_CK(solve(Q, false, kp, epoch, st, launches));
+        }
+        if (uo == G.state[1]) GS_CK(cudaStreamWaitEvent(st, G.join, 0));
+        gs_remove_p_kernel<<<cells2, threads, 0, st>>>(GsVel{u, v, G.p, uo, vo, n, pitch, h, dt0});
+        ++*launches;
+        return cudaGetLastError();
+    };
+    GS_CK(project(G.dif[1], G.dif[2], G.vel[0], G.vel[1]));
+    gs_gather_kernel<<<cells2, threads, 0, st>>>(GsVel{G.vel[0], G.vel[1], nullptr, G.dif[1], G.dif[2], n, pitch, h, dt0});
+    ++*launches;
+    return project(G.dif[1], G.dif[2], G.state[1], G.state[2]);
+#undef GS_CK
 }
 
 }  // namespace fs

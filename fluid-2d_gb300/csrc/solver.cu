@@ -888,19 +888,26 @@ int enqueue_velocity_tail(fs_solver* s, const float* dif_u, const float* dif_v, 
 int enqueue_step(fs_solver* s, float diff, float visc, float dt, Counter& cnt) {
     int rc;
     if (s->cfg.method == FS_METHOD_GAUSS_SEIDEL) {
+        // the scratch fields follow one another from x0[0] on
         GsFields F;
-        F.d = s->st[F_D];
-        F.u = s->st[F_U];
-        F.v = s->st[F_V];
-        F.ds = s->src[F_D];
-        F.us = s->src[F_U];
-        F.vs = s->src[F_V];
-        for (int k = 0; k < 3; ++k) F.scratch[k] = s->x0[k];
-        F.scratch[3] = s->acc;
-        F.scratch[4] = s->p[0];
-        F.aux = s->div;  // unused by this method
+        auto scratch = [&](int k) { return s->x0[0] + (size_t)k * s->field_floats; };
+        for (int k = 0; k < 3; ++k) {
+            F.state[k] = s->st[k];
+            F.src[k] = s->src[k];
+            F.big[k] = scratch(2 * k);
+            F.dif[k] = scratch(6 + k);
+        }
+        F.vel[0] = scratch(9);
+        F.vel[1] = scratch(10);
+        F.p = scratch(11);
+        F.head = reinterpret_cast<int*>(scratch(12));
+        F.next = reinterpret_cast<int*>(scratch(13));
+        F.words = scratch(14);
         F.ctrl = s->ctrl;
         F.poll_limit = reinterpret_cast<const unsigned*>(s->flags + 1);
+        F.side = s->side;
+        F.fork = s->side_ev[0];
+        F.join = s->side_ev[1];
         int launches = 0;
         CK(gs_step(F, s->rows, s->pitch, s->cfg.diffuse_iterations, s->cfg.pressure_iterations, diff, visc, dt,
                    s->stream, &launches));
@@ -1022,7 +1029,7 @@ int check_flags(fs_solver* s) {
         }
     }
     // the tiled Gauss-Seidel solves' grid barriers (control block 0), once per step
-    if (s->cfg.method == FS_METHOD_GAUSS_SEIDEL && s->rows > gs_max_size() && s->stats.steps > 0 &&
+    if (s->cfg.method == FS_METHOD_GAUSS_SEIDEL && s->rows > gs_one_cta_size() && s->stats.steps > 0 &&
         s->steps_reported != s->stats.steps) {
         s->steps_reported = s->stats.steps;
         SolveCtrl c[2];
@@ -1344,7 +1351,7 @@ int fs_create(const fs_config* cfg, fs_solver** out) {
 
 int fs_gauss_seidel_max_size(int* n) {
     if (!n) return fail(FS_ERR_ARG, "fs_gauss_seidel_max_size: null argument");
-    *n = gs_max_size() > 0 ? gs_tiled_max_size() : 0;
+    *n = gs_tiled_max_size();
     return *n > 0 ? FS_OK : fail(FS_ERR_CUDA, "fs_gauss_seidel_max_size: no CUDA device");
 }
 
