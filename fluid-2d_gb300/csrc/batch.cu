@@ -82,7 +82,6 @@ struct fs_batch {
     std::vector<Lane> lanes;
     cudaEvent_t fork = nullptr;
     int n_diffuse = 0, n_project = 0;
-    bool split = false;  // projections end with a separate gradient launch
     void* d_plan = nullptr;
     size_t d_plan_bytes = 0;
     AdvectJob* d_jobs = nullptr;
@@ -138,10 +137,6 @@ int build_plan(fs_batch* b, float diff, float visc, float dt) {
     const std::vector<int> pplan = plan_passes(b->cfg.pressure_iterations, K);
     b->n_diffuse = (int)dplan.size();
     b->n_project = (int)pplan.size();
-    // multi-pass projections end with an ordinary pass and a separate gradient launch (the
-    // fused gradient epilogue's loads and stores made the last pass ~1.6x a middle one)
-    const bool split = b->n_project >= 2;
-    b->split = split;
     const int dkinds[3][5] = {{K_ST_D, K_SRC_D, K_X0_D, K_PP_D0, K_PP_D1},
                               {K_ST_U, K_SRC_U, K_X0_U, K_PP_U0, K_PP_U1},
                               {K_ST_V, K_SRC_V, K_X0_V, K_PP_V0, K_PP_V1}};
@@ -168,7 +163,7 @@ int build_plan(fs_batch* b, float diff, float visc, float dt) {
                     if (pass == 0) {
                         f.kind = PASS_DIFFUSE_FIRST;
                         f.x2 = b->fld(k[1], g);
-                        f.cst_out = b->fld(k[2], g);
+                        f.cst_out = dplan.size() > 1 ? b->fld(k[2], g) : nullptr;
                     } else {
                         f.kind = PASS_DIFFUSE;
                         f.cst = b->fld(k[2], g);
@@ -180,46 +175,36 @@ int build_plan(fs_batch* b, float diff, float visc, float dt) {
         // ---- two projections over the lane's grids (one pressure field each)
         for (int proj = 0; proj < 2; ++proj) {
             for (int pass = 0; pass < b->n_project; ++pass) {
-                const bool last = pass == b->n_project - 1;
                 std::vector<StencilField> fl;
                 for (int g : L.grids) {
                     StencilField f{};
+                    // a region's border columns have no divergence of their own
                     field_tiling(f, b->rows[g], b->cols[g], b->pitch[g], b->tile_rows,
-                                   pplan[pass] + (last && !split ? 1 : 0));
-                    const float h = grid_spacing(b->rows[g], b->cols[g]);
+                                 std::max(pplan[pass], pass == 0 ? 1 : 0));
                     f.s_lr = f.s_tb = 1.f;
                     f.sweeps = pplan[pass];
-                    f.cdiv = -0.5f * h;
-                    f.h = h;
+                    f.cdiv = -0.5f * grid_spacing(b->rows[g], b->cols[g]);
                     const float* uin = proj == 0 ? b->fld(K_PP_U0 + dlast, g) : b->fld(K_VEL_U, g);
                     const float* vin = proj == 0 ? b->fld(K_PP_V0 + dlast, g) : b->fld(K_VEL_V, g);
                     if (pass == 0) {
                         f.kind = PASS_PRESSURE_FIRST;
                         f.x = uin;
                         f.x2 = vin;
-                        f.cst_out = b->fld(K_DIV, g);
+                        f.cst_out = b->n_project > 1 ? b->fld(K_DIV, g) : nullptr;
                     } else {
                         f.kind = PASS_PRESSURE;
                         f.x = b->fld(K_P0 + ((pass - 1) & 1), g);
                         f.cst = b->fld(K_DIV, g);
                     }
-                    f.y = last && !split ? nullptr : b->fld(K_P0 + (pass & 1), g);
-                    if (last && !split) {
-                        f.epilogue = 1;
-                        f.u_in = uin;
-                        f.v_in = vin;
-                        f.u_out = b->fld(K_ST_U, g);
-                        f.v_out = b->fld(K_ST_V, g);
-                        f.nonfinite = b->cfg.check_finite ? b->flags : nullptr;
-                    }
+                    f.y = b->fld(K_P0 + (pass & 1), g);
                     fl.push_back(f);
                 }
                 L.passes.push_back(add_pass(b, fl, false));
             }
         }
-        // ---- advection jobs: splat, finish, velocity backtrace; with multi-pass
-        // projections, the gradient subtract of each projection (gradient_batch_kernel)
-        for (int op = 0; op < (split ? 5 : 3); ++op) {
+        // ---- advection jobs: splat, finish, velocity backtrace, and the gradient subtract
+        // of each projection (gradient_batch_kernel)
+        for (int op = 0; op < 5; ++op) {
             L.job_off[op] = b->h_jobs.size();
             L.jprefix_off[op] = b->h_jprefix.size();
             L.jmap_off[op] = b->h_map.size();
@@ -307,7 +292,6 @@ int enqueue_lane(fs_batch* b, const fs_batch::Lane& L, int& launches) {
                               b->d_map + L.jmap_off[1], L.job_blocks[1], nf, st));
     launches += 2;
     auto gradient = [&](int op) {
-        if (!b->split) return cudaSuccess;
         launches++;
         return launch_gradient_batch(b->d_jobs + L.job_off[op], b->d_jprefix + L.jprefix_off[op],
                                      b->d_map + L.jmap_off[op], L.job_blocks[op], nf, st);
@@ -519,10 +503,10 @@ int fs_batch_step(fs_batch* b, float diffusion_rate, float viscosity, float dt, 
             b->graph = g;
             FS_CK(cudaGraphInstantiate(&b->gexec, g, 0));
         } else {
-            // stencil launches + three advection launches (+ two gradient launches), per lane
+            // stencil launches + three advection and two gradient launches, per lane
             for (const fs_batch::Lane& L : b->lanes) {
                 for (const fs_batch::Pass& P : L.passes) launches += P.count;
-                launches += 3 + (b->split ? 2 : 0);
+                launches += 5;
             }
         }
         b->launches_per_step = launches;

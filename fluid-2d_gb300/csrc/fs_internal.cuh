@@ -38,29 +38,20 @@ struct StencilField {
     const float* x2;    // sources s (diffuse first) or v (pressure first)
     const float* cst;   // x0 (diffuse) or div (pressure) for non-first passes
     // outputs
-    float* y;           // state out (x or p); may be null for a last pressure pass
+    float* y;           // state out (x or p); null: none (a pass of no sweeps)
     float* cst_out;     // first pass: x0 or div out
-    // gradient-subtract epilogue (last pressure pass): u,v in -> out
-    const float* u_in;
-    const float* v_in;
-    float* u_out;
-    float* v_out;
     // constants
     float a, rh, rl;      // diffuse: a and the FP32 pair for 1/(1+4a) (see stencil.cu)
     float dt;             // add_sources
     float cdiv;           // divergence factor -0.5f*h
-    float h;              // gradient divisor
     float s_lr, s_tb;     // boundary signs of this field
     int kind;             // PassKind
     int sweeps;           // Jacobi sweeps in this pass
-    int epilogue;         // 1: gradient subtract + velocity fills after the sweeps
     int halo;             // H: a region's margin around its output tile (field_tiling)
     int rows, cols, pitch;
     int tile_w, tile_h, tiles_x, tiles_y;
     int gx_last, gy_last; // first column and row of the last regions
-    int caller_rows;      // 1: u_out, v_out are a caller's buffers, their row padding is not written
     int tile_begin;       // first block index of this field in the launch
-    int* nonfinite;       // optional flag (epilogue outputs)
 };
 
 constexpr int kMaxStencilFields = 4;

@@ -105,25 +105,23 @@ extern "C" int fs_project_noalloc(const float* u, const float* v, float* u_out, 
     float* pbuf[2] = {base + kCells, base + 2 * kCells};
     cudaStream_t st = static_cast<cudaStream_t>(stream);
 
-    // Same plan as a handle's projection: depth-8 temporally blocked passes over
-    // 64-row regions, divergence fused into the first pass, gradient subtract and
-    // reflecting fills into the last.
+    // Same plan as a handle's projection: depth-8 temporally blocked passes over 64-row
+    // regions, divergence fused into the first pass, then the gradient subtract and the
+    // reflecting fills. The scratch has the caller's pitch; row padding of the caller's
+    // outputs is not written.
     const int depth = 8, tile_rows = 64;
     const int m = std::max(1, (iterations + depth - 1) / depth);
     std::vector<int> plan(m, iterations / m);
     for (int i = 0; i < iterations % m; ++i) plan[i] += 1;
     const float h = 1.0f / sqrtf((float)((size_t)rows * (size_t)cols));
     for (int pass = 0; pass < m; ++pass) {
-        const bool last = pass == m - 1;
         StencilLaunch L{};
         L.nfields = 1;
         StencilField& f = L.f[0];
-        const int halo = plan[pass] + (last ? 1 : 0);
-        field_tiling(f, rows, cols, pitch, tile_rows, halo);
+        field_tiling(f, rows, cols, pitch, tile_rows, std::max(plan[pass], pass == 0 ? 1 : 0));
         f.s_lr = f.s_tb = 1.f;
         f.sweeps = plan[pass];
         f.cdiv = -0.5f * h;
-        f.h = h;
         if (pass == 0) {
             f.kind = PASS_PRESSURE_FIRST;
             f.x = u;
@@ -135,17 +133,11 @@ extern "C" int fs_project_noalloc(const float* u, const float* v, float* u_out, 
             f.x = pbuf[(pass - 1) & 1];
             f.cst = div;
         }
-        f.y = last ? nullptr : pbuf[pass & 1];
-        if (last) {
-            f.epilogue = 1;
-            f.caller_rows = 1;
-            f.u_in = u;
-            f.v_in = v;
-            f.u_out = u_out;
-            f.v_out = v_out;
-        }
+        f.y = pbuf[pass & 1];
         cudaError_t e = launch_stencil(L, tile_rows, st);
         if (e != cudaSuccess) return record_error(FS_ERR_CUDA, "fs_project_noalloc: stencil launch failed");
     }
+    if (launch_gradient(pbuf[(m - 1) & 1], u, v, u_out, v_out, rows, cols, pitch, h, nullptr, st) != cudaSuccess)
+        return record_error(FS_ERR_CUDA, "fs_project_noalloc: gradient launch failed");
     return FS_OK;
 }

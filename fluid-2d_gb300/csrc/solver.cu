@@ -176,12 +176,14 @@ struct fs_solver {
 
 namespace {
 
-// Default temporal-blocking depth (sweeps per pass). From 1024^2 up, 8 is within 3 %
-// of the best depth measured on GB300 (4 to 16 sweeps, 64- and 128-row regions). A grid
-// whose one-field pass at depth 8 fills less than half a wave of CTAs is launch-bound
-// instead: there the fewest passes win (512^2: 0.222 -> 0.205 ms per 40/40 step; 130^2:
-// 0.116 -> 0.087 ms per 20/20 step), as long as output tiles keep 16 rows. Solves to a
-// residual target keep depth 8, since their pass count is not fixed.
+// Default temporal-blocking depth (sweeps per pass), by the tiles of a one-field pass at
+// depth 8 against the CTAs resident at once (two per SM). From one wave of tiles up, 8 is
+// within 3 % of the best depth (4 to 20 sweeps, 1400^2 to 8192^2). Below, a pass costs
+// about 4 us whatever it does, so fewer and deeper passes win until the halos eat the gain:
+// depth 10 (1026^2, 40/40 sweeps: 184 -> 176 us per step; 771x1283, 15/20: 99 -> 90), and
+// below a quarter of a wave the fewest passes whose output tiles keep 16 rows (514^2, 15/20:
+// 64 -> 50; 130^2: 58 -> 41; 800^2, 40/40, above the line: 146 against 121 at depth 10).
+// Solves to a residual target keep depth 8, since their pass count is not fixed.
 int default_sweeps(const fs_config* cfg, int dev, int maxk) {
     const int k8 = std::min(8, maxk);
     if (cfg->pressure_tolerance > 0.f) return k8;
@@ -189,13 +191,12 @@ int default_sweeps(const fs_config* cfg, int dev, int maxk) {
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return k8;
     const int slots = sms * (tr <= 64 ? 2 : 1);
-    auto tiles = [&](int halo) {
-        const long tw = kRegionW - 2 * halo, th = tr - 2 * halo;
-        return ((cfg->cols + tw - 1) / tw) * ((cfg->rows + th - 1) / th);
-    };
-    if (2 * tiles(k8 + 1) >= slots) return k8;
+    StencilField f{};
+    field_tiling(f, cfg->rows, cfg->cols, cfg->cols, tr, k8);
+    const long tiles = (long)f.tiles_x * f.tiles_y;
+    if (tiles >= slots) return k8;
     const int kmax = std::min(maxk, (tr - 16) / 2 - 1);
-    if (kmax <= k8) return k8;
+    if (4 * tiles >= slots || kmax <= k8) return std::min(10, maxk);
     const int total = std::max(cfg->diffuse_iterations, cfg->pressure_iterations);
     const int passes = std::max(1, (total + kmax - 1) / kmax);
     return std::max(k8, (total + passes - 1) / passes);
@@ -330,7 +331,7 @@ int enqueue_diffuse(fs_solver* s, const int* fields, int nf, const float* rates,
             if (pass == 0) {
                 f.kind = PASS_DIFFUSE_FIRST;
                 f.x2 = s->src[fid];
-                f.cst_out = s->x0[fid];
+                f.cst_out = plan.size() > 1 ? s->x0[fid] : nullptr;
             } else {
                 f.kind = PASS_DIFFUSE;
                 f.cst = s->x0[fid];
@@ -382,7 +383,6 @@ int enqueue_div_pass(fs_solver* s, const float* u_in, const float* v_in, Counter
     f.kind = PASS_PRESSURE_FIRST;
     f.sweeps = 0;
     f.cdiv = -0.5f * h;
-    f.h = h;
     f.x = u_in;
     f.x2 = v_in;
     f.cst_out = s->div;
@@ -567,7 +567,6 @@ int enqueue_project_learned_cycles(fs_solver* s, const float* u_in, const float*
     set_geometry(P.mid, s, K + 1);
     P.mid.s_lr = P.mid.s_tb = 1.f;
     P.mid.sweeps = K;
-    P.mid.h = grid_h(s->rows, s->cols);
     P.mid.kind = PASS_PRESSURE;
     P.mid.cst = s->div;
     P.first = P.mid;
@@ -630,7 +629,6 @@ int enqueue_project_learned_defect(fs_solver* s, const float* u_in, const float*
     set_geometry(P.mid, s, K + 1);
     P.mid.s_lr = P.mid.s_tb = 1.f;
     P.mid.sweeps = K;
-    P.mid.h = grid_h(s->rows, s->cols);
     P.mid.kind = PASS_PRESSURE;
     P.mid.cst = s->rhs;
     P.first = P.mid;
@@ -710,7 +708,6 @@ int enqueue_project_to_residual(fs_solver* s, const float* u_in, const float* v_
         f->s_lr = f->s_tb = 1.f;
         f->sweeps = K;
         f->cdiv = -0.5f * h;
-        f->h = h;
     }
     const float* pin = nullptr;
     int rc = projection_start(s, u_in, v_in, slot, cnt, &pin);
@@ -755,55 +752,41 @@ int enqueue_project(fs_solver* s, const float* u_in, const float* v_in, float* u
     const float* pin = nullptr;
     int rc = projection_start(s, u_in, v_in, slot, cnt, &pin);
     if (rc != FS_OK) return rc;
-    // A single pass fuses the gradient subtract into its epilogue. With more passes the
-    // last is an ordinary pass that stores the final pressure (edges filled) and a separate
-    // bandwidth-bound launch subtracts the gradient (gradient_kernel): the epilogue's loads
-    // and stores, issued behind the sweeps of each tile, had made that pass twice as long
-    // as a middle one (60 against 29 us at 2048^2).
-    const bool split = m >= 2;
+    // The passes end with the final pressure (edges filled) and a separate bandwidth-bound
+    // launch subtracts the gradient. Fused into the last pass it had cost more at every size:
+    // behind each tile's sweeps it made a 2048^2 pass 60 us instead of 29, and at 130^2, where
+    // one pass holds a solve, its straight-line code (4500 instructions run once by each warp)
+    // took 35 of the pass's 45 us to fetch, against a 3 us launch.
     float* pfinal = nullptr;
     for (int pass = 0; pass < m; ++pass) {
         const bool last = pass == m - 1;
-        const bool fused = last && !split;
         StencilLaunch L{};
         L.nfields = 1;
         StencilField& f = L.f[0];
-        set_geometry(f, s, plan[pass] + (fused ? 1 : 0));
+        // a region's border columns have no divergence of their own
+        set_geometry(f, s, std::max(plan[pass], pass == 0 ? 1 : 0));
         f.s_lr = f.s_tb = 1.f;
         f.sweeps = plan[pass];
         f.cdiv = -0.5f * h;
-        f.h = h;
-        float* pout = s->p[pass & 1];
-        if (last && split && warm) pout = s->pwarm[slot];
-        if (fused) pout = warm ? s->p[0] : nullptr;
+        // a single pass reads its start (pwarm) beside the tiles it writes: not in place
+        float* pout = last && warm && m > 1 ? s->pwarm[slot] : s->p[pass & 1];
         if (last) pfinal = pout;
         if (pass == 0) {
             f.kind = PASS_PRESSURE_FIRST;
             f.x = u_in;
             f.x2 = v_in;
             f.cst = pin;  // starting pressure (null: zero, as the reference)
-            f.cst_out = s->div;
+            f.cst_out = m > 1 || s->cfg.capture ? s->div : nullptr;
         } else {
             f.kind = PASS_PRESSURE;
             f.x = s->p[(pass - 1) & 1];
             f.cst = s->div;
         }
         f.y = pout;
-        if (fused) {
-            f.epilogue = 1;
-            f.u_in = u_in;
-            f.v_in = v_in;
-            f.u_out = u_out;
-            f.v_out = v_out;
-            f.nonfinite = s->cfg.check_finite ? s->flags : nullptr;
-        }
-        // 12 B/cell per sweep (read p and div, write p), + 12 divergence, + 20 gradient;
-        // the pass itself reads p and div (first: u and v, and p when warm) and writes p
-        // (first: and div; a fused last pass: u and v instead of p)
-        const double bytes =
-            interior_cells(s) * (12.0 * plan[pass] + (pass == 0 ? 12.0 : 0.0) + (fused ? 20.0 : 0.0));
-        const double pass_bytes =
-            interior_cells(s) * ((pass == 0 ? 8.0 + (pin ? 4.0 : 0.0) + 4.0 : 8.0) + (fused ? 16.0 : 4.0));
+        // 12 B/cell per sweep (read p and div, write p), + 12 divergence; the pass itself
+        // reads p and div (first: u and v, and p when warm) and writes p (first: and div)
+        const double bytes = interior_cells(s) * (12.0 * plan[pass] + (pass == 0 ? 12.0 : 0.0));
+        const double pass_bytes = interior_cells(s) * ((pass == 0 ? 8.0 + (pin ? 4.0 : 0.0) + 4.0 : 8.0) + 4.0);
         PROF_BEGIN(s);
         CK(launch_stencil(L, s->tile_rows, s->stream));
         PROF_END_PASS(s, s->stream, FS_KIND_STENCIL, bytes, pass_bytes);
@@ -811,18 +794,10 @@ int enqueue_project(fs_solver* s, const float* u_in, const float* v_in, float* u
         cnt.passes++;
         if (pass == 0 && (rc = capture_div(s, slot)) != FS_OK) return rc;
     }
-    if (split) {
-        // read p, u, v; write u, v
-        PROF_BEGIN(s);
-        CK(launch_gradient(pfinal, u_in, v_in, u_out, v_out, s->rows, s->cols, s->pitch, h,
-                           s->cfg.check_finite ? s->flags : nullptr, s->stream));
-        PROF_END_PASS(s, s->stream, FS_KIND_GRADIENT, interior_cells(s) * 20.0, interior_cells(s) * 20.0);
-        cnt.launches++;
-    }
-    if (warm && m == 1) {
-        CK(cudaMemcpyAsync(s->pwarm[slot], s->p[0], s->field_floats * sizeof(float), cudaMemcpyDeviceToDevice,
+    if ((rc = enqueue_fin_pass(s, pfinal, u_in, v_in, u_out, v_out, cnt)) != FS_OK) return rc;
+    if (warm && m == 1)
+        CK(cudaMemcpyAsync(s->pwarm[slot], pfinal, s->field_floats * sizeof(float), cudaMemcpyDeviceToDevice,
                            s->stream));
-    }
     return FS_OK;
 }
 

@@ -10,8 +10,8 @@
 // (its output tile grown by a halo of at least `sweeps` cells) in registers, sweeps it
 // with the boundary fill's effect reproduced exactly after every sweep, and writes only
 // its output tile back. The first pass of a solve fuses what precedes it (add_sources for
-// diffusion, the divergence for pressure) and a projection of one pass fuses the gradient
-// subtract and the two reflecting fills.
+// diffusion, the divergence for pressure); the gradient subtract and the two reflecting
+// fills follow a projection's passes as a launch of their own (gradient_kernel).
 //
 // Arithmetic follows the reference's operand order with explicit round-to-nearest
 // intrinsics and a fused multiply-add exactly where the reference's compiled kernels fuse
@@ -314,10 +314,6 @@ __device__ __forceinline__ void store_filled(float2 (&X)[R][2], float* __restric
     }
 }
 
-// What a pass may carry besides its sweeps (the kernel's variants).
-constexpr int kModeGrad = 1;   // a fused gradient epilogue
-constexpr int kModeResid = 2;  // residual partial sums
-
 // The sweeps of one tile on its block X with constant terms K.
 template <int R, int NW, bool DIFF, bool EDGE>
 __device__ __forceinline__ void run_sweeps(float2 (&X)[R][2], const float2 (&K)[R][2], float* E0, float* E1, int n,
@@ -399,12 +395,11 @@ __device__ __forceinline__ void prefetch_tile(const StencilField& F, int b, cons
 }
 
 // One tile of one pass: load the region (fusing add_sources or the divergence into the
-// first pass), run F.sweeps sweeps, store the output tile, then the optional
-// gradient-subtract epilogue and the optional residual partial sums (for residual-driven
-// pressure solves). xin/yout stand in for F.x/F.y so a persistent caller can ping-pong
+// first pass), run F.sweeps sweeps, store the output tile, then the optional residual
+// partial sums (for residual-driven pressure solves). xin/yout stand in for F.x/F.y so a persistent caller can ping-pong
 // buffers across passes. VEC: the block comes from the prefetch, and `next` starts the next
 // tile's once it has been read.
-template <int R, int NW, bool DIFF, bool VEC, int MODE, class Next>
+template <int R, int NW, bool DIFF, bool VEC, bool RESID, class Next>
 __device__ __forceinline__ void process_tile(const StencilField& F, int b, const float* __restrict__ xin,
                                              float* __restrict__ yout, bool resid, float& rnum, float& rden,
                                              Next&& next) {
@@ -553,54 +548,12 @@ __device__ __forceinline__ void process_tile(const StencilField& F, int b, const
                 if (i >= t.r_lo && i < hi) store4<VEC>(yout + o + (size_t)i * pitch, row4(X[i]), t.ncol);
         }
     }
-    float* const E = (n & 1) ? E1 : E0;  // the exchange buffer the last sweep did not use
-
-    // ---------------------------------------------- gradient subtract epilogue
-    // remove_p_kernel (fluid_solver_gpu.cu:202-203): u -= (0.5*(pR - pL))/h, v -=
-    // (0.5*(pD - pU))/h, then set_boundary_opposite_horizontal(u) / _vertical(v)
-    // (fluid_solver_gpu.cu:402-403): an edge cell takes its inner neighbour's updated value,
-    // negated for the normal component; corners keep their input.
-    if ((MODE & kModeGrad) && F.epilogue) {
-        const float h = F.h, rhh = __frcp_rn(h);  // RN(1/h) for div_by
-        int bad = 0;
-        float2 G[R][2], V[R][2];
-        auto slope = [&](float hi, float lo) { return div_by(__fmul_rn(0.5f, __fsub_rn(hi, lo)), h, rhh); };
-        for_neighbours<R, NW, true>(X, E, t.w, t.lane, n > 0, e,
-                                    [&](int i, float l, float r, const float2 (&U)[2], const float2 (&D)[2]) {
-                                        const float2 (&x)[2] = X[i];
-                                        G[i][0] = make_float2(slope(x[0].y, l), slope(x[1].x, x[0].x));
-                                        G[i][1] = make_float2(slope(x[1].y, x[0].y), slope(r, x[1].x));
-                                        V[i][0] = make_float2(slope(D[0].x, U[0].x), slope(D[0].y, U[0].y));
-                                        V[i][1] = make_float2(slope(D[1].x, U[1].x), slope(D[1].y, U[1].y));
-                                    });
-        auto subtract = [&](float2 (&A)[R][2], const float* __restrict__ in) {
-#pragma unroll
-            for (int i = 0; i < R; ++i) {
-                const float4 x = load(in, i);
-                const float xv[4] = {x.x, x.y, x.z, x.w};
-                float r[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    const bool live = int_row(i) && int_col(q);
-                    r[q] = live ? __fsub_rn(xv[q], colval(A[i], q)) : xv[q];
-                    // edge cells repeat an interior one; the corners are outputs of their own
-                    const bool corner = i < t.nrow && q < t.ncol && !int_row(i) && !int_col(q);
-                    if ((live || corner) && t.ocol && i >= t.r_lo && i < t.r_hi) bad |= !isfinite(r[q]);
-                }
-                put(A[i], make_float4(r[0], r[1], r[2], r[3]));
-            }
-        };
-        subtract(G, F.u_in);
-        store_filled<R, VEC>(G, F.u_out, F.u_in, t, e, -1.f, 1.f, o, pitch, true);
-        subtract(V, F.v_in);
-        store_filled<R, VEC>(V, F.v_out, F.v_in, t, e, 1.f, -1.f, o, pitch, true);
-        if (bad && F.nonfinite) atomicOr(F.nonfinite, 1);
-    }
 
     // ------------------------------------------------ residual partial sums
     // ||div + sum(nbrs) - 4p||^2 and ||div||^2 over this tile's interior output cells,
     // from the final p (valid one ring beyond the tile: halo = sweeps + 1).
-    if ((MODE & kModeResid) && resid) {
+    if (RESID && resid) {
+        float* const E = (n & 1) ? E1 : E0;  // the exchange buffer the last sweep did not use
         for_neighbours<R, NW, true>(X, E, t.w, t.lane, n > 0, e,
                                     [&](int i, float l, float r, const float2 (&U)[2], const float2 (&D)[2]) {
             const bool row = t.ocol && i >= t.r_lo && i < t.r_hi && int_row(i);
@@ -702,7 +655,9 @@ __device__ __forceinline__ bool gradient_group(const float* __restrict__ p, cons
     return bad;
 }
 
-// One thread per four consecutive cells of a row (gradient_group).
+// One thread per four consecutive cells of a row: gradient_group, or for rows without
+// 16-byte alignment (VEC false) and a caller's rows cell by cell.
+template <bool VEC>
 __global__ void __launch_bounds__(256) gradient_kernel(const float* p0, const float* __restrict__ u_in,
                                                        const float* __restrict__ v_in, float* __restrict__ u_out,
                                                        float* __restrict__ v_out, int rows, int cols, int pitch,
@@ -710,7 +665,19 @@ __global__ void __launch_bounds__(256) gradient_kernel(const float* p0, const fl
     const int j0 = 4 * (blockIdx.x * 32 + threadIdx.x), i = blockIdx.y * 8 + threadIdx.y;
     if (i >= rows || j0 >= cols) return;
     const float* __restrict__ p = (sel != nullptr && __ldcg(sel) != 0) ? p_alt : p0;
-    const bool bad = gradient_group(p, u_in, v_in, u_out, v_out, i, j0, rows, cols, (size_t)pitch, h, __frcp_rn(h));
+    const float rh = __frcp_rn(h);
+    bool bad = false;
+    if (VEC) {
+        bad = gradient_group(p, u_in, v_in, u_out, v_out, i, j0, rows, cols, (size_t)pitch, h, rh);
+    } else {
+        for (int j = j0; j < min(cols, j0 + 4); ++j) {
+            float un, vn;
+            gradient_cell(p, u_in, v_in, i, j, rows, cols, (size_t)pitch, h, rh, un, vn);
+            u_out[(size_t)i * pitch + j] = un;
+            v_out[(size_t)i * pitch + j] = vn;
+            bad |= !(isfinite(un) && isfinite(vn));
+        }
+    }
     if (bad && nonfinite) atomicOr(nonfinite, 1);
 }
 
@@ -746,9 +713,8 @@ constexpr int kR = 8;
 
 // One launch = one pass over the tiles of up to kMaxStencilFields fields: persistent CTAs,
 // as many as are resident at once, each taking every gridDim.x-th tile and prefetching the
-// next one while it sweeps. VEC: 16-byte rows (see load4); single-pass projections carry
-// the gradient epilogue (GRAD).
-template <int NW, bool DIFF, bool VEC, bool GRAD>
+// next one while it sweeps. VEC: 16-byte rows (see load4).
+template <int NW, bool DIFF, bool VEC>
 __global__ void __launch_bounds__(32 * NW, (NW <= 8 ? 2 : 1))
     stencil_kernel(const __grid_constant__ StencilLaunch L, int total) {
     auto field_of = [&](int b) {
@@ -765,7 +731,7 @@ __global__ void __launch_bounds__(32 * NW, (NW <= 8 ? 2 : 1))
         const int nb = b + gridDim.x;
         const int nf = nb < total ? field_of(nb) : f;
         const StencilField& F = L.f[f];
-        process_tile<kR, NW, DIFF, VEC, GRAD ? kModeGrad : 0>(F, b - F.tile_begin, F.x, F.y, false, rn, rd, [&] {
+        process_tile<kR, NW, DIFF, VEC, false>(F, b - F.tile_begin, F.x, F.y, false, rn, rd, [&] {
             if (nb < total) prefetch_tile<kR, NW, DIFF>(L.f[nf], nb - L.f[nf].tile_begin, L.f[nf].x);
         });
         b = nb;
@@ -777,7 +743,7 @@ __global__ void __launch_bounds__(32 * NW, (NW <= 8 ? 2 : 1))
 // One pass over the fields of a batch of grids of uneven size, up to kMaxWideFields
 // of them, with their descriptors in the launch's parameters like the single-grid
 // kernel's, a tile's field found by a binary search of the fields' first tiles.
-template <int NW, bool DIFF, bool GRAD>
+template <int NW, bool DIFF>
 __global__ void __launch_bounds__(32 * NW, (NW <= 8 ? 2 : 1)) stencil_wide_kernel(const __grid_constant__ WideLaunch L) {
     auto field_of = [&](int b) {
         int lo = 0, hi = L.nfields - 1;
@@ -800,7 +766,7 @@ __global__ void __launch_bounds__(32 * NW, (NW <= 8 ? 2 : 1)) stencil_wide_kerne
         const int nb = b + gridDim.x;
         const int nf = nb < total ? field_of(nb) : f;
         const StencilField& F = L.f[f];
-        process_tile<kR, NW, DIFF, true, GRAD ? kModeGrad : 0>(F, b - L.begin[f], F.x, F.y, false, rn, rd, [&] {
+        process_tile<kR, NW, DIFF, true, false>(F, b - L.begin[f], F.x, F.y, false, rn, rd, [&] {
             if (nb < total) prefetch_tile<kR, NW, DIFF>(L.f[nf], nb - L.begin[nf], L.f[nf].x);
         });
         b = nb;
@@ -907,7 +873,7 @@ __global__ void __launch_bounds__(32 * NW, (NW <= 8 ? 2 : 1))
         if (blockIdx.x < ntiles) prefetch_tile<kR, NW, false>(F, blockIdx.x, x);
 #pragma unroll 1
         for (unsigned t = blockIdx.x; t < ntiles; t += G) {
-            process_tile<kR, NW, false, true, kModeResid>(F, t, x, P.p[dst], check, rn, rd, [&] {
+            process_tile<kR, NW, false, true, true>(F, t, x, P.p[dst], check, rn, rd, [&] {
                 if (t + G < ntiles) prefetch_tile<kR, NW, false>(F, t + G, x);
             });
             __syncthreads();  // the next tile reuses the exchange rows
@@ -979,19 +945,17 @@ template <class K> cudaError_t opt_in(K* kernel, int nw) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(nw));
 }
 template <int NW> cudaError_t prepare_variant() {
-    cudaError_t e = opt_in(stencil_kernel<NW, true, true, false>, NW);
-    if (e == cudaSuccess) e = opt_in(stencil_kernel<NW, false, true, false>, NW);
-    if (e == cudaSuccess) e = opt_in(stencil_kernel<NW, false, true, true>, NW);
-    if (e == cudaSuccess) e = opt_in(stencil_kernel<NW, false, false, true>, NW);
+    cudaError_t e = opt_in(stencil_kernel<NW, true, true>, NW);
+    if (e == cudaSuccess) e = opt_in(stencil_kernel<NW, false, true>, NW);
+    if (e == cudaSuccess) e = opt_in(stencil_kernel<NW, false, false>, NW);
     if (e == cudaSuccess) e = opt_in(pressure_solve_kernel<NW>, NW);
-    if (e == cudaSuccess) e = opt_in(stencil_wide_kernel<NW, true, false>, NW);
-    if (e == cudaSuccess) e = opt_in(stencil_wide_kernel<NW, false, true>, NW);
-    if (e == cudaSuccess) e = opt_in(stencil_wide_kernel<NW, false, false>, NW);
+    if (e == cudaSuccess) e = opt_in(stencil_wide_kernel<NW, true>, NW);
+    if (e == cudaSuccess) e = opt_in(stencil_wide_kernel<NW, false>, NW);
     return e;
 }
 
 template <int NW>
-cudaError_t launch_wide_variant(const WideLaunch& L, bool diffuse, bool grad, cudaStream_t st) {
+cudaError_t launch_wide_variant(const WideLaunch& L, bool diffuse, cudaStream_t st) {
     if (L.nfields <= 0 || L.nfields > kMaxWideFields) return cudaErrorInvalidValue;
     const int total = L.begin[L.nfields];
     if (total <= 0) return cudaSuccess;
@@ -1000,11 +964,9 @@ cudaError_t launch_wide_variant(const WideLaunch& L, bool diffuse, bool grad, cu
     if (e != cudaSuccess) return e;
     ctas = std::min(ctas, total);
     if (diffuse)
-        stencil_wide_kernel<NW, true, false><<<ctas, 32 * NW, smem_bytes(NW), st>>>(L);
-    else if (grad)
-        stencil_wide_kernel<NW, false, true><<<ctas, 32 * NW, smem_bytes(NW), st>>>(L);
+        stencil_wide_kernel<NW, true><<<ctas, 32 * NW, smem_bytes(NW), st>>>(L);
     else
-        stencil_wide_kernel<NW, false, false><<<ctas, 32 * NW, smem_bytes(NW), st>>>(L);
+        stencil_wide_kernel<NW, false><<<ctas, 32 * NW, smem_bytes(NW), st>>>(L);
     return cudaGetLastError();
 }
 
@@ -1034,11 +996,9 @@ cudaError_t launch_solve_variant(const PressureSolve& P, int blocks, cudaStream_
     return cudaLaunchKernelEx(&cfg, pressure_solve_kernel<NW>, P);
 }
 
-// 16-byte rows: every buffer of the field aligned, and the pitch; in caller-owned rows the
-// columns behind the last one are not ours to write, so there the last group must be whole.
+// 16-byte rows: every buffer of the field aligned, and the pitch.
 bool vector_rows(const StencilField& f) {
-    if (f.caller_rows && f.cols % 4 != 0) return false;
-    const void* ptrs[] = {f.x, f.x2, f.cst, f.y, f.cst_out, f.u_in, f.v_in, f.u_out, f.v_out};
+    const void* ptrs[] = {f.x, f.x2, f.cst, f.y, f.cst_out};
     uintptr_t bits = (uintptr_t)f.pitch * sizeof(float);
     for (const void* p : ptrs) bits |= reinterpret_cast<uintptr_t>(p);
     return (bits & 15) == 0;
@@ -1048,11 +1008,10 @@ template <int NW>
 cudaError_t launch_variant(const StencilLaunch& L, cudaStream_t st) {
     const size_t smem = smem_bytes(NW);
     int blocks = 0;
-    bool vec = true, grad = false;
+    bool vec = true;
     for (int i = 0; i < L.nfields; ++i) {
         blocks += L.f[i].tiles_x * L.f[i].tiles_y;
         vec = vec && vector_rows(L.f[i]);
-        grad = grad || L.f[i].epilogue;
     }
     if (blocks == 0) return cudaSuccess;
     int ctas = 0;
@@ -1060,17 +1019,15 @@ cudaError_t launch_variant(const StencilLaunch& L, cudaStream_t st) {
     if (e != cudaSuccess) return e;
     ctas = std::min(ctas, blocks);
     // all fields of one launch are of the same class (diffusion or pressure); a handle's and
-    // a batch's fields have 128-byte rows, only caller-owned buffers of a projection may not
+    // a batch's fields have 128-byte rows, only a caller's velocity may not
     const bool diff = L.f[0].kind == PASS_DIFFUSE_FIRST || L.f[0].kind == PASS_DIFFUSE;
     if (diff && !vec) return cudaErrorInvalidValue;
     if (diff)
-        stencil_kernel<NW, true, true, false><<<ctas, 32 * NW, smem, st>>>(L, blocks);
-    else if (!vec)
-        stencil_kernel<NW, false, false, true><<<ctas, 32 * NW, smem, st>>>(L, blocks);
-    else if (grad)
-        stencil_kernel<NW, false, true, true><<<ctas, 32 * NW, smem, st>>>(L, blocks);
+        stencil_kernel<NW, true, true><<<ctas, 32 * NW, smem, st>>>(L, blocks);
+    else if (vec)
+        stencil_kernel<NW, false, true><<<ctas, 32 * NW, smem, st>>>(L, blocks);
     else
-        stencil_kernel<NW, false, true, false><<<ctas, 32 * NW, smem, st>>>(L, blocks);
+        stencil_kernel<NW, false, false><<<ctas, 32 * NW, smem, st>>>(L, blocks);
     return cudaGetLastError();
 }
 
@@ -1091,13 +1048,17 @@ cudaError_t stencil_prepare() {
 cudaError_t launch_gradient(const float* p, const float* u_in, const float* v_in, float* u_out, float* v_out, int rows,
                             int cols, int pitch, float h, int* nonfinite, cudaStream_t st, const float* p_alt,
                             const int* sel) {
-    if (pitch % 4 != 0 || ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(p_alt) |
-                            reinterpret_cast<uintptr_t>(u_in) | reinterpret_cast<uintptr_t>(v_in) |
-                            reinterpret_cast<uintptr_t>(u_out) | reinterpret_cast<uintptr_t>(v_out)) & 15) != 0)
-        return cudaErrorInvalidValue;  // the handles' fields are 128-byte aligned rows
+    const bool vec = pitch % 4 == 0 &&
+                     ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(p_alt) |
+                       reinterpret_cast<uintptr_t>(u_in) | reinterpret_cast<uintptr_t>(v_in) |
+                       reinterpret_cast<uintptr_t>(u_out) | reinterpret_cast<uintptr_t>(v_out)) & 15) == 0;
     const dim3 grid(((cols + 3) / 4 + 31) / 32, (rows + 7) / 8);
-    gradient_kernel<<<grid, dim3(32, 8), 0, st>>>(p, u_in, v_in, u_out, v_out, rows, cols, pitch, h, nonfinite, p_alt,
-                                                  sel);
+    if (vec)
+        gradient_kernel<true><<<grid, dim3(32, 8), 0, st>>>(p, u_in, v_in, u_out, v_out, rows, cols, pitch, h, nonfinite,
+                                                            p_alt, sel);
+    else
+        gradient_kernel<false><<<grid, dim3(32, 8), 0, st>>>(p, u_in, v_in, u_out, v_out, rows, cols, pitch, h,
+                                                             nonfinite, p_alt, sel);
     return cudaGetLastError();
 }
 
@@ -1129,10 +1090,9 @@ cudaError_t launch_pressure_solve(const PressureSolve& P, int tile_rows, int blo
 }
 
 cudaError_t launch_stencil_wide(const WideLaunch& L, bool diffuse, int tile_rows, cudaStream_t st) {
-    bool grad = false;
-    for (int i = 0; i < L.nfields; ++i) grad = grad || L.f[i].epilogue;
-    if (tile_rows == 128) return launch_wide_variant<16>(L, diffuse, grad, st);
-    return launch_wide_variant<8>(L, diffuse, grad, st);
+
+    if (tile_rows == 128) return launch_wide_variant<16>(L, diffuse, st);
+    return launch_wide_variant<8>(L, diffuse, st);
 }
 
 }  // namespace fs
