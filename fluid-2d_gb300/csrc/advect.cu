@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(256) density_finish_kernel(const float* __rest
     for (int i = blockIdx.y * blockDim.y + threadIdx.y; i < A.rows; i += blockDim.y * gridDim.y)
         for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < A.cols; j += blockDim.x * gridDim.x)
             bad |= finish_cell(acc, d, smooth, A, i, j);
-    if (bad && nonfinite) atomicOr(nonfinite, 1);
+    if (bad && nonfinite) report_nonfinite(nonfinite);
 }
 
 __global__ void __launch_bounds__(256) advect_velocity_kernel(const float* __restrict__ u0,
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(256) advect_batch_kernel(const AdvectJob* __re
             if (i < J.A.rows && j < J.A.cols) advect_cell(J.in0, J.in1, J.out0, J.out1, J.A, i, j);
         }
     }
-    if (bad && nonfinite) atomicOr(nonfinite, 1);
+    if (bad && nonfinite) report_nonfinite(nonfinite);
 }
 
 dim3 grid_for(int rows, int cols) {

@@ -50,7 +50,8 @@ struct fs_batch {
     std::vector<size_t> off;  // per-grid offset (floats) inside each field-kind range
     size_t range_floats = 0;  // floats per field kind (all grids)
     float* slab = nullptr;
-    int* flags = nullptr;
+    int* flags = nullptr;   // NonFinite
+    int* host_flag = nullptr;  // its copy in page-locked memory
     cudaStream_t stream = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t gexec = nullptr;
@@ -400,6 +401,14 @@ int fs_batch_create(const fs_config* cfg, int count, const int* rows, const int*
         return rc;
     }
     b->flags = reinterpret_cast<int*>(b->slab + (size_t)K_COUNT * total);
+    NonFinite flag{0, 0, nullptr};
+    if ((e = cudaHostAlloc(&b->host_flag, sizeof(int), cudaHostAllocMapped)) != cudaSuccess ||
+        (*b->host_flag = 0, e = cudaHostGetDevicePointer(&flag.host, b->host_flag, 0)) != cudaSuccess ||
+        (e = cudaMemcpy(b->flags, &flag, sizeof(flag), cudaMemcpyHostToDevice)) != cudaSuccess) {
+        const int rc = cuda_error(e, "fs_batch_create: page-locked flag");
+        fs_batch_destroy(b);
+        return rc;
+    }
     // lanes: grids dealt longest-first to the lane with the fewest cells so far
     const int nlanes = std::min(kBatchLanes, count);
     b->lanes.resize(nlanes);
@@ -443,6 +452,7 @@ int fs_batch_destroy(fs_batch* b) {
         if (b->lanes[l].done) cudaEventDestroy(b->lanes[l].done);
     }
     if (b->fork) cudaEventDestroy(b->fork);
+    if (b->host_flag) cudaFreeHost(b->host_flag);
     if (b->stream) cudaStreamDestroy(b->stream);
     cudaFree(b->slab);
     delete b;
@@ -532,14 +542,11 @@ int fs_batch_sync(fs_batch* b) {
     if (!b) return fail(FS_ERR_ARG, "fs_batch_sync: null handle");
     DeviceScope scope(b->device);
     FS_CK(cudaStreamSynchronize(b->stream));
-    if (b->cfg.check_finite) {
-        int h = 0;
-        FS_CK(cudaMemcpy(&h, b->flags, sizeof(int), cudaMemcpyDeviceToHost));
-        if (h) {
-            FS_CK(cudaMemset(b->flags, 0, sizeof(int)));
-            b->stats.nonfinite = 1;
-            return fail(FS_ERR_NONFINITE, "a batched step produced a non-finite value");
-        }
+    if (b->cfg.check_finite && *reinterpret_cast<volatile int*>(b->host_flag)) {
+        *b->host_flag = 0;
+        FS_CK(cudaMemset(b->flags, 0, sizeof(int)));
+        b->stats.nonfinite = 1;
+        return fail(FS_ERR_NONFINITE, "a batched step produced a non-finite value");
     }
     return FS_OK;
 }

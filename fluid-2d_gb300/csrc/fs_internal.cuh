@@ -139,6 +139,20 @@ inline void field_tiling(StencilField& f, int rows, int cols, int pitch, int reg
     f.tiles_y = 1 + (f.gy_last + f.tile_h - 1) / f.tile_h;
 }
 
+// The non-finite flag: a device word, followed two words later by the address of its copy in
+// page-locked host memory, which a synchronised host reads without a copy of its own. The
+// first report writes both.
+struct NonFinite {
+    int device;
+    unsigned poll_limit;  // polls before a wait between CTAs gives up (0 = default)
+    int* host;
+};
+__device__ __forceinline__ void report_nonfinite(int* flag) {
+    if (atomicOr(flag, 1) != 0) return;
+    int* const host = reinterpret_cast<const NonFinite*>(flag)->host;
+    if (host) *reinterpret_cast<volatile int*>(host) = 1;
+}
+
 // Sets the calling thread's fs_last_error() message and returns code (solver.cu).
 int record_error(int code, const char* msg);
 

@@ -678,7 +678,7 @@ __global__ void __launch_bounds__(256) gradient_kernel(const float* p0, const fl
             bad |= !(isfinite(un) && isfinite(vn));
         }
     }
-    if (bad && nonfinite) atomicOr(nonfinite, 1);
+    if (bad && nonfinite) report_nonfinite(nonfinite);
 }
 
 // Batched form: blocks of 32 x 8 threads over 128 columns x kGradBatchRows rows of one
@@ -704,7 +704,7 @@ __global__ void __launch_bounds__(256) gradient_batch_kernel(const AdvectJob* __
         if (i >= rows || j0 >= cols) continue;
         bad |= gradient_group(J.in0, J.in1, J.in2, J.out0, J.out1, i, j0, rows, cols, (size_t)J.A.pitch, h, rh);
     }
-    if (bad && nonfinite) atomicOr(nonfinite, 1);
+    if (bad && nonfinite) report_nonfinite(nonfinite);
 }
 
 // Rows a warp owns and warps of a CTA: 8 x 8 rows (64-row regions, two CTAs per SM) or
