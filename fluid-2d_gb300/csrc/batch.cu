@@ -248,6 +248,7 @@ int build_plan(fs_batch* b, float diff, float visc, float dt) {
             L.job_blocks[op] = blocks;
         }
     }
+    for (WideLaunch& W : b->h_wide) FS_CK(prepare_stencil_wide(W));
     // ---- upload the job tables (one buffer)
     const size_t job_bytes = b->h_jobs.size() * sizeof(AdvectJob);
     const size_t jpre_bytes = b->h_jprefix.size() * sizeof(int);

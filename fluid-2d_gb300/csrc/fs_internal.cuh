@@ -6,6 +6,7 @@
 // src/linear_buffer.hpp:34-40: pitch = cols*4 B), which leaves most rows misaligned.
 #pragma once
 
+#include <cuda.h>  // CUtensorMap
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -33,6 +34,8 @@ enum PassKind : int {
 constexpr int kRegionW = 128;
 
 struct StencilField {
+    // tensor maps of x and of the second array (x2 or cst), set by the launchers
+    CUtensorMap mx, mk;
     // inputs
     const float* x;     // state in: x (diffuse), p (pressure; may be null = zero start), u (pressure first)
     const float* x2;    // sources s (diffuse first) or v (pressure first)
@@ -83,6 +86,7 @@ struct SolveCtrl {
 // ctrl->converged is already set; otherwise it runs passes from p_cur until the target
 // or max_passes and copies the final pressure back to p_cur. ctrl->passes accumulates.
 struct PressureSolve {
+    CUtensorMap mp[2];  // of p[0] and p[1]
     StencilField first, mid;
     float* p[2];
     float* p_out;      // receives the final pressure (warm start); may be null
@@ -158,7 +162,7 @@ int record_error(int code, const char* msg);
 
 // Launchers (stencil.cu, advect.cu).
 cudaError_t stencil_prepare();
-cudaError_t launch_stencil(const StencilLaunch& L, int tile_rows, cudaStream_t st);
+cudaError_t launch_stencil(StencilLaunch& L, int tile_rows, cudaStream_t st);
 // remove_p and the reflecting fills of u and v from a final pressure p whose edges are
 // filled (the last pass of a multi-pass projection stores it): u_out, v_out on every cell.
 cudaError_t launch_gradient(const float* p, const float* u_in, const float* v_in, float* u_out, float* v_out, int rows,
@@ -173,7 +177,7 @@ cudaError_t launch_gradient_batch(const AdvectJob* jobs, const int* prefix, cons
 int stencil_max_halo(int tile_rows);
 // Co-resident CTAs of the persistent pressure solve on the current device.
 cudaError_t pressure_solve_max_blocks(int tile_rows, int* blocks);
-cudaError_t launch_pressure_solve(const PressureSolve& P, int tile_rows, int blocks, cudaStream_t st);
+cudaError_t launch_pressure_solve(PressureSolve& P, int tile_rows, int blocks, cudaStream_t st);
 cudaError_t launch_splat(const float* d0, const float* u, const float* v, float* acc, const AdvectArgs& A,
                          cudaStream_t st);
 cudaError_t launch_density_finish(const float* acc, float* d, int smooth, const AdvectArgs& A, int* nonfinite,
@@ -239,13 +243,15 @@ cudaError_t launch_advect_batch(int op, const AdvectJob* jobs, const int* prefix
 // Stencil pass over many fields of one class (diffusion or pressure) of a batch's grids,
 // the descriptors carried in the launch's parameters (at most 32,764 bytes on this
 // architecture): field f owns the tiles [begin[f], begin[f + 1]) of the launch.
-constexpr int kMaxWideFields = 168;
+constexpr int kMaxWideFields = 70;
 struct WideLaunch {
     int nfields;
     int begin[kMaxWideFields + 1];
     StencilField f[kMaxWideFields];
 };
 static_assert(sizeof(WideLaunch) <= 32764, "a launch's parameter space holds 32,764 bytes");
+// The fields' tensor maps (once per plan), then the launches.
+cudaError_t prepare_stencil_wide(WideLaunch& L);
 cudaError_t launch_stencil_wide(const WideLaunch& L, bool diffuse, int tile_rows, cudaStream_t st);
 cudaError_t launch_advect_velocity(const float* u0, const float* v0, float* u, float* v, const AdvectArgs& A,
                                    cudaStream_t st);

@@ -27,6 +27,7 @@
 #include <algorithm>
 
 #include "fs_internal.cuh"
+#include "tc.cuh"
 
 namespace fs {
 namespace {
@@ -51,9 +52,11 @@ namespace {
 // cell, a diffusion sweep 6. (Pairs of rows (i, i + 4) instead would be packed throughout,
 // but every 16-byte access and every published or received row then needs its registers
 // moved: 2435 against 1743 warp instructions per tile and warp of 8 diffusion sweeps.)
-// At 2050 x 2050 a pass of 8 sweeps takes 41.5 us for two diffused fields and 22.5 us for
+// At 2050 x 2050 a pass of 8 sweeps takes 37.3 us for two diffused fields and 21.2 us for
 // the pressure (ncu, cold caches; 51-53 and 28-29 us with the field in registers but the
-// constant term in shared memory and edge tiles staged there), the FP32 pipe 53 % busy.
+// constant term in shared memory and edge tiles staged there), the FP32 pipe 57 % busy. At
+// 8194 x 8194 a pressure pass takes 143 us up to 4 sweeps, the rate of HBM (5.6 TB/s), 220 us
+// with 8 and 0.35 us more per sweep and tile beyond, 88 % of the FP32 pipe's rate.
 //
 // Regions and tiles (field_tiling). Every region lies inside the grid where the grid is
 // large enough: the first one starts at row (column) 0 and the last one ends at the last
@@ -197,8 +200,10 @@ __device__ __forceinline__ void for_neighbours(float2 (&X)[R][2], float* __restr
     constexpr unsigned FULL = 0xffffffffu;
     if (EDGE && fold) fill_in_thread<R>(X, e, e.s_lr, e.s_tb);
     const int my_top = 2 * w * RW + 4 * lane, my_bot = my_top + RW;
-    *reinterpret_cast<float4*>(E + my_top) = make_float4(X[0][0].x, X[0][0].y, X[0][1].x, X[0][1].y);
-    *reinterpret_cast<float4*>(E + my_bot) = make_float4(X[R - 1][0].x, X[R - 1][0].y, X[R - 1][1].x, X[R - 1][1].y);
+    *reinterpret_cast<float2*>(E + my_top) = X[0][0];
+    *reinterpret_cast<float2*>(E + my_top + 2) = X[0][1];
+    *reinterpret_cast<float2*>(E + my_bot) = X[R - 1][0];
+    *reinterpret_cast<float2*>(E + my_bot + 2) = X[R - 1][1];
     const bool over_r = EDGE && fold && (e.flags & kERightN);
     auto row = [&](int i, const float2 (&U)[2], const float2 (&D)[2]) {
         const float l = __shfl_up_sync(FULL, X[i][1].y, 1);
@@ -274,9 +279,10 @@ __device__ __forceinline__ void store_filled(float2 (&X)[R][2], float* __restric
     constexpr unsigned FULL = 0xffffffffu;
     if (!edge_tile) {
         if (!t.ocol) return;
+        float* p = y + o;
 #pragma unroll
-        for (int i = 0; i < R; ++i)
-            if (i >= t.r_lo && i < t.r_hi) store4<VEC>(y + o + (size_t)i * pitch, row4(X[i]), t.ncol);
+        for (int i = 0; i < R; ++i, p += pitch)
+            if (i >= t.r_lo && i < t.r_hi) store4<VEC>(p, row4(X[i]), t.ncol);
         return;
     }
     fill_in_thread<R>(X, e, s_lr, s_tb);
@@ -341,78 +347,125 @@ __device__ __forceinline__ void run_sweeps(float2 (&X)[R][2], const float2 (&K)[
     }
 }
 
-// Region of tile b: its first row and column, this thread's block.
+// A CTA's walk over the tiles of a field, every `stride`-th from tile t on, without a
+// division per tile. The columns rotate by one tile per tile row: a CTA would otherwise stay
+// in one column (the slower edge column) where its stride is a multiple of the tiles per row.
+struct TileWalk {
+    int ty, tx;         // tile row and (unrotated) column
+    int rot;            // ty mod n
+    int n, dy, dx, dr;  // tiles per row; the stride in rows and columns, dy mod n
+    __device__ __forceinline__ void start(const StencilField& F, int t, int stride) {
+        n = F.tiles_x;
+        ty = t / n;
+        tx = t - ty * n;
+        rot = ty % n;
+        dy = stride / n;
+        dx = stride - dy * n;
+        dr = dy % n;
+    }
+    __device__ __forceinline__ void next() {
+        tx += dx;
+        const int carry = tx >= n ? 1 : 0;
+        tx -= carry ? n : 0;
+        ty += dy + carry;
+        rot += dr + carry;
+        rot -= rot >= n ? n : 0;
+    }
+    __device__ __forceinline__ int col() const { return tx + rot >= n ? tx + rot - n : tx + rot; }
+};
+
+// First row and column of this thread's block in tile (ty, tx).
 template <int R>
-__device__ __forceinline__ void tile_origin(const StencilField& F, int b, int w, int lane, int& ty, int& tx, int& gyb,
-                                            int& c0) {
-    // columns rotate by one tile per tile row: a CTA takes every gridDim.x-th tile, and
-    // would otherwise stay in one column (the slower edge column) where that is a multiple
-    // of the tiles per row
-    ty = b / F.tiles_x;
-    tx = (b - ty * F.tiles_x + ty) % F.tiles_x;
+__device__ __forceinline__ void tile_origin(const StencilField& F, int ty, int tx, int w, int lane, int& gyb, int& c0) {
     gyb = min(ty * F.tile_h, F.gy_last) + w * R;
     c0 = min(tx * F.tile_w, F.gx_last) + 4 * lane;
 }
 
-// Prefetch of a tile's block into shared memory, 16 bytes per cp.async, each thread its own
-// rows (so no barrier is needed to read them back): R rows of the field, then R rows of the
-// second array (constant term, sources, or v of a first pressure pass, with its rows above
-// and below the block behind them). Rows and lanes outside the grid are zero-filled. A CTA
-// prefetches its next tile while it sweeps the current one; loading each tile only when its
-// turn came left the warps waiting on global loads for 37 % of their time.
+// Prefetch of a tile's block into shared memory by the TMA engine: each warp copies its own
+// rows on its own mbarrier (no CTA barrier is needed to read them back), R rows of the field
+// and R rows of the second array (constant term or sources; of v in a first pressure pass
+// R + 2, from the row above the block on), 512 bytes a row. What lies outside the grid is
+// zero-filled. A CTA prefetches its next tile while it sweeps the current one: loading each
+// tile only when its turn came left the warps waiting on global loads for 37 % of their time,
+// and one 16-byte cp.async per thread and row held up the shuffles and exchange rows behind
+// it in the load/store unit's queue (two diffused fields at 2050^2, 8 sweeps: 39.6 us a pass
+// against 37.3).
 template <int R> constexpr int stage_rows() { return 2 * R + 2; }
-__device__ __forceinline__ void cp_async16(float4* dst, const float* src, bool ok) {
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    const int bytes = ok ? 16 : 0;
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
-}
 template <int R, int NW> __device__ __forceinline__ float4* stage_ptr() {
-    extern __shared__ float4 smem4[];
-    return smem4 + 4 * NW * (kRegionW / 4) + (threadIdx.x >> 5) * stage_rows<R>() * 32 + (threadIdx.x & 31);
+    extern __shared__ __align__(128) float4 smem4[];
+    return smem4 + (4 * NW + (threadIdx.x >> 5) * stage_rows<R>()) * (kRegionW / 4);
 }
-template <int R, int NW, bool DIFF>
-__device__ __forceinline__ void prefetch_tile(const StencilField& F, int b, const float* __restrict__ xin) {
-    float4* const S = stage_ptr<R, NW>();
-    int ty, tx, gyb, c0;
-    tile_origin<R>(F, b, threadIdx.x >> 5, threadIdx.x & 31, ty, tx, gyb, c0);
-    const size_t pitch = (size_t)F.pitch;
-    const bool first = F.kind == (DIFF ? PASS_DIFFUSE_FIRST : PASS_PRESSURE_FIRST);
-    const bool lane_in = c0 < F.cols;
-    const int nrow = lane_in ? F.rows - gyb : 0;
-    // rows and lanes outside the grid read nothing; their address is the array's start
-    const size_t o = nrow > 0 ? (size_t)gyb * pitch + c0 : 0;
-    const float* k = first ? F.x2 : F.cst;
-#pragma unroll
-    for (int i = 0; i < R; ++i) cp_async16(S + i * 32, i < nrow ? xin + o + (size_t)i * pitch : xin, i < nrow);
-#pragma unroll
-    for (int i = 0; i < R; ++i) cp_async16(S + (R + i) * 32, i < nrow ? k + o + (size_t)i * pitch : k, i < nrow);
-    if (!DIFF && first) {
-        const bool up = nrow > 0 && gyb > 0, dn = nrow > R;
-        cp_async16(S + 2 * R * 32, up ? k + o - pitch : k, up);
-        cp_async16(S + (2 * R + 1) * 32, dn ? k + o + (size_t)R * pitch : k, dn);
+template <int R, int NW> __device__ __forceinline__ uint64_t* stage_bar() {
+    extern __shared__ __align__(128) float4 smem4[];
+    return reinterpret_cast<uint64_t*>(smem4 + (4 + stage_rows<R>()) * NW * (kRegionW / 4)) + (threadIdx.x >> 5);
+}
+// Once per kernel, by every warp.
+template <int R, int NW> __device__ __forceinline__ void stage_init() {
+    if ((threadIdx.x & 31) == 0) {
+        tc::mbar_init(stage_bar<R, NW>(), 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        tc::fence_proxy_async_smem();
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
+    __syncwarp();
+}
+__device__ __forceinline__ void tma_load(unsigned dst, const CUtensorMap* map, int x, int y, unsigned bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
+        : "memory");
+}
+// mx, mk: the tensor maps of the field and of the second array (boxes of 128 columns x R, for
+// v R + 2, rows). Column coordinates are multiples of four (16 bytes).
+template <int R, int NW, bool DIFF>
+__device__ __forceinline__ void prefetch_tile(const StencilField& F, int ty, int tx, const CUtensorMap* mx,
+                                              const CUtensorMap* mk) {
+    int gyb, gx;
+    tile_origin<R>(F, ty, tx, threadIdx.x >> 5, 0, gyb, gx);
+    if ((threadIdx.x & 31) == 0) {
+        const bool border = !DIFF && F.kind == PASS_PRESSURE_FIRST;
+        const unsigned bar = tc::smem_u32(stage_bar<R, NW>()), dst = tc::smem_u32(stage_ptr<R, NW>());
+        constexpr unsigned row = 4 * kRegionW;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                     "r"((border ? 2 * R + 2 : 2 * R) * row)
+                     : "memory");
+        tma_load(dst, mx, gx, gyb, bar);
+        tma_load(dst + R * row, mk, gx, border ? gyb - 1 : gyb, bar);
+    }
+}
+// Waits for the warp's prefetch; false when it gave up (a bound, and the same again).
+constexpr unsigned kStageWait = 1u << 20;
+__device__ __forceinline__ bool stage_wait(uint64_t* bar, unsigned parity) {
+    for (unsigned k = 0; k < 2 * kStageWait; ++k)
+        if (tc::mbar_try_wait(bar, parity)) return true;
+    return false;
 }
 
-// One tile of one pass: load the region (fusing add_sources or the divergence into the
+// What a warp carries from tile to tile: the parity of its prefetch, and the exchange buffer
+// that the next sweep uses (so that no barrier is needed between tiles).
+struct Carry {
+    unsigned phase = 0;
+    int buf = 0;
+};
+
+// Tile (ty, tx) of one pass: load the region (fusing add_sources or the divergence into the
 // first pass), run F.sweeps sweeps, store the output tile, then the optional residual
 // partial sums (for residual-driven pressure solves). xin/yout stand in for F.x/F.y so a persistent caller can ping-pong
 // buffers across passes. VEC: the block comes from the prefetch, and `next` starts the next
 // tile's once it has been read.
 template <int R, int NW, bool DIFF, bool VEC, bool RESID, class Next>
-__device__ __forceinline__ void process_tile(const StencilField& F, int b, const float* __restrict__ xin,
+__device__ __forceinline__ void process_tile(const StencilField& F, int ty, int tx, const float* __restrict__ xin,
                                              float* __restrict__ yout, bool resid, float& rnum, float& rden,
-                                             Next&& next) {
+                                             Carry& carry, Next&& next) {
     constexpr int RW = kRegionW;
     constexpr unsigned FULL = 0xffffffffu;
     extern __shared__ float4 smem4[];
-    float* const E0 = reinterpret_cast<float*>(smem4);
-    float* const E1 = E0 + 2 * NW * RW;
+    // the two exchange buffers, the next sweep's first
+    float* const E0 = reinterpret_cast<float*>(smem4) + carry.buf * (2 * NW * RW);
+    float* const E1 = reinterpret_cast<float*>(smem4) + (carry.buf ^ 1) * (2 * NW * RW);
     Place t;
     t.w = threadIdx.x >> 5;
     t.lane = threadIdx.x & 31;
-    int ty, tx;
-    tile_origin<R>(F, b, t.w, t.lane, ty, tx, t.gyb, t.c0);
+    tile_origin<R>(F, ty, tx, t.w, t.lane, t.gyb, t.c0);
     const int rows = F.rows, cols = F.cols;
     const size_t pitch = (size_t)F.pitch;
     t.nrow = rows - t.gyb;
@@ -422,17 +475,19 @@ __device__ __forceinline__ void process_tile(const StencilField& F, int b, const
     t.r_hi = (ty == F.tiles_y - 1 ? rows : (ty + 1) * F.tile_h + F.halo) - t.gyb;
     t.ocol = t.c0 >= (tx == 0 ? 0 : tx * F.tile_w + hx) && t.c0 < (tx == F.tiles_x - 1 ? cols : (tx + 1) * F.tile_w + hx);
     const bool edge_tile = ty == 0 || tx == 0 || ty == F.tiles_y - 1 || tx == F.tiles_x - 1;
-    Edge e;
-    e.s_lr = F.s_lr;
-    e.s_tb = F.s_tb;
-    e.qe = (cols - 1) & 3;
-    e.ib = t.nrow - 1;
-    e.flags = (t.c0 == 0 ? kELeft : 0) | (t.ncol >= 2 && t.ncol <= 4 ? kERight : 0) | (t.ncol == 5 ? kERightN : 0) |
-              (t.gyb == 0 ? kETop : 0) | (t.nrow >= 2 && t.nrow <= R ? kEBot : 0) | (t.nrow == R + 1 ? kEBotN : 0) |
-              (t.ncol == 1 || t.nrow == 1 ? kEOnly : 0);
+    Edge e{};
+    if (edge_tile) {
+        e.s_lr = F.s_lr;
+        e.s_tb = F.s_tb;
+        e.qe = (cols - 1) & 3;
+        e.ib = t.nrow - 1;
+        e.flags = (t.c0 == 0 ? kELeft : 0) | (t.ncol >= 2 && t.ncol <= 4 ? kERight : 0) | (t.ncol == 5 ? kERightN : 0) |
+                  (t.gyb == 0 ? kETop : 0) | (t.nrow >= 2 && t.nrow <= R ? kEBot : 0) | (t.nrow == R + 1 ? kEBotN : 0) |
+                  (t.ncol == 1 || t.nrow == 1 ? kEOnly : 0);
+    }
     const size_t o = (size_t)t.gyb * pitch + t.c0;
     const bool lane_in = t.ncol > 0;
-    const float4* const S = stage_ptr<R, NW>();
+    const float4* const S = stage_ptr<R, NW>() + t.lane;
 
     float2 X[R][2], K[R][2];
     auto put = [](float2 (&x)[2], float4 v) {
@@ -445,15 +500,20 @@ __device__ __forceinline__ void process_tile(const StencilField& F, int b, const
     };
     // row i of the field and of the second array (rows -1 and R of a first pressure pass too)
     auto load_x = [&](int i) { return VEC ? S[i * 32] : load(xin, i); };
+    const int k0 = !DIFF && F.kind == PASS_PRESSURE_FIRST ? R + 1 : R;
     auto load_k = [&](const float* base, int i) {
-        if (VEC) return S[(i < 0 ? 2 * R : i < R ? R + i : 2 * R + 1) * 32];
+        if (VEC) return S[(k0 + i) * 32];
         if (i < 0) return lane_in && t.gyb > 0 && t.nrow > 0 ? load4<VEC>(base + o - pitch, t.ncol) : zero4;
         return load(base, i);
     };
     // columns q of this block and rows i that are interior cells of the grid
     auto int_col = [&](int q) { return t.c0 + q >= 1 && q <= t.ncol - 2; };
     auto int_row = [&](int i) { return t.gyb + i >= 1 && i <= t.nrow - 2; };
-    if (VEC) asm volatile("cp.async.wait_all;" ::: "memory");
+    bool arrived = true;
+    if (VEC) {
+        arrived = stage_wait(stage_bar<R, NW>(), carry.phase);
+        carry.phase ^= 1;
+    }
 
     // ------------------------------------------------------------------ load
     if (!DIFF && F.kind == PASS_PRESSURE_FIRST) {
@@ -518,6 +578,7 @@ __device__ __forceinline__ void process_tile(const StencilField& F, int b, const
     if (VEC) {
         __syncwarp();  // the block has been read
         next();
+        if (!arrived) X[0][0].x = __int_as_float(0x7fffffff);  // reported as a non-finite step
     }
     if ((DIFF ? F.kind == PASS_DIFFUSE_FIRST : F.kind == PASS_PRESSURE_FIRST) && F.cst_out != nullptr && t.ocol) {
         const int hi = min(t.r_hi, t.nrow);
@@ -552,8 +613,10 @@ __device__ __forceinline__ void process_tile(const StencilField& F, int b, const
     // ------------------------------------------------ residual partial sums
     // ||div + sum(nbrs) - 4p||^2 and ||div||^2 over this tile's interior output cells,
     // from the final p (valid one ring beyond the tile: halo = sweeps + 1).
+    carry.buf ^= n & 1;
     if (RESID && resid) {
-        float* const E = (n & 1) ? E1 : E0;  // the exchange buffer the last sweep did not use
+        float* const E = (n & 1) ? E1 : E0;
+        carry.buf ^= 1;
         for_neighbours<R, NW, true>(X, E, t.w, t.lane, n > 0, e,
                                     [&](int i, float l, float r, const float2 (&U)[2], const float2 (&D)[2]) {
             const bool row = t.ocol && i >= t.r_lo && i < t.r_hi && int_row(i);
@@ -724,19 +787,28 @@ __global__ void __launch_bounds__(32 * NW, (NW <= 8 ? 2 : 1))
         return f;
     };
     int b = blockIdx.x, f = field_of(b);
-    if (VEC) prefetch_tile<kR, NW, DIFF>(L.f[f], b - L.f[f].tile_begin, L.f[f].x);
+    TileWalk walk;
+    walk.start(L.f[f], b - L.f[f].tile_begin, gridDim.x);
+    Carry carry;
+    if (VEC) {
+        stage_init<kR, NW>();
+        prefetch_tile<kR, NW, DIFF>(L.f[f], walk.ty, walk.col(), &L.f[f].mx, &L.f[f].mk);
+    }
     float rn = 0.f, rd = 0.f;
 #pragma unroll 1
     while (b < total) {
-        const int nb = b + gridDim.x;
+        const int ty = walk.ty, tx = walk.col(), nb = b + gridDim.x;
         const int nf = nb < total ? field_of(nb) : f;
+        if (nf == f)
+            walk.next();
+        else
+            walk.start(L.f[nf], nb - L.f[nf].tile_begin, gridDim.x);
         const StencilField& F = L.f[f];
-        process_tile<kR, NW, DIFF, VEC, false>(F, b - F.tile_begin, F.x, F.y, false, rn, rd, [&] {
-            if (nb < total) prefetch_tile<kR, NW, DIFF>(L.f[nf], nb - L.f[nf].tile_begin, L.f[nf].x);
+        process_tile<kR, NW, DIFF, VEC, false>(F, ty, tx, F.x, F.y, false, rn, rd, carry, [&] {
+            if (nb < total) prefetch_tile<kR, NW, DIFF>(L.f[nf], walk.ty, walk.col(), &L.f[nf].mx, &L.f[nf].mk);
         });
         b = nb;
         f = nf;
-        if (b < total) __syncthreads();  // the next tile reuses the exchange rows
     }
 }
 
@@ -759,19 +831,26 @@ __global__ void __launch_bounds__(32 * NW, (NW <= 8 ? 2 : 1)) stencil_wide_kerne
     };
     const int total = L.begin[L.nfields];
     int b = blockIdx.x, f = field_of(b);
-    prefetch_tile<kR, NW, DIFF>(L.f[f], b - L.begin[f], L.f[f].x);
+    TileWalk walk;
+    walk.start(L.f[f], b - L.begin[f], gridDim.x);
+    Carry carry;
+    stage_init<kR, NW>();
+    prefetch_tile<kR, NW, DIFF>(L.f[f], walk.ty, walk.col(), &L.f[f].mx, &L.f[f].mk);
     float rn = 0.f, rd = 0.f;
 #pragma unroll 1
     while (b < total) {
-        const int nb = b + gridDim.x;
+        const int ty = walk.ty, tx = walk.col(), nb = b + gridDim.x;
         const int nf = nb < total ? field_of(nb) : f;
+        if (nf == f)
+            walk.next();
+        else
+            walk.start(L.f[nf], nb - L.begin[nf], gridDim.x);
         const StencilField& F = L.f[f];
-        process_tile<kR, NW, DIFF, true, false>(F, b - L.begin[f], F.x, F.y, false, rn, rd, [&] {
-            if (nb < total) prefetch_tile<kR, NW, DIFF>(L.f[nf], nb - L.begin[nf], L.f[nf].x);
+        process_tile<kR, NW, DIFF, true, false>(F, ty, tx, F.x, F.y, false, rn, rd, carry, [&] {
+            if (nb < total) prefetch_tile<kR, NW, DIFF>(L.f[nf], walk.ty, walk.col(), &L.f[nf].mx, &L.f[nf].mk);
         });
         b = nb;
         f = nf;
-        if (b < total) __syncthreads();  // the next tile reuses the exchange rows
     }
 }
 
@@ -859,24 +938,32 @@ __global__ void __launch_bounds__(32 * NW, (NW <= 8 ? 2 : 1))
     if (P.segment && __ldcg(&P.ctrl->converged)) return;
     const unsigned lim_set = P.poll_limit ? __ldcg(P.poll_limit) : 0u;
     const unsigned limit = lim_set ? lim_set : kBarrierSpinLimit;
+    Carry carry;
+    stage_init<kR, NW>();
     int pass = 0;
 #pragma unroll 1
     for (; ok && !done && pass < P.max_passes; ++pass) {
         const StencilField& F = cur < 0 ? P.first : P.mid;
         const float* x = cur < 0 ? F.x : P.p[cur];
+        const CUtensorMap* const mx = cur < 0 ? &F.mx : &P.mp[cur];
         const int dst = cur < 0 ? 0 : cur ^ 1;
         // the residual is formed and tested every second pass (and on the last one allowed):
         // a pass without it skips the residual sums and the reduction, and a solve runs at
         // most one pass beyond the one that met the target
         const bool check = (pass & 1) || pass + 1 >= P.max_passes;
         float rn = 0.f, rd = 0.f;
-        if (blockIdx.x < ntiles) prefetch_tile<kR, NW, false>(F, blockIdx.x, x);
+        TileWalk walk;
+        walk.start(F, blockIdx.x, G);
+        // the previous pass's stores, ordered by the grid barrier, before the TMA engine reads
+        asm volatile("fence.proxy.async;" ::: "memory");
+        if (blockIdx.x < ntiles) prefetch_tile<kR, NW, false>(F, walk.ty, walk.col(), mx, &F.mk);
 #pragma unroll 1
         for (unsigned t = blockIdx.x; t < ntiles; t += G) {
-            process_tile<kR, NW, false, true, true>(F, t, x, P.p[dst], check, rn, rd, [&] {
-                if (t + G < ntiles) prefetch_tile<kR, NW, false>(F, t + G, x);
+            const int ty = walk.ty, tx = walk.col();
+            walk.next();
+            process_tile<kR, NW, false, true, true>(F, ty, tx, x, P.p[dst], check, rn, rd, carry, [&] {
+                if (t + G < ntiles) prefetch_tile<kR, NW, false>(F, walk.ty, walk.col(), mx, &F.mk);
             });
-            __syncthreads();  // the next tile reuses the exchange rows
         }
         double a = rn, b = rd;
         double* part = P.partials + (size_t)(pass & 1) * 2 * G;
@@ -929,8 +1016,9 @@ __global__ void __launch_bounds__(32 * NW, (NW <= 8 ? 2 : 1))
     }
 }
 
-// Exchange rows (two per warp, double-buffered) and the prefetched block of each warp.
-constexpr size_t smem_bytes(int nw) { return (size_t)nw * (4 + stage_rows<kR>()) * kRegionW * sizeof(float); }
+// Exchange rows (two per warp, double-buffered), the prefetched block of each warp and its
+// barrier.
+constexpr size_t smem_bytes(int nw) { return (size_t)nw * ((4 + stage_rows<kR>()) * kRegionW * sizeof(float) + 8); }
 
 // CTAs of a pass that are resident at once on the current device.
 cudaError_t resident_ctas(int nw, int* n) {
@@ -951,6 +1039,37 @@ template <int NW> cudaError_t prepare_variant() {
     if (e == cudaSuccess) e = opt_in(pressure_solve_kernel<NW>, NW);
     if (e == cudaSuccess) e = opt_in(stencil_wide_kernel<NW, true>, NW);
     if (e == cudaSuccess) e = opt_in(stencil_wide_kernel<NW, false>, NW);
+    return e;
+}
+
+// Tensor map of a field's rows in boxes of `box` rows x 128 columns (base and pitch 16-byte
+// aligned); a null base leaves the map zero.
+cudaError_t encode_map(CUtensorMap* map, const float* base, int rows, int cols, int pitch, int box) {
+    if (!base) return cudaSuccess;
+    using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static const Encode encode = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult found;
+        if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &found) != cudaSuccess)
+            fn = nullptr;
+        return reinterpret_cast<Encode>(fn);
+    }();
+    if (!encode) return cudaErrorNotSupported;
+    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)pitch * sizeof(float)};
+    const cuuint32_t boxes[2] = {(cuuint32_t)kRegionW, (cuuint32_t)box}, steps[2] = {1, 1};
+    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims, strides, boxes, steps,
+                              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
+}
+
+cudaError_t encode_field(StencilField& f) {
+    const bool first = f.kind == PASS_DIFFUSE_FIRST || f.kind == PASS_PRESSURE_FIRST;
+    cudaError_t e = encode_map(&f.mx, f.x, f.rows, f.cols, f.pitch, kR);
+    if (e == cudaSuccess)
+        e = encode_map(&f.mk, first ? f.x2 : f.cst, f.rows, f.cols, f.pitch, f.kind == PASS_PRESSURE_FIRST ? kR + 2 : kR);
     return e;
 }
 
@@ -1005,7 +1124,7 @@ bool vector_rows(const StencilField& f) {
 }
 
 template <int NW>
-cudaError_t launch_variant(const StencilLaunch& L, cudaStream_t st) {
+cudaError_t launch_variant(StencilLaunch& L, cudaStream_t st) {
     const size_t smem = smem_bytes(NW);
     int blocks = 0;
     bool vec = true;
@@ -1018,6 +1137,8 @@ cudaError_t launch_variant(const StencilLaunch& L, cudaStream_t st) {
     cudaError_t e = resident_ctas(NW, &ctas);
     if (e != cudaSuccess) return e;
     ctas = std::min(ctas, blocks);
+    for (int i = 0; vec && i < L.nfields; ++i)
+        if ((e = encode_field(L.f[i])) != cudaSuccess) return e;
     // all fields of one launch are of the same class (diffusion or pressure); a handle's and
     // a batch's fields have 128-byte rows, only a caller's velocity may not
     const bool diff = L.f[0].kind == PASS_DIFFUSE_FIRST || L.f[0].kind == PASS_DIFFUSE;
@@ -1073,7 +1194,7 @@ cudaError_t launch_gradient_batch(const AdvectJob* jobs, const int* prefix, cons
     return cudaGetLastError();
 }
 
-cudaError_t launch_stencil(const StencilLaunch& L, int tile_rows, cudaStream_t st) {
+cudaError_t launch_stencil(StencilLaunch& L, int tile_rows, cudaStream_t st) {
     if (tile_rows == 128) return launch_variant<16>(L, st);
     return launch_variant<8>(L, st);
 }
@@ -1083,10 +1204,21 @@ cudaError_t pressure_solve_max_blocks(int tile_rows, int* blocks) {
     return solve_blocks<8>(blocks);
 }
 
-cudaError_t launch_pressure_solve(const PressureSolve& P, int tile_rows, int blocks, cudaStream_t st) {
+cudaError_t launch_pressure_solve(PressureSolve& P, int tile_rows, int blocks, cudaStream_t st) {
     if (blocks <= 0) return cudaErrorInvalidValue;
+    cudaError_t e = encode_field(P.first);
+    if (e == cudaSuccess) e = encode_field(P.mid);
+    for (int k = 0; k < 2 && e == cudaSuccess; ++k)
+        e = encode_map(&P.mp[k], P.p[k], P.mid.rows, P.mid.cols, P.mid.pitch, kR);
+    if (e != cudaSuccess) return e;
     if (tile_rows == 128) return launch_solve_variant<16>(P, blocks, st);
     return launch_solve_variant<8>(P, blocks, st);
+}
+
+cudaError_t prepare_stencil_wide(WideLaunch& L) {
+    cudaError_t e = cudaSuccess;
+    for (int i = 0; i < L.nfields && e == cudaSuccess; ++i) e = encode_field(L.f[i]);
+    return e;
 }
 
 cudaError_t launch_stencil_wide(const WideLaunch& L, bool diffuse, int tile_rows, cudaStream_t st) {
