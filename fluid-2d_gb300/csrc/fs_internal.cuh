@@ -235,7 +235,7 @@ cudaError_t launch_accumulate_df(float* p_hi, float* p_lo, const float* e, long 
 cudaError_t launch_accept_best(float* p_cur, const float* pa, const float* pb, long n_floats, const double* gain,
                                const int* converged, unsigned long long* counters, cudaStream_t st);
 
-int advect_batch_blocks(int rows, int cols);
+int advect_batch_blocks(int op, int rows, int cols);
 // op 0: splat, 1: density finish, 2: velocity backtrace; each block (32x8 threads)
 // covers 32x32 cells; prefix[g] = first block of job g, block_job[b] = job of block b.
 cudaError_t launch_advect_batch(int op, const AdvectJob* jobs, const int* prefix, const int* block_job, int nblocks,

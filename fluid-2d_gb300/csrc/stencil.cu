@@ -725,20 +725,22 @@ __global__ void __launch_bounds__(256) gradient_kernel(const float* p0, const fl
                                                        const float* __restrict__ v_in, float* __restrict__ u_out,
                                                        float* __restrict__ v_out, int rows, int cols, int pitch,
                                                        float h, int* nonfinite, const float* p_alt, const int* sel) {
-    const int j0 = 4 * (blockIdx.x * 32 + threadIdx.x), i = blockIdx.y * 8 + threadIdx.y;
-    if (i >= rows || j0 >= cols) return;
+    const int j0 = 4 * (blockIdx.x * 32 + threadIdx.x);
+    if (j0 >= cols) return;
     const float* __restrict__ p = (sel != nullptr && __ldcg(sel) != 0) ? p_alt : p0;
     const float rh = __frcp_rn(h);
     bool bad = false;
-    if (VEC) {
-        bad = gradient_group(p, u_in, v_in, u_out, v_out, i, j0, rows, cols, (size_t)pitch, h, rh);
-    } else {
-        for (int j = j0; j < min(cols, j0 + 4); ++j) {
-            float un, vn;
-            gradient_cell(p, u_in, v_in, i, j, rows, cols, (size_t)pitch, h, rh, un, vn);
-            u_out[(size_t)i * pitch + j] = un;
-            v_out[(size_t)i * pitch + j] = vn;
-            bad |= !(isfinite(un) && isfinite(vn));
+    for (int i = blockIdx.y * 8 + threadIdx.y; i < rows; i += 8 * gridDim.y) {
+        if (VEC) {
+            bad |= gradient_group(p, u_in, v_in, u_out, v_out, i, j0, rows, cols, (size_t)pitch, h, rh);
+        } else {
+            for (int j = j0; j < min(cols, j0 + 4); ++j) {
+                float un, vn;
+                gradient_cell(p, u_in, v_in, i, j, rows, cols, (size_t)pitch, h, rh, un, vn);
+                u_out[(size_t)i * pitch + j] = un;
+                v_out[(size_t)i * pitch + j] = vn;
+                bad |= !(isfinite(un) && isfinite(vn));
+            }
         }
     }
     if (bad && nonfinite) report_nonfinite(nonfinite);
@@ -1173,7 +1175,7 @@ cudaError_t launch_gradient(const float* p, const float* u_in, const float* v_in
                      ((reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(p_alt) |
                        reinterpret_cast<uintptr_t>(u_in) | reinterpret_cast<uintptr_t>(v_in) |
                        reinterpret_cast<uintptr_t>(u_out) | reinterpret_cast<uintptr_t>(v_out)) & 15) == 0;
-    const dim3 grid(((cols + 3) / 4 + 31) / 32, (rows + 7) / 8);
+    const dim3 grid(((cols + 3) / 4 + 31) / 32, std::min((rows + 7) / 8, 65535));
     if (vec)
         gradient_kernel<true><<<grid, dim3(32, 8), 0, st>>>(p, u_in, v_in, u_out, v_out, rows, cols, pitch, h, nonfinite,
                                                             p_alt, sel);
