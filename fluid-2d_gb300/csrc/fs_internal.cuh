@@ -185,10 +185,11 @@ cudaError_t launch_density_finish(const float* acc, float* d, int smooth, const 
 // Tensor-core conv set-up (shared-memory opt-in) on the current device (conv.cu).
 cudaError_t conv_prepare();
 // fs_conv3x3 with a skip flag: when skip_if (nullable) points at a non-zero value the
-// launch does nothing (a converged pressure solve skips its remaining corrections).
+// launch does nothing (a converged pressure solve skips its remaining corrections), and a
+// mask: outputs are zero where it is not positive (a ReLU backward).
 int conv3x3_launch(const void* x, const void* wpk, const float* w32, const float* bias, const void* skip, void* y,
                    float* yf, int H, int W, int img_h, int up, int relu, int use_tensor_cores, int* err,
-                   const int* skip_if, void* stream);
+                   const int* skip_if, void* stream, const void* mask = nullptr);
 // The whole network on `images` 32 x 32 grids, one launch (fs_net_infer32), with the
 // same skip flag.
 int net_infer32_launch(const void* x0, const void* wpk, const float* params, void* e1, float* y, int images,

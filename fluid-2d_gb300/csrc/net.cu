@@ -75,6 +75,67 @@ __global__ void relu_bwd_kernel(const float* __restrict__ da, const float* __res
     dzb[i] = __float2bfloat16_rn(g);
 }
 
+// The ReLU backward behind a pooling or an upsampling, in one pass: da is the gradient at
+// the output of the layer's successor, SRC = 0 at this layer's resolution, 1 below it (the
+// backward of avgpool2: a quarter of the coarse cell's), 2 above it (the backward of the
+// nearest upsample: the sum of the 2 x 2 block, in upsample2_bwd_kernel's order). Eight
+// channels per thread, 16-byte accesses; dz only where the caller keeps it.
+template <int SRC>
+__global__ void __launch_bounds__(256) relu_bwd_from_kernel(const float* __restrict__ da, const float* __restrict__ da2,
+                                                            const __nv_bfloat16* __restrict__ a, float* __restrict__ dz,
+                                                            __nv_bfloat16* __restrict__ dzb, long n8, int w, int relu) {
+    const long e = (long)blockIdx.x * blockDim.x + threadIdx.x;  // (pixel, channel group)
+    if (e >= n8) return;
+    float g[8];
+    auto load8 = [](const float* p, float (&v)[8]) {
+        const float4 lo = __ldg(reinterpret_cast<const float4*>(p)), hi = __ldg(reinterpret_cast<const float4*>(p) + 1);
+        v[0] = lo.x, v[1] = lo.y, v[2] = lo.z, v[3] = lo.w, v[4] = hi.x, v[5] = hi.y, v[6] = hi.z, v[7] = hi.w;
+    };
+    if (SRC == 0) {
+        load8(da + e * 8, g);
+    } else {
+        const long p = e >> 2, y = p / w;
+        const int x = (int)(p - y * w), c = (int)(e & 3) * 8;
+        if (SRC == 1) {
+            load8(da + ((y >> 1) * (w >> 1) + (x >> 1)) * kC + c, g);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) g[k] *= 0.25f;
+        } else {
+            const float* q = da + (2 * y * (2 * w) + 2 * x) * kC + c;
+            load8(q, g);
+#pragma unroll
+            for (int b = 1; b < 4; ++b) {
+                float t[8];
+                load8(q + ((b & 1) + (long)(b >> 1) * 2 * w) * kC, t);
+#pragma unroll
+                for (int k = 0; k < 8; ++k) g[k] += t[k];
+            }
+        }
+    }
+    if (da2) {
+        float t[8];
+        load8(da2 + e * 8, t);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) g[k] += t[k];
+    }
+    if (relu) {
+        const uint4 m = __ldg(reinterpret_cast<const uint4*>(a) + e);
+        const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(&m);
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (!(__bfloat162float(h[k]) > 0.f)) g[k] = 0.f;
+    }
+    if (dz) {
+        reinterpret_cast<float4*>(dz)[2 * e] = make_float4(g[0], g[1], g[2], g[3]);
+        reinterpret_cast<float4*>(dz)[2 * e + 1] = make_float4(g[4], g[5], g[6], g[7]);
+    }
+    uint4 o;
+    __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&o);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) h[k] = __floats2bfloat162_rn(g[2 * k], g[2 * k + 1]);
+    reinterpret_cast<uint4*>(dzb)[e] = o;
+}
+
 // ------------------------------------------------------------- weight gradient
 // dW[co][t][ci] += sum_p dz[p][co] * x(p, tap t)[ci]; db[co] += sum_p dz[p][co].
 // CUDA cores: a CTA stages 64 pixels' dz rows and im2col rows in shared memory and
@@ -145,16 +206,19 @@ __global__ void flip_weights_kernel(const float* __restrict__ w, float* __restri
 // channel 0, zero elsewhere; the per-CTA partial sums of (y - t)^2 go to loss_part.
 __global__ void mse_kernel(const float* __restrict__ y, const float* __restrict__ target, float* __restrict__ dy,
                            float* __restrict__ loss_part, long n) {
-    __shared__ float red[256];
-    const long p = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ float red[256], grad[256];
+    const long p0 = (long)blockIdx.x * 256, p = p0 + threadIdx.x;
     float e2 = 0.f;
     if (p < n) {
         const float e = y[p * kC] - target[p];
         e2 = e * e;
-        dy[p * kC] = 2.f * e / (float)n;
-#pragma unroll
-        for (int c = 1; c < kC; ++c) dy[p * kC + c] = 0.f;
+        grad[threadIdx.x] = 2.f * e / (float)n;
     }
+    __syncthreads();
+    // the block's 256 x 32 gradients in order (a pixel's 32 per thread took 16 us for 65,536
+    // pixels, this 5: 8 MB of zeros but for channel 0)
+    const int left = (int)min(256L, n - p0) * kC;
+    for (int e = threadIdx.x; e < left; e += 256) dy[p0 * kC + e] = (e & (kC - 1)) == 0 ? grad[e / kC] : 0.f;
     red[threadIdx.x] = e2;
     __syncthreads();
     for (int s = 128; s > 0; s >>= 1) {
@@ -679,6 +743,23 @@ int fs_net_relu_bwd(const float* da, const float* da2, const void* a, float* dz,
     relu_bwd_kernel<<<blocks_for(n, 256), 256, 0, (cudaStream_t)stream>>>(da, da2, (const __nv_bfloat16*)a, dz,
                                                                            (__nv_bfloat16*)dzb, n, relu);
     return launched("fs_net_relu_bwd");
+}
+
+int fs_net_relu_bwd_from(const float* da, int src, const float* da2, const void* a, float* dz, void* dzb, int rows,
+                         int w, int relu, void* stream) {
+    if (!da || !dzb || (relu && !a) || rows < 1 || w < 1 || src < 0 || src > 2 || (src == 1 && ((rows | w) & 1)))
+        return record_error(FS_ERR_ARG, "fs_net_relu_bwd_from: bad argument");
+    if (((uintptr_t)da | (uintptr_t)da2 | (uintptr_t)a | (uintptr_t)dz | (uintptr_t)dzb) & 15)
+        return record_error(FS_ERR_ARG, "fs_net_relu_bwd_from: 16-byte aligned buffers required");
+    const long n8 = (long)rows * w * (kC / 8);
+    const int blocks = blocks_for(n8, 256);
+    cudaStream_t st = (cudaStream_t)stream;
+    const __nv_bfloat16* act = (const __nv_bfloat16*)a;
+    __nv_bfloat16* out = (__nv_bfloat16*)dzb;
+    if (src == 0) relu_bwd_from_kernel<0><<<blocks, 256, 0, st>>>(da, da2, act, dz, out, n8, w, relu);
+    else if (src == 1) relu_bwd_from_kernel<1><<<blocks, 256, 0, st>>>(da, da2, act, dz, out, n8, w, relu);
+    else relu_bwd_from_kernel<2><<<blocks, 256, 0, st>>>(da, da2, act, dz, out, n8, w, relu);
+    return launched("fs_net_relu_bwd_from");
 }
 
 int fs_net_weight_grad(const float* dz, const void* x, float* dw, float* db, int H, int W, int img_h, int up,

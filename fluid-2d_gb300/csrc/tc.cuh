@@ -75,6 +75,13 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
            | ((uint32_t)(M >> 4) << 24);      // M / 16
 }
 
+// The same with A and B MN-major (bits 15 and 16): rows contiguous in memory. For such an
+// operand, no swizzle, a core matrix is 8 K-steps of 16 bytes (8 rows each); smem_desc's
+// `lbo` is the byte distance to the next 8 K-steps, `sbo` to the next 8 rows.
+__host__ __device__ constexpr uint32_t idesc_bf16_f32_mn(int M, int N) {
+    return idesc_bf16_f32(M, N) | (1u << 15) | (1u << 16);
+}
+
 // D[tmem] (+)= A[smem] * B[smem]^T, issued by one thread.
 __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                          bool accumulate) {
@@ -114,6 +121,10 @@ __device__ __forceinline__ void cp_async16(void* dst_smem, const void* src, uint
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst_smem)), "l"(src),
                  "r"(src_bytes)
                  : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() {  // all but the last N groups
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 

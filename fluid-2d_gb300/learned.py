@@ -138,11 +138,8 @@ class Net:
         return self.params[li * NPARAM_LAYER + CH * 9 * CH: (li + 1) * NPARAM_LAYER]
 
     def repack(self, stream=None):
-        L = _lib()
-        for li in range(NLAYER):
-            _chk(L.fs_conv_pack_weights(_p(self.w(li)), _p(self.wpk[li]), stream))
-            _chk(L.fs_net_flip_weights(_p(self.w(li)), _p(self.wflip[li]), stream))
-            _chk(L.fs_conv_pack_weights(_p(self.wflip[li]), _p(self.wflip_pk[li]), stream))
+        _chk(_lib().fs_net_pack_layers(_p(self.params), NLAYER, NPARAM_LAYER, _p(self.wpk), _p(self.wflip),
+                                       _p(self.wflip_pk), stream))
 
     # ------------------------------------------------------------- forward
     def forward(self, x0, stream=None, tensor_cores=True):
@@ -175,12 +172,11 @@ class Net:
         """Gradient of the loss w.r.t. all parameters (FP32 [NPARAM]) given dL/dy. With
         tensor_cores the weight gradients run as tcgen05 implicit GEMMs over the pixels
         (BF16 dz), otherwise on CUDA cores (FP32 dz, the checked reference)."""
+        if tensor_cores:
+            return self._backward_tc(x0, dy, stream)
         torch = self.torch
         L = _lib()
         a = self.act
-        if tensor_cores and getattr(self, "wg_work", None) is None:
-            self.wg_work = torch.empty(int(L.fs_net_weight_grad_tc_work_floats(0, 0)), dtype=torch.float32,
-                                       device=self.dev)
         grad = torch.zeros(NPARAM, dtype=torch.float32, device=self.dev)
         gw = lambda li: grad[li * NPARAM_LAYER: li * NPARAM_LAYER + CH * 9 * CH]
         gb = lambda li: grad[li * NPARAM_LAYER + CH * 9 * CH: (li + 1) * NPARAM_LAYER]
@@ -197,13 +193,8 @@ class Net:
             dz = torch.empty((r, c, CH), dtype=torch.float32, device=self.dev)
             dzb = torch.empty((r, c, CH), dtype=torch.bfloat16, device=self.dev)
             _chk(L.fs_net_relu_bwd(_p(da), _p(da2), _p(out_act), _p(dz), _p(dzb), n, int(relu), stream))
-            if tensor_cores:
-                _chk(L.fs_net_weight_grad_tc(_p(dzb), _p(x_in), _p(gw(li)), _p(gb(li)), _p(self.wg_work),
-                                             self.wg_work.numel(), r, c, self.g >> lvl_out, int(up), _p(self.err),
-                                             stream))
-            else:
-                _chk(L.fs_net_weight_grad(_p(dz), _p(x_in), _p(gw(li)), _p(gb(li)), r, c, self.g >> lvl_out,
-                                          int(up), stream))
+            _chk(L.fs_net_weight_grad(_p(dz), _p(x_in), _p(gw(li)), _p(gb(li)), r, c, self.g >> lvl_out, int(up),
+                                      stream))
             if not want_dx:
                 return None, dz
             dxh = torch.empty((r, c, CH), dtype=torch.float32, device=self.dev)
@@ -227,6 +218,69 @@ class Net:
         d_e1 = zeros(0)
         _chk(L.fs_net_avgpool2_bwd(_p(d_p1), _p(d_e1), *self.shapes[0], stream))
         back(0, d_e1, dz_d2, a["e1"], x0, 0, False, want_dx=False)
+        return grad
+
+    def _backward_tc(self, x0, dy, stream):
+        """The same gradients on the tensor cores: what lies between two convolutions (ReLU,
+        pooling, upsampling, skips) is one launch, or the epilogue of the first one."""
+        torch = self.torch
+        L = _lib()
+        a = self.act
+        level = [lvl for _n, lvl, *_r in LAYERS]
+        if getattr(self, "wg_work", None) is None:
+            f32, bf = torch.float32, torch.bfloat16
+            buf = lambda li, dt: torch.empty((*self.shapes[level[li]], CH), dtype=dt, device=self.dev)
+            self.wg_work = torch.empty(int(L.fs_net_weight_grad_tc_work_floats(0, 0)), dtype=f32, device=self.dev)
+            self.dzb = [buf(li, bf) for li in range(NLAYER)]      # gradient at each layer's output
+            self.dz = {li: buf(li, f32) for li in (5, 6)}         # FP32 where a skip adds it
+            self.dx = [buf(li, f32) for li in (0, 1, 3)]          # gradient at a layer's input, by level
+        grad = torch.zeros(NPARAM, dtype=torch.float32, device=self.dev)
+        base = grad.data_ptr()
+        dzb, dz, dx = self.dzb, self.dz, self.dx
+
+        def wgrad(li, x_in, up=0):
+            r, c = self.shapes[level[li]]
+            gw = base + 4 * li * NPARAM_LAYER
+            _chk(L.fs_net_weight_grad_tc(_p(dzb[li]), _p(x_in), gw, gw + 4 * CH * 9 * CH, _p(self.wg_work),
+                                         self.wg_work.numel(), r, c, self.g >> level[li], up, _p(self.err), stream))
+
+        def to_input(li):
+            r, c = self.shapes[level[li]]
+            _chk(L.fs_conv3x3(_p(dzb[li]), _p(self.wflip_pk[li]), _p(self.wflip[li]), None, None, None,
+                              _p(dx[level[li]]), r, c, self.g >> level[li], 0, 0, 1, _p(self.err), stream))
+
+        def to_layer(li, act):  # the layer below, at the same resolution
+            r, c = self.shapes[level[li]]
+            _chk(L.fs_conv3x3_relu_bwd(_p(dzb[li]), _p(self.wflip_pk[li]), _p(act), _p(dzb[li - 1]),
+                                       _p(dz.get(li - 1)), r, c, self.g >> level[li], _p(self.err), stream))
+
+        def relu(li, da, src, act, da2=None):
+            _chk(L.fs_net_relu_bwd_from(_p(da), src, _p(da2), _p(act), _p(dz.get(li)), _p(dzb[li]),
+                                        *self.shapes[level[li]], int(LAYERS[li][4]), stream))
+
+        if dy.data_ptr() % 16 == 0:
+            relu(7, dy, 0, a["out"])
+        else:  # a caller's view; its FP32 copy goes to a buffer that is free until layer 6's input
+            _chk(L.fs_net_relu_bwd(_p(dy), None, _p(a["out"]), _p(dx[0]), _p(dzb[7]), dy.numel(), 0, stream))
+        wgrad(7, a["d2"])
+        to_layer(7, a["d2"])
+        wgrad(6, a["d1"], 1)
+        to_input(6)
+        relu(5, dx[0], 2, a["d1"])
+        wgrad(5, a["b2"], 1)
+        to_input(5)
+        relu(4, dx[1], 2, a["b2"])
+        wgrad(4, a["b1"])
+        to_layer(4, a["b1"])
+        wgrad(3, self.pool2)
+        to_input(3)
+        relu(2, dx[2], 1, a["e3"], dz[5])   # d1's skip
+        wgrad(2, a["e2"])
+        to_layer(2, a["e2"])
+        wgrad(1, self.pool1)
+        to_input(1)
+        relu(0, dx[1], 1, a["e1"], dz[6])   # d2's skip
+        wgrad(0, x0)
         return grad
 
 

@@ -384,6 +384,21 @@ FS_API int fs_net_avgpool2_bwd(const float* dy, float* dx, int rows_in, int w_in
 FS_API int fs_net_upsample2_bwd(const float* dup, float* dlow, int rows_low, int w_low, void* stream);
 FS_API int fs_net_relu_bwd(const float* da, const float* da2, const void* a, float* dz, void* dzb, long long n,
                            int relu, void* stream);
+/* The tensor-core training path's forms of the above, fewer launches for the same values:
+ *   pack_layers: fs_conv_pack_weights of the weights, fs_net_flip_weights, and pack of the
+ *   flipped ones, for `layers` layers whose weights lie `stride` floats apart in params;
+ *   conv3x3_relu_bwd: the backward-data convolution of dzb with the packed flipped weights,
+ *   then the ReLU backward of the layer below (a: its output), dzb_in (BF16) and, if not
+ *   null, dz_in (FP32);
+ *   relu_bwd_from: relu_bwd of rows x w pixels with da at this resolution (src = 0), before
+ *   the backward of an avgpool2 (1: rows/2 x w/2) or of an upsample2 (2: 2 rows x 2 w); dz
+ *   may be null; buffers 16-byte aligned. */
+FS_API int fs_net_pack_layers(const float* params, int layers, int stride, void* wpk, float* wflip, void* wflip_pk,
+                              void* stream);
+FS_API int fs_conv3x3_relu_bwd(const void* dzb, const void* wpk_flip, const void* a, void* dzb_in, float* dz_in, int H,
+                               int W, int img_h, int* err, void* stream);
+FS_API int fs_net_relu_bwd_from(const float* da, int src, const float* da2, const void* a, float* dz, void* dzb,
+                                int rows, int w, int relu, void* stream);
 FS_API int fs_net_weight_grad(const float* dz, const void* x, float* dw, float* db, int H, int W, int img_h, int up,
                               void* stream);
 /* The weight gradient on the tensor cores: dw += sum_p dz x im2col(x) and db += sum_p dz
