@@ -66,8 +66,7 @@ struct StencilLaunch {
 // Control block of one residual-driven pressure solve (device memory, cleared before
 // each solve): grid-barrier state, the barrier-timeout flag, and the outcome.
 struct SolveCtrl {
-    unsigned bar_count;
-    unsigned bar_gen;
+    unsigned long long bar;  // arrivals at the grid barrier, G per barrier; top bit: it gave up
     int error;      // 1: a grid barrier gave up waiting (FS_ERR_TIMEOUT)
     int passes;     // passes executed (each runs `sweeps` Jacobi sweeps)
     int converged;  // 1: relative residual <= tol
@@ -93,7 +92,8 @@ struct PressureSolve {
     double* partials;  // 4 doubles per CTA (residual sums, double-buffered by pass)
     SolveCtrl* ctrl;
     float tol;
-    int max_passes;
+    int max_passes;                 // passes of mid.sweeps sweeps
+    int pair;                       // 1: run two passes as one of twice the sweeps (the halo holds them)
     int segment;                    // 1: segment mode
     float* p_cur;                   // segment: start and final pressure
     const unsigned* poll_limit;     // device word: polls before a grid barrier gives up

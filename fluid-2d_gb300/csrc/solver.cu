@@ -123,7 +123,8 @@ struct fs_solver {
     // and the per-CTA residual partial sums of the persistent kernel
     SolveCtrl* ctrl = nullptr;
     double* partials[2] = {};
-    int solve_blocks = 0;
+    int solve_blocks = 0;       // CTAs of a residual-driven solve resident at once: regions of
+    int solve_blocks_tall = 0;  // tile_rows rows, and of 128
     // training-data capture: each projection's divergence and starting pressure
     float* cap_div[2] = {};
     float* cap_start[2] = {};
@@ -252,6 +253,37 @@ std::vector<int> split_sweeps(int total, int k) {
 
 void set_geometry(StencilField& f, const fs_solver* s, int halo) {
     field_tiling(f, s->rows, s->cols, s->pitch, s->tile_rows, halo);
+}
+
+// The tiles of a residual-driven solve: sets the geometry of f for its passes and whether
+// they run in pairs (PressureSolve::pair); returns the regions' rows, and the CTAs to launch.
+// A pass costs its grid barrier and the latency of its loads and stores (5 us in all) beside
+// its sweeps, so two passes run as one where every region of a two-pass halo has an SM to
+// itself: with 64-row regions, or, if those of a single pass do not all have one either, with
+// 128-row regions (a longer sweep, less halo). 256 sweeps of 8, us, single passes and pairs:
+// 514 x 514 385 and 289 (64 rows; with a barrier of 3 us), 800 x 800 295 and 311 (128 rows:
+// single passes stay), 1026 x 1026 370 and 317 (128 rows), 1154 x 1154 382 and 398 (128 rows
+// throughout: more than one region an SM).
+int solve_geometry(StencilField& f, const fs_solver* s, int& pair, int& blocks) {
+    const int K = s->sweeps;
+    int sms = 0;
+    const bool known = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s->device) == cudaSuccess;
+    auto tiles = [&](int rows, int halo) {
+        field_tiling(f, s->rows, s->cols, s->pitch, rows, halo);
+        return f.tiles_x * f.tiles_y;
+    };
+    for (int rows : {64, 128}) {
+        if (!known || (s->cfg.tile_rows && rows != s->tile_rows) || 2 * K + 1 > stencil_max_halo(rows)) continue;
+        if (rows > s->tile_rows && tiles(s->tile_rows, K + 1) <= sms) continue;
+        blocks = tiles(rows, 2 * K + 1);
+        if (blocks <= std::min(sms, rows == s->tile_rows ? s->solve_blocks : s->solve_blocks_tall)) {
+            pair = 1;
+            return rows;
+        }
+    }
+    pair = 0;
+    blocks = std::min(s->solve_blocks, tiles(s->tile_rows, K + 1));
+    return s->tile_rows;
 }
 
 AdvectArgs advect_args(const fs_solver* s, float dt) {
@@ -576,7 +608,8 @@ int enqueue_project_learned_cycles(fs_solver* s, const float* u_in, const float*
                            s->stream));
     CK(cudaMemsetAsync(s->ctrl + slot, 0, sizeof(SolveCtrl), s->stream));
     PressureSolve P{};
-    set_geometry(P.mid, s, K + 1);
+    int blocks = 0;
+    const int region_rows = solve_geometry(P.mid, s, P.pair, blocks);
     P.mid.s_lr = P.mid.s_tb = 1.f;
     P.mid.sweeps = K;
     P.mid.kind = PASS_PRESSURE;
@@ -591,13 +624,12 @@ int enqueue_project_learned_cycles(fs_solver* s, const float* u_in, const float*
     P.tol = s->cfg.pressure_tolerance;
     P.segment = 1;
     P.p_cur = pcur;
-    const int blocks = std::min(s->solve_blocks, P.mid.tiles_x * P.mid.tiles_y);
     for (int c = 0; c < cycles; ++c) {
         if ((rc = enqueue_network_correction(s, s->div, pcur, &P.ctrl->converged, cnt)) != FS_OK) return rc;
         const int budget = c + 1 < cycles ? per : std::max(per, cap - (cycles - 1) * per);
         P.max_passes = std::max(1, (budget + K - 1) / K);
         PROF_BEGIN(s);
-        CK(launch_pressure_solve(P, s->tile_rows, blocks, s->stream));
+        CK(launch_pressure_solve(P, region_rows, blocks, s->stream));
         PROF_END(s, FS_KIND_STENCIL, 0.0);  // bytes depend on the iteration count reached
         cnt.launches++;
         cnt.passes++;
@@ -638,7 +670,8 @@ int enqueue_project_learned_defect(fs_solver* s, const float* u_in, const float*
     double* dsums = reinterpret_cast<double*>(s->flags + 4);  // two doubles in the flag block
     double* hsums = reinterpret_cast<double*>(s->host_ctrl + 1);
     PressureSolve P{};
-    set_geometry(P.mid, s, K + 1);
+    int blocks = 0;
+    const int region_rows = solve_geometry(P.mid, s, P.pair, blocks);
     P.mid.s_lr = P.mid.s_tb = 1.f;
     P.mid.sweeps = K;
     P.mid.kind = PASS_PRESSURE;
@@ -652,7 +685,6 @@ int enqueue_project_learned_defect(fs_solver* s, const float* u_in, const float*
     P.poll_limit = reinterpret_cast<const unsigned*>(s->flags + 1);
     P.segment = 1;
     P.p_cur = s->ecur;
-    const int blocks = std::min(s->solve_blocks, P.mid.tiles_x * P.mid.tiles_y);
     int passes = 0, used = 0;
     double ratio = 1.0;
     bool converged = false, timed_out = false;
@@ -674,7 +706,7 @@ int enqueue_project_learned_defect(fs_solver* s, const float* u_in, const float*
         P.max_passes = std::max(1, (budget + K - 1) / K);
         P.tol = (float)std::min(0.5, hsums[0] > 0.0 ? tol * std::sqrt(hsums[1] / hsums[0]) : 1.0);
         PROF_BEGIN(s);
-        CK(launch_pressure_solve(P, s->tile_rows, blocks, s->stream));
+        CK(launch_pressure_solve(P, region_rows, blocks, s->stream));
         PROF_END(s, FS_KIND_STENCIL, 0.0);  // bytes depend on the iteration count reached
         cnt.launches++;
         cnt.passes++;
@@ -715,8 +747,9 @@ int enqueue_project_to_residual(fs_solver* s, const float* u_in, const float* v_
     const float h = grid_h(s->rows, s->cols);
     const int K = s->sweeps;
     PressureSolve P{};
+    int blocks = 0, region_rows = 0;
     for (StencilField* f : {&P.first, &P.mid}) {
-        set_geometry(*f, s, K + 1);
+        region_rows = solve_geometry(*f, s, P.pair, blocks);
         f->s_lr = f->s_tb = 1.f;
         f->sweeps = K;
         f->cdiv = -0.5f * h;
@@ -740,9 +773,8 @@ int enqueue_project_to_residual(fs_solver* s, const float* u_in, const float* v_
     P.tol = s->cfg.pressure_tolerance;
     P.max_passes = std::max(1, (s->cfg.pressure_max_iterations + K - 1) / K);
     CK(cudaMemsetAsync(P.ctrl, 0, sizeof(SolveCtrl), s->stream));
-    const int blocks = std::min(s->solve_blocks, P.mid.tiles_x * P.mid.tiles_y);
     PROF_BEGIN(s);
-    CK(launch_pressure_solve(P, s->tile_rows, blocks, s->stream));
+    CK(launch_pressure_solve(P, region_rows, blocks, s->stream));
     PROF_END(s, FS_KIND_STENCIL, 0.0);  // bytes depend on the iteration count reached
     // gradient subtract from the buffer the solve ended in (P.ctrl->cur)
     PROF_BEGIN(s);
@@ -1281,6 +1313,7 @@ int fs_create(const fs_config* cfg, fs_solver** out) {
     }
     cudaError_t e = stencil_prepare();
     if (e == cudaSuccess) e = pressure_solve_max_blocks(s->tile_rows, &s->solve_blocks);
+    if (e == cudaSuccess) e = pressure_solve_max_blocks(128, &s->solve_blocks_tall);
     if (e == cudaSuccess && cfg->method == FS_METHOD_GAUSS_SEIDEL) e = gs_prepare();
     if (e != cudaSuccess) {
         delete s;
@@ -1289,7 +1322,7 @@ int fs_create(const fs_config* cfg, fs_solver** out) {
     const bool learned = cfg->warm_start == FS_WARM_LEARNED;
     const int nfields = 6 + 9 + 6 + 2 + (cfg->capture ? 4 : 0) + (learned ? 4 : 0);
     // tail: flags (256 B), two solve control blocks, two partial-sum arrays
-    const size_t part_doubles = 4 * (size_t)std::max(1, s->solve_blocks);
+    const size_t part_doubles = 4 * (size_t)std::max({1, s->solve_blocks, s->solve_blocks_tall});
     const size_t tail = 256 + 2 * 256 + 2 * part_doubles * sizeof(double);
     const size_t slab_bytes = (size_t)nfields * s->field_floats * sizeof(float) + tail;
     e = cudaMalloc(&s->slab, slab_bytes);

@@ -448,12 +448,12 @@ struct Carry {
 };
 
 // Tile (ty, tx) of one pass: load the region (fusing add_sources or the divergence into the
-// first pass), run F.sweeps sweeps, store the output tile, then the optional residual
+// first pass), run n sweeps, store the output tile, then the optional residual
 // partial sums (for residual-driven pressure solves). xin/yout stand in for F.x/F.y so a persistent caller can ping-pong
 // buffers across passes. VEC: the block comes from the prefetch, and `next` starts the next
 // tile's once it has been read.
 template <int R, int NW, bool DIFF, bool VEC, bool RESID, class Next>
-__device__ __forceinline__ void process_tile(const StencilField& F, int ty, int tx, const float* __restrict__ xin,
+__device__ __forceinline__ void process_tile(const StencilField& F, int n, int ty, int tx, const float* __restrict__ xin,
                                              float* __restrict__ yout, bool resid, float& rnum, float& rden,
                                              Carry& carry, Next&& next) {
     constexpr int RW = kRegionW;
@@ -588,7 +588,6 @@ __device__ __forceinline__ void process_tile(const StencilField& F, int ty, int 
     }
 
     // ------------------------------------------------------------------ sweeps
-    const int n = F.sweeps;
     if (n > 0) {
         const Coef2 c = {make_float2(F.a, F.a), make_float2(F.rh, F.rh), make_float2(F.rl, F.rl)};
         if (edge_tile)
@@ -806,7 +805,7 @@ __global__ void __launch_bounds__(32 * NW, (NW <= 8 ? 2 : 1))
         else
             walk.start(L.f[nf], nb - L.f[nf].tile_begin, gridDim.x);
         const StencilField& F = L.f[f];
-        process_tile<kR, NW, DIFF, VEC, false>(F, ty, tx, F.x, F.y, false, rn, rd, carry, [&] {
+        process_tile<kR, NW, DIFF, VEC, false>(F, F.sweeps, ty, tx, F.x, F.y, false, rn, rd, carry, [&] {
             if (nb < total) prefetch_tile<kR, NW, DIFF>(L.f[nf], walk.ty, walk.col(), &L.f[nf].mx, &L.f[nf].mk);
         });
         b = nb;
@@ -848,7 +847,7 @@ __global__ void __launch_bounds__(32 * NW, (NW <= 8 ? 2 : 1)) stencil_wide_kerne
         else
             walk.start(L.f[nf], nb - L.begin[nf], gridDim.x);
         const StencilField& F = L.f[f];
-        process_tile<kR, NW, DIFF, true, false>(F, ty, tx, F.x, F.y, false, rn, rd, carry, [&] {
+        process_tile<kR, NW, DIFF, true, false>(F, F.sweeps, ty, tx, F.x, F.y, false, rn, rd, carry, [&] {
             if (nb < total) prefetch_tile<kR, NW, DIFF>(L.f[nf], walk.ty, walk.col(), &L.f[nf].mx, &L.f[nf].mk);
         });
         b = nb;
@@ -857,72 +856,65 @@ __global__ void __launch_bounds__(32 * NW, (NW <= 8 ? 2 : 1)) stencil_wide_kerne
 }
 
 // ---------------------------------------------------------------------------
-// Residual-driven pressure solve in one persistent cooperative launch.
+// Residual-driven pressure solve in one persistent cooperative launch. What bounds it on
+// small and middle grids is what a round costs beside its sweeps. Cycles of a 16-sweep round
+// at 514 x 514 before the sums, the outcome and the barrier took their present form: sweeps
+// 8,900 (13,900 in an edge tile), load 1,000, store 600-2,400, residual sums 3,300, barrier
+// 6,200, outcome 6,300. 256 sweeps there: 385 us in single passes, 289 in pairs, 230 with
+// short sums and the one-word barrier (1026 x 1026: 472 and 317 us, 2050 x 2050: 874 and 787).
 
 constexpr unsigned kBarrierSpinLimit = 1u << 24;  // default: ~2 s of polling, then give up
 
-// Grid-wide barrier for a cooperative launch (all CTAs co-resident). The wait is
-// bounded: after `limit` polls the CTA sets ctrl->error and continues, and every later
-// barrier returns at once, so the kernel always terminates. Returns false once an error
-// has been flagged.
-__device__ __forceinline__ bool grid_barrier(SolveCtrl* ctrl, unsigned nblocks, unsigned limit) {
+// Grid-wide barrier for a cooperative launch (all CTAs co-resident): a CTA adds its arrival
+// and waits until `target` arrivals are there, one word and one trip to the L2 each way. The
+// wait is bounded: after `limit` polls the CTA sets ctrl->error and the word's top bit, which
+// ends every wait, so the kernel always terminates. Returns false once that has happened.
+constexpr unsigned long long kBarrierGaveUp = 1ull << 63;
+__device__ __forceinline__ unsigned long long poll_arrivals(const unsigned long long* bar) {
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(bar) : "memory");
+    return v;
+}
+__device__ __forceinline__ bool grid_barrier(SolveCtrl* ctrl, unsigned long long target, unsigned limit) {
     __shared__ int s_ok;
     __syncthreads();
     if (threadIdx.x == 0) {
-        volatile unsigned* gen = &ctrl->bar_gen;
-        volatile int* err = &ctrl->error;
-        const unsigned g = *gen;
-        __threadfence();
-        if (atomicAdd(&ctrl->bar_count, 1u) == nblocks - 1) {
-            atomicExch(&ctrl->bar_count, 0u);
-            __threadfence();
-            atomicAdd(&ctrl->bar_gen, 1u);
-        } else {
-            unsigned spins = 0;
-            while (*gen == g && *err == 0) {
-                if (++spins > limit) {
-                    atomicExch(&ctrl->error, 1);
-                    break;
-                }
-                __nanosleep(64);
+        asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(&ctrl->bar) : "memory");
+        unsigned spins = 0;
+        unsigned long long v;
+        while ((v = poll_arrivals(&ctrl->bar)) < target) {
+            if (++spins > limit) {
+                atomicExch(&ctrl->error, 1);
+                atomicOr(&ctrl->bar, kBarrierGaveUp);
+                v = kBarrierGaveUp;
+                break;
             }
+            __nanosleep(32);
         }
-        __threadfence();
-        s_ok = (*err == 0);
+        s_ok = v < kBarrierGaveUp;
     }
     __syncthreads();
     return s_ok != 0;
 }
 
-// Fixed-order block sum of two doubles (shuffle tree, then warps in order); every
-// thread receives the result.
-__device__ __forceinline__ void block_sum2(double& a, double& b) {
-    __shared__ double sa[32], sb[32];
-    const int tid = threadIdx.x;
-    const int nw = (blockDim.x + 31) / 32;
+// Sums of n values of two arrays in double, by one warp: lanes 0-15 sum the first, lanes
+// 16-31 the second, in a fixed order; lanes 0 and 16 (and their half-warps) receive them.
+// FP64 is slow on GB300 (with every thread of the CTA summing in double, the sums and the
+// outcome took 9,500 of a pass's 33,000 cycles at 514 x 514), so few lanes add much each.
+template <class Get>
+__device__ __forceinline__ double half_warp_sum(int n, Get&& get) {
+    const int l = threadIdx.x & 15;
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    int i = l;
+#pragma unroll 1
+    for (; i + 48 < n; i += 64)
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        a += __shfl_xor_sync(0xffffffffu, a, o);
-        b += __shfl_xor_sync(0xffffffffu, b, o);
-    }
-    __syncthreads();
-    if ((tid & 31) == 0) {
-        sa[tid >> 5] = a;
-        sb[tid >> 5] = b;
-    }
-    __syncthreads();
-    if (tid == 0) {
-        double x = 0, y = 0;
-        for (int w = 0; w < nw; ++w) {
-            x += sa[w];
-            y += sb[w];
-        }
-        sa[0] = x;
-        sb[0] = y;
-    }
-    __syncthreads();
-    a = sa[0];
-    b = sb[0];
+        for (int k = 0; k < 4; ++k) s[k] += (double)get(i + 16 * k);
+    for (; i < n; i += 16) s[0] += (double)get(i);
+    double t = (s[0] + s[1]) + (s[2] + s[3]);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
 }
 
 template <int NW>
@@ -942,17 +934,24 @@ __global__ void __launch_bounds__(32 * NW, (NW <= 8 ? 2 : 1))
     const unsigned limit = lim_set ? lim_set : kBarrierSpinLimit;
     Carry carry;
     stage_init<kR, NW>();
-    int pass = 0;
+    __shared__ float s_sum[2][32 * NW];
+    __shared__ double s_ratio;
+    // the next barrier's arrivals: earlier segments left a multiple of G, and none of this
+    // launch's barriers completes before this CTA's arrival
+    unsigned long long target = poll_arrivals(&P.ctrl->bar);
+    target = target - target % G;
 #pragma unroll 1
-    for (; ok && !done && pass < P.max_passes; ++pass) {
+    for (int round = 0; ok && !done && passes < P.max_passes; ++round) {
         const StencilField& F = cur < 0 ? P.first : P.mid;
         const float* x = cur < 0 ? F.x : P.p[cur];
         const CUtensorMap* const mx = cur < 0 ? &F.mx : &P.mp[cur];
         const int dst = cur < 0 ? 0 : cur ^ 1;
-        // the residual is formed and tested every second pass (and on the last one allowed):
-        // a pass without it skips the residual sums and the reduction, and a solve runs at
-        // most one pass beyond the one that met the target
-        const bool check = (pass & 1) || pass + 1 >= P.max_passes;
+        // the residual is formed and tested after every second pass (and the last one
+        // allowed): a pass without it skips the residual sums and the reduction, and a solve
+        // runs at most one pass beyond the one that met the target. In pairs a round is two
+        // passes, or a last one by itself.
+        const int take = P.pair ? min(2, P.max_passes - passes) : 1;
+        const bool check = P.pair || (passes & 1) || passes + 1 >= P.max_passes;
         float rn = 0.f, rd = 0.f;
         TileWalk walk;
         walk.start(F, blockIdx.x, G);
@@ -963,33 +962,36 @@ __global__ void __launch_bounds__(32 * NW, (NW <= 8 ? 2 : 1))
         for (unsigned t = blockIdx.x; t < ntiles; t += G) {
             const int ty = walk.ty, tx = walk.col();
             walk.next();
-            process_tile<kR, NW, false, true, true>(F, ty, tx, x, P.p[dst], check, rn, rd, carry, [&] {
+            process_tile<kR, NW, false, true, true>(F, take * F.sweeps, ty, tx, x, P.p[dst], check, rn, rd, carry, [&] {
                 if (t + G < ntiles) prefetch_tile<kR, NW, false>(F, walk.ty, walk.col(), mx, &F.mk);
             });
         }
-        double a = rn, b = rd;
-        double* part = P.partials + (size_t)(pass & 1) * 2 * G;
+        double* part = P.partials + (size_t)(round & 1) * 2 * G;
         if (check) {
-            block_sum2(a, b);
-            if (tid == 0) {
-                part[2 * blockIdx.x] = a;
-                part[2 * blockIdx.x + 1] = b;
+            s_sum[0][tid] = rn;
+            s_sum[1][tid] = rd;
+            __syncthreads();
+            if (tid < 32) {
+                const float* v = s_sum[tid >> 4];
+                const double t = half_warp_sum(32 * NW, [&](int i) { return v[i]; });
+                if ((tid & 15) == 0) part[2 * blockIdx.x + (tid >> 4)] = t;
             }
         }
-        ok = grid_barrier(P.ctrl, G, limit);
-        passes++;
+        target += G;
+        ok = grid_barrier(P.ctrl, target, limit);
+        passes += take;
         cur = dst;
         if (!ok) break;
         if (!check) continue;
         // every CTA sums all partials in the same order, so all agree on the outcome
-        a = 0.0;
-        b = 0.0;
-        for (unsigned i = tid; i < G; i += nt) {
-            a += __ldcg(part + 2 * i);
-            b += __ldcg(part + 2 * i + 1);
+        if (tid < 32) {
+            const double* v = part + (tid >> 4);
+            const double t = half_warp_sum((int)G, [&](int i) { return __ldcg(v + 2 * i); });
+            const double a = __shfl_sync(0xffffffffu, t, 0), b = __shfl_sync(0xffffffffu, t, 16);
+            if (tid == 0) s_ratio = b > 0.0 ? sqrt(a / b) : sqrt(a);
         }
-        block_sum2(a, b);
-        ratio = b > 0.0 ? sqrt(a / b) : sqrt(a);
+        __syncthreads();
+        ratio = s_ratio;
         done = ratio <= (double)P.tol;
     }
     if (ok && cur >= 0) {
