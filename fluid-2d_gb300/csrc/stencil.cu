@@ -138,8 +138,13 @@ constexpr int kETop = 8;     // its row 0 is grid row 0
 constexpr int kEBot = 16;    // its row ib > 0 is grid row rows - 1
 constexpr int kEBotN = 32;   // grid row rows - 1 is the next warp's row 0
 constexpr int kEOnly = 64;   // its column 0 is column cols - 1, or its row 0 row rows - 1
+// Edge::tile, the same in every thread of the CTA: some lane has the column flag. A branch on
+// these is one the whole warp takes or not, and the lane's own flag then only selects (a
+// branch on the lane's flag took both sides one after the other: 41.0 against 39.5 us for a
+// step of 130 x 130).
+constexpr int kTLeft = 128, kTRight = 256, kTRightN = 512;
 struct Edge {
-    int flags;
+    int flags, tile;
     int qe, ib;
     float s_lr, s_tb;
 };
@@ -155,20 +160,23 @@ template <int R, int DST, int SRC> __device__ __forceinline__ void fill_row(floa
         X[DST % R][1] = scale2(sg, X[SRC % R][1]);
     }
 }
-template <int R, int DST, int SRC> __device__ __forceinline__ void fill_col(float2 (&X)[R][2], float sg) {
+template <int R, int DST, int SRC> __device__ __forceinline__ void fill_col(float2 (&X)[R][2], bool mine, float sg) {
 #pragma unroll
-    for (int i = 0; i < R; ++i) colref<DST>(X[i]) = __fmul_rn(sg, colref<SRC>(X[i]));
+    for (int i = 0; i < R; ++i) {
+        const float v = __fmul_rn(sg, colref<SRC>(X[i]));
+        colref<DST>(X[i]) = mine ? v : colref<DST>(X[i]);
+    }
 }
 
 // The reference's edge fill where edge and inner cell share this thread's block. Corner
 // cells this also writes are never read by interior cells.
 template <int R> __device__ __forceinline__ void fill_in_thread(float2 (&X)[R][2], const Edge& e, float s_lr, float s_tb) {
-    if (!(e.flags & (kELeft | kERight | kETop | kEBot))) return;
-    if (e.flags & kELeft) fill_col<R, 0, 1>(X, s_lr);
-    if (e.flags & kERight) {
-        if (e.qe == 1) fill_col<R, 1, 0>(X, s_lr);
-        else if (e.qe == 2) fill_col<R, 2, 1>(X, s_lr);
-        else fill_col<R, 3, 2>(X, s_lr);
+    if (e.tile & kTLeft) fill_col<R, 0, 1>(X, e.flags & kELeft, s_lr);
+    if (e.tile & kTRight) {
+        const bool mine = e.flags & kERight;
+        if (e.qe == 1) fill_col<R, 1, 0>(X, mine, s_lr);
+        else if (e.qe == 2) fill_col<R, 2, 1>(X, mine, s_lr);
+        else fill_col<R, 3, 2>(X, mine, s_lr);
     }
     if (e.flags & kETop) fill_row<R, 0, 1>(X, s_tb);
     if (e.flags & kEBot) {
@@ -204,11 +212,11 @@ __device__ __forceinline__ void for_neighbours(float2 (&X)[R][2], float* __restr
     *reinterpret_cast<float2*>(E + my_top + 2) = X[0][1];
     *reinterpret_cast<float2*>(E + my_bot) = X[R - 1][0];
     *reinterpret_cast<float2*>(E + my_bot + 2) = X[R - 1][1];
-    const bool over_r = EDGE && fold && (e.flags & kERightN);
+    const bool over_r = e.flags & kERightN;
     auto row = [&](int i, const float2 (&U)[2], const float2 (&D)[2]) {
         const float l = __shfl_up_sync(FULL, X[i][1].y, 1);
         float r = __shfl_down_sync(FULL, X[i][0].x, 1);
-        if (EDGE && over_r) r = __fmul_rn(e.s_lr, X[i][1].y);
+        if (EDGE && fold && (e.tile & kTRightN)) r = over_r ? __fmul_rn(e.s_lr, X[i][1].y) : r;
         body(i, l, r, U, D);
     };
     // rows that need no published row
@@ -476,14 +484,18 @@ __device__ __forceinline__ void process_tile(const StencilField& F, int n, int t
     t.ocol = t.c0 >= (tx == 0 ? 0 : tx * F.tile_w + hx) && t.c0 < (tx == F.tiles_x - 1 ? cols : (tx + 1) * F.tile_w + hx);
     const bool edge_tile = ty == 0 || tx == 0 || ty == F.tiles_y - 1 || tx == F.tiles_x - 1;
     Edge e{};
+    e.s_lr = DIFF ? F.s_lr : 1.f;  // the pressure's fill is a copy
+    e.s_tb = DIFF ? F.s_tb : 1.f;
     if (edge_tile) {
-        e.s_lr = F.s_lr;
-        e.s_tb = F.s_tb;
         e.qe = (cols - 1) & 3;
         e.ib = t.nrow - 1;
         e.flags = (t.c0 == 0 ? kELeft : 0) | (t.ncol >= 2 && t.ncol <= 4 ? kERight : 0) | (t.ncol == 5 ? kERightN : 0) |
                   (t.gyb == 0 ? kETop : 0) | (t.nrow >= 2 && t.nrow <= R ? kEBot : 0) | (t.nrow == R + 1 ? kEBotN : 0) |
                   (t.ncol == 1 || t.nrow == 1 ? kEOnly : 0);
+        e.tile = (tx == 0 ? kTLeft : 0) | (tx == F.tiles_x - 1 ? (e.qe == 0 ? kTRightN : kTRight) : 0);
+        // the residual-driven solve has no register left for it: one word with the lane's flags
+        // (256 sweeps at 1026 x 1026 310 us, 316 with its own)
+        if (RESID) e.tile = e.flags |= e.tile;
     }
     const size_t o = (size_t)t.gyb * pitch + t.c0;
     const bool lane_in = t.ncol > 0;
@@ -600,7 +612,7 @@ __device__ __forceinline__ void process_tile(const StencilField& F, int n, int t
     const float* src = !DIFF && F.kind == PASS_PRESSURE_FIRST ? F.cst : xin;
     if (yout != nullptr) {
         if (n > 0) {
-            store_filled<R, VEC>(X, yout, src, t, e, F.s_lr, F.s_tb, o, pitch, edge_tile);
+            store_filled<R, VEC>(X, yout, src, t, e, e.s_lr, e.s_tb, o, pitch, edge_tile);
         } else if (t.ocol) {
             const int hi = min(t.r_hi, t.nrow);
 #pragma unroll
