@@ -160,11 +160,19 @@ __device__ __forceinline__ void report_nonfinite(int* flag) {
 // Sets the calling thread's fs_last_error() message and returns code (solver.cu).
 int record_error(int code, const char* msg);
 
+// Dense host grids (rows x cols floats each) to pitched fields or back by one kernel that
+// addresses the host memory itself (solver.cu), where the device can.
+struct HostGrids {
+    float* host[6];
+    float* field[6];
+};
+cudaError_t launch_host_grids(const HostGrids& G, int count, bool up, int rows, int cols, int pitch, cudaStream_t st);
+
 // Launchers (stencil.cu, advect.cu).
 cudaError_t stencil_prepare();
 cudaError_t launch_stencil(StencilLaunch& L, int tile_rows, cudaStream_t st);
 // remove_p and the reflecting fills of u and v from a final pressure p whose edges are
-// filled (the last pass of a multi-pass projection stores it): u_out, v_out on every cell.
+// filled (the last pass of a projection stores it): u_out, v_out on every cell.
 cudaError_t launch_gradient(const float* p, const float* u_in, const float* v_in, float* u_out, float* v_out, int rows,
                             int cols, int pitch, float h, int* nonfinite, cudaStream_t st,
                             const float* p_alt = nullptr, const int* sel = nullptr);  // p_alt when *sel != 0

@@ -83,7 +83,7 @@ extern "C" int fs_project_noalloc(const float* u, const float* v, float* u_out, 
         return record_error(FS_ERR_ARG,
                             "fs_project_noalloc: rows * pitch exceeds FS_NOALLOC_MAX_CELLS (1048576 floats); "
                             "use a solver handle for larger grids");
-    // The last pass reads u and v around each output cell while other CTAs write the
+    // The gradient launch reads u and v around each output cell while other CTAs write the
     // outputs, so no output may overlap an input or the other output anywhere in its
     // rows x pitch extent (the inputs may overlap each other: they are only read).
     {

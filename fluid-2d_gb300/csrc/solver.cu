@@ -7,8 +7,8 @@
 //   diffuse d,u,v  : ceil(Kd/K) stencil passes, all three fields in each launch
 //                    (add_sources fused into the first pass)
 //   advect d       : memset + forward splat + finish (Neumann fill + smoothing)
-//   project        : ceil(Kp/K) stencil passes (divergence fused into the first,
-//                    gradient subtract + reflecting fills into the last)
+//   project        : ceil(Kp/K) stencil passes (divergence fused into the first), then the
+//                    gradient subtract + reflecting fills
 //   advect u,v     : one backtrace kernel for both components
 //   project        : as above
 //
@@ -1106,12 +1106,7 @@ __global__ void repack_kernel(const Repack6 R, int rows, int cols, int pitch) {
 // one field per blockIdx.y, four values of the dense grid per thread (one 16-byte access to
 // the host side when its base allows). Loads and stores over the link reach the copy
 // engine's rate for page-locked memory and pass it for pageable memory, and a whole call's
-// grids move in one launch. VEC: every host grid 16-byte aligned.
-struct HostGrids {
-    float* host[6];
-    float* field[6];
-};
-
+// grids move in one launch (HostGrids). VEC: every host grid 16-byte aligned.
 template <bool VEC, bool UP>
 __global__ void __launch_bounds__(256) host_grids_kernel(const HostGrids G, int rows, int cols, int pitch) {
     const unsigned n = (unsigned)rows * (unsigned)cols;
@@ -1158,15 +1153,7 @@ __global__ void __launch_bounds__(256) host_grids_kernel(const HostGrids G, int 
 }
 
 template <bool UP> int move_host_grids(fs_solver* s, const HostGrids& G, int count) {
-    uintptr_t bits = 0;
-    for (int k = 0; k < count; ++k) bits |= reinterpret_cast<uintptr_t>(G.host[k]);
-    const long n = (long)s->rows * s->cols;
-    const dim3 grid((unsigned)((n + 1023) / 1024), count);
-    if (bits & 15)
-        host_grids_kernel<false, UP><<<grid, 256, 0, s->stream>>>(G, s->rows, s->cols, s->pitch);
-    else
-        host_grids_kernel<true, UP><<<grid, 256, 0, s->stream>>>(G, s->rows, s->cols, s->pitch);
-    CK(cudaGetLastError());
+    CK(launch_host_grids(G, count, UP, s->rows, s->cols, s->pitch, s->stream));
     s->stats.kernel_launches++;
     return FS_OK;
 }
@@ -2012,3 +1999,15 @@ int fs_host_free(void* ptr) {
 }
 
 }  // extern "C"
+
+cudaError_t fs::launch_host_grids(const HostGrids& G, int count, bool up, int rows, int cols, int pitch, cudaStream_t st) {
+    uintptr_t bits = 0;
+    for (int k = 0; k < count; ++k) bits |= reinterpret_cast<uintptr_t>(G.host[k]);
+    const dim3 grid((unsigned)(((long)rows * cols + 1023) / 1024), count);
+    const bool vec = (bits & 15) == 0;
+    if (up && vec) host_grids_kernel<true, true><<<grid, 256, 0, st>>>(G, rows, cols, pitch);
+    else if (up) host_grids_kernel<false, true><<<grid, 256, 0, st>>>(G, rows, cols, pitch);
+    else if (vec) host_grids_kernel<true, false><<<grid, 256, 0, st>>>(G, rows, cols, pitch);
+    else host_grids_kernel<false, false><<<grid, 256, 0, st>>>(G, rows, cols, pitch);
+    return cudaGetLastError();
+}

@@ -134,9 +134,9 @@ FS_API int fs_config_init(fs_config* cfg, int rows, int cols);
 FS_API int fs_create(const fs_config* cfg, fs_solver** out);
 
 /* Largest grid side (rows = cols, boundary included) that FS_METHOD_GAUSS_SEIDEL accepts
- * on the calling thread's current device (16384). Grids whose field fits one SM's shared
- * memory (234 a side on a GB300) run each solve in one CTA; larger ones run it as a tiled
- * wavefront over the whole GPU. Writes 0 when no device is usable. */
+ * on the calling thread's current device (16384). A solve runs as bands of 32 rows whose
+ * sweeps follow one another as a pipeline of warps; small grids (141 a side and less) in one
+ * CTA. Writes 0 when no device is usable. */
 FS_API int fs_gauss_seidel_max_size(int* n);
 
 /* Device-resident simulation driver: the reference's simulation::add_*_source and
@@ -306,7 +306,7 @@ FS_API int fs_batch_stream(fs_batch* b, void** stream);
 #define FS_KIND_FINISH 2    /* density fill + smoothing */
 #define FS_KIND_ADVECT 3    /* velocity backtrace advection */
 #define FS_KIND_MEMSET 4    /* accumulator clear (a memset node, not a kernel) */
-#define FS_KIND_GRADIENT 5  /* gradient subtract + reflecting fills after a multi-pass projection */
+#define FS_KIND_GRADIENT 5  /* gradient subtract + reflecting fills after a projection */
 #define FS_NUM_KINDS 6
 typedef struct fs_kernel_times {
     int launches[FS_NUM_KINDS];
