@@ -476,8 +476,10 @@ __global__ void __launch_bounds__(32 * kRedWarps) wgrad_reduce_kernel(const floa
 // separate shared buffer and that of layer 6 (e1) in global memory. Pooling and
 // upsampling move data between the level buffers; only interior pixels are written,
 // so the borders stay zero.
+// Bound by the latency of eight dependent layers in one CTA: 57 us (67 with each layer's
+// weights fetched when its turn came, 8 warps and pooling one channel at a time).
 constexpr int kInfG = 32;
-constexpr int kInfThreads = 256;
+constexpr int kInfThreads = 512;
 struct InfLevel {
     int g, P, npad, tiles, guard, slots, PL, bytes;
 };
@@ -492,8 +494,8 @@ __host__ __device__ constexpr InfLevel inf_level(int g) {
                     4 * 16 * ((g + 3) + ((g + 2) * (g + 2) + 127) / 128 * 128 + (g + 3))};
 }
 constexpr InfLevel kL0 = inf_level(kInfG), kL1 = inf_level(kInfG / 2), kL2 = inf_level(kInfG / 4);
-constexpr int kInfWOff = 0;                           // packed weights of the current layer
-constexpr int kInfB0 = kInfWOff + kBbytes;            // level buffers
+constexpr int kInfWOff = 0;                           // packed weights of the current and the next layer
+constexpr int kInfB0 = kInfWOff + 2 * kBbytes;        // level buffers
 constexpr int kInfB1 = kInfB0 + kL0.bytes;
 constexpr int kInfB2 = kInfB1 + kL1.bytes;
 constexpr int kInfE3 = kInfB2 + kL2.bytes;            // e3, NHWC 16 x 16 x 32
@@ -538,6 +540,14 @@ __global__ void __launch_bounds__(kInfThreads) net_infer32_kernel(const InferArg
     __nv_bfloat16* e1g = A.e1 + (size_t)img * G * G * kC;
     float* yout = A.y + (size_t)img * G * G * kC;
 
+    // a layer's weights to its buffer, one copy group (an empty one after the last layer)
+    auto load_weights = [&](int li) {
+        const __nv_bfloat16* src = A.wpk + (size_t)li * (kC * kK);
+        if (li < 8)
+            for (int c = tid; c < kC * kKC; c += kInfThreads) tc::cp_async16(Ws + (li & 1) * kBbytes + c * 16, src + c * 8, 16);
+        tc::cp_async_commit();
+    };
+    load_weights(0);
     if (warp == 0) {
         tc::tmem_alloc(s_taddr, 512);
         tc::tmem_relinquish();
@@ -558,20 +568,26 @@ __global__ void __launch_bounds__(kInfThreads) net_infer32_kernel(const InferArg
     const uint32_t taddr = *s_taddr;
 
     auto pool = [&](uint8_t* src, const InfLevel Ls, uint8_t* dst, const InfLevel Ld) {
-        // 2x2 average (avgpool2_kernel's order and rounding) into the next level
-        for (int e = tid; e < Ld.g * Ld.g * kC; e += kInfThreads) {
-            const int c = e % kC, p = e / kC, Y = p / Ld.g, X = p % Ld.g;
-            const int cg = c >> 3, ci = c & 7;
-            auto at = [&](int y, int x) {
-                const __nv_bfloat16* q = reinterpret_cast<const __nv_bfloat16*>(
-                    inf_slot(src, Ls, inf_interior(Ls, y, x), cg));
-                return __bfloat162float(q[ci]);
-            };
-            const float sum = __fadd_rn(__fadd_rn(__fadd_rn(at(2 * Y, 2 * X), at(2 * Y, 2 * X + 1)),
-                                                  at(2 * Y + 1, 2 * X)),
-                                        at(2 * Y + 1, 2 * X + 1));
-            reinterpret_cast<__nv_bfloat16*>(inf_slot(dst, Ld, inf_interior(Ld, Y, X), cg))[ci] =
-                __float2bfloat16_rn(__fmul_rn(0.25f, sum));
+        // 2x2 average (avgpool2_kernel's order and rounding) into the next level, eight
+        // channels at a time
+        for (int e = tid; e < Ld.g * Ld.g * 4; e += kInfThreads) {
+            const int p = e >> 2, cg = e & 3, Y = p / Ld.g, X = p % Ld.g;
+            uint4 q[4], w;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) q[k] = *inf_slot(src, Ls, inf_interior(Ls, 2 * Y + (k >> 1), 2 * X + (k & 1)), cg);
+            const __nv_bfloat162(*h)[4] = reinterpret_cast<const __nv_bfloat162(*)[4]>(q);
+            __nv_bfloat162* o = reinterpret_cast<__nv_bfloat162*>(&w);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                float2 s = __bfloat1622float2(h[0][c]);
+#pragma unroll
+                for (int k = 1; k < 4; ++k) {
+                    const float2 f = __bfloat1622float2(h[k][c]);
+                    s = make_float2(__fadd_rn(s.x, f.x), __fadd_rn(s.y, f.y));
+                }
+                o[c] = __floats2bfloat162_rn(__fmul_rn(0.25f, s.x), __fmul_rn(0.25f, s.y));
+            }
+            *inf_slot(dst, Ld, inf_interior(Ld, Y, X), cg) = w;
         }
     };
     auto upsample = [&](uint8_t* src, const InfLevel Ls, uint8_t* dst, const InfLevel Ld) {
@@ -588,17 +604,17 @@ __global__ void __launch_bounds__(kInfThreads) net_infer32_kernel(const InferArg
     // the skip buffer, 3: FP32 to the output (no ReLU)
     auto layer = [&](int li, uint8_t* buf, const InfLevel L, int skip_kind, int out_kind) {
         if (!ok) return;
-        // the layer's weights (the previous layer's MMAs are complete)
-        const __nv_bfloat16* wsrc = A.wpk + (size_t)li * (kC * kK);
-        for (int c = tid; c < kC * kKC; c += kInfThreads) tc::cp_async16(Ws + c * 16, wsrc + c * 8, 16);
-        tc::cp_async_wait_all();
+        // the next layer's weights into the other buffer (the MMAs of the layer before, which
+        // read it, are complete); this layer's are on their way since then
+        load_weights(li + 1);
+        tc::cp_async_wait<1>();
         tc::fence_proxy_async_smem();  // weights and the activations written by this CTA
         tc::fence_before_sync();
         __syncthreads();
         tc::fence_after_sync();
         if (tid == 0) {
             constexpr uint32_t idesc = tc::idesc_bf16_f32(128, 32);
-            const uint32_t a0 = tc::smem_u32(buf), w0 = tc::smem_u32(Ws);
+            const uint32_t a0 = tc::smem_u32(buf), w0 = tc::smem_u32(Ws + (li & 1) * kBbytes);
             for (int T = 0; T < L.tiles; ++T) {
 #pragma unroll
                 for (int t = 0; t < 9; ++t) {
@@ -698,6 +714,7 @@ __global__ void __launch_bounds__(kInfThreads) net_infer32_kernel(const InferArg
     }
     layer(6, B0, kL0, 1, 0);  // d2 = relu(conv(up d1) + b + e1)
     layer(7, B0, kL0, 0, 3);  // out
+    tc::cp_async_wait<0>();
     if (!ok && tid == 0 && A.err) atomicOr(A.err, 1);
     // every MMA was waited for, unless a wait gave up: then keep the allocation rather
     // than free columns an MMA may still write

@@ -160,6 +160,26 @@ __device__ __forceinline__ void report_nonfinite(int* flag) {
 // Sets the calling thread's fs_last_error() message and returns code (solver.cu).
 int record_error(int code, const char* msg);
 
+// Sums of n values of two arrays in double, by one warp: lanes 0-15 sum the first, lanes
+// 16-31 the second, in a fixed order; lanes 0 and 16 (and their half-warps) receive them.
+// FP64 is slow on GB300 (with every thread of the CTA summing in double, the sums and the
+// outcome took 9,500 of a pass's 33,000 cycles at 514 x 514), so few lanes add much each.
+template <class Get>
+__device__ __forceinline__ double half_warp_sum(int n, Get&& get) {
+    const int l = threadIdx.x & 15;
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    int i = l;
+#pragma unroll 1
+    for (; i + 48 < n; i += 64)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) s[k] += (double)get(i + 16 * k);
+    for (; i < n; i += 16) s[0] += (double)get(i);
+    double t = (s[0] + s[1]) + (s[2] + s[3]);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
+}
+
 // Dense host grids (rows x cols floats each) to pitched fields or back by one kernel that
 // addresses the host memory itself (solver.cu), where the device can.
 struct HostGrids {

@@ -297,20 +297,28 @@ __global__ void coarse_input_kernel(const float* __restrict__ bs, int G, float* 
     for (int c = threadIdx.x; c < G * G; c += blockDim.x) acc += (double)bs[c] * bs[c];
     red[threadIdx.x] = acc;
     __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) red[threadIdx.x] += red[threadIdx.x + s];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        s_scale = (float)fmax(sqrt(red[0] / (double)(G * G)), 1e-30);
-        if (scale_out) *scale_out = s_scale;
-        if (norm2) *norm2 = red[0];
+    if (threadIdx.x < 32) {
+        const double* v = red + (threadIdx.x & 16) * 32;  // a half each
+        const double t = half_warp_sum(512, [&](int i) { return v[i]; });
+        const double sum = t + __shfl_xor_sync(0xffffffffu, t, 16);
+        if (threadIdx.x == 0) {
+            s_scale = (float)fmax(sqrt(sum / (double)(G * G)), 1e-30);
+            if (scale_out) *scale_out = s_scale;
+            if (norm2) *norm2 = sum;
+        }
     }
     __syncthreads();
     if (!xin) return;
     const float inv = 1.f / s_scale;
-    for (int e = threadIdx.x; e < G * G * kC; e += blockDim.x)
-        xin[e] = __float2bfloat16_rn((e % kC) == 0 ? bs[e / kC] * inv : 0.f);
+    if ((reinterpret_cast<uintptr_t>(xin) & 15) == 0) {  // eight channels at a time
+        for (int e = threadIdx.x; e < G * G * (kC / 8); e += blockDim.x) {
+            const __nv_bfloat162 first = __floats2bfloat162_rn((e & 3) == 0 ? bs[e >> 2] * inv : 0.f, 0.f);
+            reinterpret_cast<uint4*>(xin)[e] = make_uint4(reinterpret_cast<const uint32_t&>(first), 0, 0, 0);
+        }
+    } else {
+        for (int e = threadIdx.x; e < G * G * kC; e += blockDim.x)
+            xin[e] = __float2bfloat16_rn((e % kC) == 0 ? bs[e / kC] * inv : 0.f);
+    }
 }
 
 // Coarse post-smoothing of a coarse correction (one CTA, G*G <= 4096): e = y_in[.,0] *
@@ -425,7 +433,7 @@ __global__ void energy_gain_kernel(const float* __restrict__ div, const float* _
                                    const float* __restrict__ p_try, int rows, int cols, int pitch,
                                    double* __restrict__ out, const int* __restrict__ skip_if) {
     if (skip_if && __ldcg(skip_if)) return;
-    __shared__ double red[256];
+    __shared__ float red[256];
     float g = 0.f;  // a thread's few cells; the CTA and grid sums are in FP64
     const int j = blockIdx.x * 256 + threadIdx.x;
     if (j >= 1 && j <= cols - 2) {
@@ -442,11 +450,12 @@ __global__ void energy_gain_kernel(const float* __restrict__ div, const float* _
     }
     red[threadIdx.x] = g;
     __syncthreads();
-    for (int k = 128; k > 0; k >>= 1) {
-        if (threadIdx.x < k) red[threadIdx.x] += red[threadIdx.x + k];
-        __syncthreads();
+    if (threadIdx.x < 32) {
+        const float* v = red + (threadIdx.x & 16) * 8;  // a half each
+        const double t = half_warp_sum(128, [&](int i) { return v[i]; });
+        const double sum = t + __shfl_xor_sync(0xffffffffu, t, 16);
+        if (threadIdx.x == 0) atomicAdd(out, sum);
     }
-    if (threadIdx.x == 0) atomicAdd(out, red[0]);
 }
 
 // One damped Jacobi step, p_out = p + (J(p) - p) / 2 with J(p) = (div + sum(nbrs p)) / 4,
@@ -563,11 +572,12 @@ inline dim3 row_grid(int rows, int cols) {
 // r = div + sum(nbrs of p) - 4p for p = p_hi + p_lo, to about twice FP32 precision: the
 // FP32 heads (and div, and -4*p_hi, which is exact) are summed with their rounding errors
 // (sum2), the tails, which are ~2^-24 of the heads, in FP32; zero on the boundary.
-// sums[0] += ||r||^2 and sums[1] += ||div||^2 over the interior.
+// sums[0] += ||r||^2 and sums[1] += ||div||^2 over the interior. (514 x 514: 10 us, 17 with
+// the CTA's FP64 sums as a tree over all threads.)
 __global__ void residual_df_kernel(const float* __restrict__ div, const float* __restrict__ ph,
                                    const float* __restrict__ pl, float* __restrict__ r, int rows, int cols, int pitch,
                                    double* __restrict__ sums) {
-    __shared__ double red[2][256];
+    __shared__ float red[2][256];
     float rr = 0.f, dd = 0.f;
     const int j = blockIdx.x * 256 + threadIdx.x;
     if (j < cols) {
@@ -597,16 +607,10 @@ __global__ void residual_df_kernel(const float* __restrict__ div, const float* _
     red[0][threadIdx.x] = rr;
     red[1][threadIdx.x] = dd;
     __syncthreads();
-    for (int k = 128; k > 0; k >>= 1) {
-        if (threadIdx.x < k) {
-            red[0][threadIdx.x] += red[0][threadIdx.x + k];
-            red[1][threadIdx.x] += red[1][threadIdx.x + k];
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        atomicAdd(sums, red[0][0]);
-        atomicAdd(sums + 1, red[1][0]);
+    if (threadIdx.x < 32) {
+        const float* v = red[threadIdx.x >> 4];
+        const double t = half_warp_sum(256, [&](int i) { return v[i]; });
+        if ((threadIdx.x & 15) == 0) atomicAdd(sums + (threadIdx.x >> 4), t);
     }
 }
 // (p_hi, p_lo) += e as a double-float sum: two_sum of the heads, the error folded into
