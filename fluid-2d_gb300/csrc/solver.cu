@@ -227,11 +227,13 @@ cudaError_t create_streams(fs_solver* s) {
 }
 
 // Whether to diffuse the density on the step's side branch instead of in the same
-// launches as u and v. Fields are independent, so the density passes can fill the SMs the
-// u/v passes leave idle in their last wave; that pays where a fused three-field pass has
-// a short last wave among few (1024^2: 0.359 -> 0.335 ms per 40/40 step, 2048^2: 1.034 ->
-// 1.023 ms) and costs where the last wave is negligible (4096^2, 31 waves: +0.5 %) or the
-// step is launch-bound (130^2: +5 %). So: when the fused pass fills 1 to 12 waves.
+// launches as u and v. Fields are independent, so on a low-priority stream the density passes
+// fill what the u/v and pressure passes leave idle: the ends of their last waves, and at
+// large sizes the time in which a memory-bound launch (splat, gradient) leaves the FP32 pipe
+// free. It costs a few launches more where the step is bound by launches. So: when a fused
+// three-field pass fills a wave. Step, us, fused and with the branch: 130 x 130 41.1 and 43.1,
+// 514 x 514 47 and 50, 771 x 1283 88.5 and 88.2, 1026 x 1026 174 and 170, 2050 x 2050 493 and
+// 458, 4098 x 4098 1693 and 1606, 8194 x 8194 3455 and 3351.
 bool density_branch_pays(const fs_solver* s, int dev) {
     int sms = 0;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return false;
@@ -239,7 +241,7 @@ bool density_branch_pays(const fs_solver* s, int dev) {
     const long tw = kRegionW - 2 * s->sweeps, th = s->tile_rows - 2 * s->sweeps;
     if (tw <= 0 || th <= 0) return false;
     const long tiles3 = 3 * ((s->cols + tw - 1) / tw) * ((s->rows + th - 1) / th);
-    return tiles3 >= slots && tiles3 <= 12L * slots;
+    return tiles3 >= slots;
 }
 
 // Split `total` sweeps into passes of at most `k` (at least one pass, possibly of
