@@ -103,9 +103,9 @@ def parse():
 # ncu on this build (profiles/stencil_kernel_2048_vortex.md): DRAM bytes read + written per
 # interior cell and field by one depth-8 pass at 2048^2, and the unit that bounds the pass
 NCU_DRAM_BYTES_PER_CELL_FIELD_PASS = 8.2
-NCU_BINDING = ("instruction issue and latency: 2 CTAs of 8 warps per SM at 128 registers (24 % of the warp "
-               "slots); ncu on a 2048^2 middle pressure pass: issue active 39 %, DRAM 15 %, L1/shared 48 %, "
-               "largest stall instruction fetch")
+NCU_BINDING = ("FP32 pipe and instruction issue: 2 CTAs of 8 warps per SM at 127 registers; ncu on a 2048^2 "
+               "middle pressure pass: issue active 56 %, FP32 pipe 47 %, L1/shared 51 %, largest stall a busy "
+               "math pipe; in the steady state of larger grids 73 % and 69 %")
 
 
 def dist_env():
