@@ -101,6 +101,31 @@ int fail(int code, const char* msg) { return record_error(code, msg); }
 
 constexpr int kBatchLanes = 4;
 
+// Default temporal-blocking depth, by the tiles of a one-field pass of all grids at depth 8
+// against the CTAs resident at once, as for a single grid (default_sweeps in solver.cu): below
+// a quarter of a wave the fewest passes whose output tiles keep 16 rows, up to three waves 10,
+// beyond 8. Steps of 30/30 sweeps, us at depths 8, 10, 15: 8 grids of 40-200 a side (37 tiles)
+// 115, 105, 94; 24 of 64-256 (145) 136, 133, 132; 32 of 120-512 (749) 401, 398, 433; 16 of
+// 512-1024 (2098) 973, 1004, 1159.
+int default_depth(const fs_batch* b, const int* rows, const int* cols, int maxk) {
+    const int k8 = std::min(8, maxk);
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device) != cudaSuccess || sms <= 0) return k8;
+    const long slots = sms * (b->tile_rows <= 64 ? 2 : 1);
+    long tiles = 0;
+    for (int g = 0; g < b->count; ++g) {
+        StencilField f{};
+        field_tiling(f, rows[g], cols[g], cols[g], b->tile_rows, k8);
+        tiles += (long)f.tiles_x * f.tiles_y;
+    }
+    if (tiles >= 3 * slots) return k8;
+    const int kmax = std::min(maxk, (b->tile_rows - 16) / 2 - 1);
+    if (4 * tiles >= slots || kmax <= k8) return std::min(10, maxk);
+    const int total = std::max(b->cfg.diffuse_iterations, b->cfg.pressure_iterations);
+    const int passes = std::max(1, (total + kmax - 1) / kmax);
+    return std::max(k8, (total + passes - 1) / passes);
+}
+
 // One stencil pass over the fields fl: ceil(n / kMaxWideFields) launches with as even a
 // share of the fields as possible, each field's tiles numbered from its launch's start.
 fs_batch::Pass add_pass(fs_batch* b, const std::vector<StencilField>& fl, bool diffuse) {
@@ -382,7 +407,7 @@ int fs_batch_create(const fs_config* cfg, int count, const int* rows, const int*
     b->count = count;
     b->tile_rows = cfg->tile_rows ? cfg->tile_rows : 64;
     const int maxk = stencil_max_halo(b->tile_rows) - 1;
-    b->sweeps = cfg->sweeps_per_pass > 0 ? std::min(cfg->sweeps_per_pass, maxk) : std::min(8, maxk);
+    b->sweeps = cfg->sweeps_per_pass > 0 ? std::min(cfg->sweeps_per_pass, maxk) : default_depth(b, rows, cols, maxk);
     size_t total = 0;
     for (int g = 0; g < count; ++g) {
         b->rows.push_back(rows[g]);
