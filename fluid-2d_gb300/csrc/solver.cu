@@ -52,6 +52,7 @@ int cuda_fail(cudaError_t e, const char* what) {
     return fail(e == cudaErrorMemoryAllocation ? FS_ERR_NOMEM : FS_ERR_CUDA, m);
 }
 
+#define CK_RC(call) do { const int rc_ = (call); if (rc_ != FS_OK) return rc_; } while (0)
 #define CK(call)                                               \
     do {                                                       \
         cudaError_t e_ = (call);                               \
@@ -177,6 +178,7 @@ struct fs_solver {
     int tile_rows = 64;
     // diffuse the density on the side branch too (see density_branch_pays)
     bool density_branch = false;
+    bool density_pending = false;  // the side branch still reads the state velocity
     int launches_per_step = 0;
     int passes_per_step = 0;
     bool warm_valid = false;
@@ -575,8 +577,11 @@ int capture_div(fs_solver* s, int slot) {
 // Residual-driven projection: one persistent cooperative launch runs depth-K passes
 // until the relative residual ||div + sum(nbrs) - 4p|| / ||div|| is <= tol or the
 // iteration cap is reached, then the gradient subtract (see pressure_solve_kernel).
+int join_density(fs_solver* s);
+
 int enqueue_fin_pass(fs_solver* s, const float* p, const float* u_in, const float* v_in, float* u_out, float* v_out,
                      Counter& cnt) {
+    if (u_out == s->st[F_U]) CK_RC(join_density(s));
     PROF_BEGIN(s);
     CK(launch_gradient(p, u_in, v_in, u_out, v_out, s->rows, s->cols, s->pitch, grid_h(s->rows, s->cols),
                        s->cfg.check_finite ? s->flags : nullptr, s->stream));
@@ -779,6 +784,7 @@ int enqueue_project_to_residual(fs_solver* s, const float* u_in, const float* v_
     CK(launch_pressure_solve(P, region_rows, blocks, s->stream));
     PROF_END(s, FS_KIND_STENCIL, 0.0);  // bytes depend on the iteration count reached
     // gradient subtract from the buffer the solve ended in (P.ctrl->cur)
+    if (u_out == s->st[F_U]) CK_RC(join_density(s));
     PROF_BEGIN(s);
     CK(launch_gradient(s->p[0], u_in, v_in, u_out, v_out, s->rows, s->cols, s->pitch, h,
                        s->cfg.check_finite ? s->flags : nullptr, s->stream, s->p[1], &P.ctrl->cur));
@@ -882,28 +888,42 @@ int fork_density(fs_solver* s, const float* dif_d, float diff, float dt, bool di
     }
     if ((rc = enqueue_advect_density(s, dif_d, s->st[F_D], s->st[F_U], s->st[F_V], dt, cnt, st)) != FS_OK) return rc;
     CK(cudaEventRecord(s->side_ev[1], s->side));
+    s->density_pending = true;
     return FS_OK;
 }
 
+// Called before the launch that writes the state velocity (the last gradient subtract), and
+// where a step fails before it.
 int join_density(fs_solver* s) {
+    if (!s->density_pending) return FS_OK;
+    s->density_pending = false;
     CK(cudaStreamWaitEvent(s->stream, s->side_ev[1], 0));
     return FS_OK;
 }
 
 // Velocity half of a step from the diffused velocity: project (into the u/v diffusion
 // scratch, free by now, so that the state keeps the initial velocity the density
-// advection reads), advect by itself, join the density half, project into the state.
-int enqueue_velocity_tail(fs_solver* s, const float* dif_u, const float* dif_v, float dt, Counter& cnt) {
-    int rc;
+// advection reads), advect by itself, project into the state, whose last launch joins the
+// density half. between: what to enqueue after the advection.
+template <class Between>
+int enqueue_velocity_tail(fs_solver* s, const float* dif_u, const float* dif_v, float dt, Counter& cnt,
+                          Between&& between) {
     float* pu = s->x0[F_U];
     float* pv = s->x0[F_V];
-    if ((rc = enqueue_project(s, dif_u, dif_v, pu, pv, 0, cnt)) != FS_OK) return rc;
-    PROF_BEGIN(s);
-    CK(launch_advect_velocity(pu, pv, s->vel1[0], s->vel1[1], advect_args(s, dt), s->stream));
-    PROF_END(s, FS_KIND_ADVECT, 16.0 * interior_cells(s));  // read u0, v0; write u, v
-    cnt.launches++;
-    if ((rc = join_density(s)) != FS_OK) return rc;
-    return enqueue_project(s, s->vel1[0], s->vel1[1], s->st[F_U], s->st[F_V], 1, cnt);
+    int rc = enqueue_project(s, dif_u, dif_v, pu, pv, 0, cnt);
+    if (rc == FS_OK) {
+        PROF_BEGIN(s);
+        CK(launch_advect_velocity(pu, pv, s->vel1[0], s->vel1[1], advect_args(s, dt), s->stream));
+        PROF_END(s, FS_KIND_ADVECT, 16.0 * interior_cells(s));  // read u0, v0; write u, v
+        cnt.launches++;
+        rc = between();
+    }
+    if (rc == FS_OK) rc = enqueue_project(s, s->vel1[0], s->vel1[1], s->st[F_U], s->st[F_V], 1, cnt);
+    if (rc != FS_OK) join_density(s);
+    return rc;
+}
+int enqueue_velocity_tail(fs_solver* s, const float* dif_u, const float* dif_v, float dt, Counter& cnt) {
+    return enqueue_velocity_tail(s, dif_u, dif_v, dt, cnt, [] { return FS_OK; });
 }
 
 int enqueue_step(fs_solver* s, float diff, float visc, float dt, Counter& cnt) {
@@ -1302,7 +1322,7 @@ int fs_create(const fs_config* cfg, fs_solver** out) {
     }
     cudaError_t e = stencil_prepare();
     if (e == cudaSuccess) e = pressure_solve_max_blocks(s->tile_rows, &s->solve_blocks);
-    if (e == cudaSuccess) e = pressure_solve_max_blocks(128, &s->solve_blocks_tall);
+    if (e == cudaSuccess && cfg->pressure_tolerance > 0.f) e = pressure_solve_max_blocks(128, &s->solve_blocks_tall);
     if (e == cudaSuccess && cfg->method == FS_METHOD_GAUSS_SEIDEL) e = gs_prepare();
     if (e != cudaSuccess) {
         delete s;
@@ -1551,8 +1571,7 @@ int launch_repack(fs_solver* s, float* const* stage, float* const* dst, int coun
 }
 
 // One Jacobi step on host grids with the copies overlapped: the six grids go up as three
-// (field, source) pairs and each field diffuses while the next pair is on its way; the
-// new density goes down while the velocity is projected and advected. Each field sees
+// (field, source) pairs and each field diffuses while the next pair is on its way. Each field sees
 // the same kernels as in enqueue_step, so the results are those of upload + step +
 // download. host: density, u, v, density source, u source, v source; out: density, u, v.
 int solve_host_overlapped(fs_solver* s, const float* const host[6], float* const out[3], float diff, float visc,
@@ -1571,30 +1590,50 @@ int solve_host_overlapped(fs_solver* s, const float* const host[6], float* const
     // uploads begin after the handle's earlier work, which may still read the scratch
     CK(cudaEventRecord(s->xev[0], s->stream));
     CK(cudaStreamWaitEvent(up, s->xev[0], 0));
-    // Three pairs go up one after another — density and its source, then u and its source,
-    // then v and its source — and each field diffuses as soon as its pair has landed, so
-    // the GPU works while the rest is still on the link (a one-field diffusion takes about
-    // as long as the next pair's upload). The density's advection, which needs the step's
-    // initial u and v, runs on the side stream beside the first projection.
-    const int pairs[3][2] = {{0, 1}, {2, 4}, {3, 5}};  // stage indices: field, source
-    const int fields[3] = {F_D, F_U, F_V};
-    const float rates[3] = {diff, visc, visc};
+    // Three pairs go up one after another — u and its source, v and its source, the density
+    // and its source — and each field diffuses as soon as its pair has landed, so the GPU works
+    // while the rest is still on the link. The velocity goes first since most of a step is
+    // its: the first projection runs while the density is on its way, and the density
+    // (diffusion, advection by the step's initial velocity, smoothing) on the side stream
+    // beside the rest. A solve whose host reads the residual would hold the density's copies
+    // back, so there they come before it.
+    const int pairs[3][2] = {{2, 4}, {3, 5}, {0, 1}};  // stage indices: field, source
+    const int fields[3] = {F_U, F_V, F_D};
+    const float rates[3] = {visc, visc, diff};
     float* dif[3] = {};
     Counter cnt;
     int rc;
-    for (int q = 0; q < 3; ++q) {
+    auto pair_up = [&](int q, cudaStream_t st) {
         for (int k : pairs[q]) CK(cudaMemcpyAsync(stage[k], from[k], bytes, cudaMemcpyHostToDevice, up));
         CK(cudaEventRecord(s->xev[1 + q], up));
-        CK(cudaStreamWaitEvent(s->stream, s->xev[1 + q], 0));
+        CK(cudaStreamWaitEvent(st, s->xev[1 + q], 0));
         float* const st2[2] = {stage[pairs[q][0]], stage[pairs[q][1]]};
         float* const ds2[2] = {dst[pairs[q][0]], dst[pairs[q][1]]};
-        if ((rc = launch_repack(s, st2, ds2, 2)) != FS_OK) return rc;
-        if ((rc = enqueue_diffuse(s, &fields[q], 1, &rates[q], dt, &dif[q], cnt)) != FS_OK) return rc;
-    }
-    if ((rc = fork_density(s, dif[0], diff, dt, false, cnt)) != FS_OK) return rc;
+        return launch_repack(s, st2, ds2, 2, st);
+    };
+    auto diffuse = [&](int q, cudaStream_t st) {
+        return enqueue_diffuse(s, &fields[q], 1, &rates[q], dt, &dif[q], cnt, st);
+    };
+    auto density = [&]() -> int {
+        CK(cudaStreamWaitEvent(s->side, s->side_ev[0], 0));  // the initial velocity is in the state
+        int r = pair_up(2, s->side);
+        if (r == FS_OK) r = diffuse(2, s->side);
+        if (r == FS_OK)
+            r = enqueue_advect_density(s, dif[2], s->st[F_D], s->st[F_U], s->st[F_V], dt, cnt, s->side);
+        if (r != FS_OK) return r;
+        CK(cudaEventRecord(s->side_ev[1], s->side));
+        s->density_pending = true;
+        return FS_OK;
+    };
+    if ((rc = pair_up(0, s->stream)) != FS_OK || (rc = diffuse(0, s->stream)) != FS_OK) return rc;
+    if ((rc = pair_up(1, s->stream)) != FS_OK) return rc;
+    CK(cudaEventRecord(s->side_ev[0], s->stream));
+    if ((rc = diffuse(1, s->stream)) != FS_OK) return rc;
+    const bool host_reads = s->cfg.pressure_tolerance > 0.f;
+    if (host_reads && (rc = density()) != FS_OK) return rc;
+    rc = enqueue_velocity_tail(s, dif[0], dif[1], dt, cnt, [&] { return host_reads ? FS_OK : density(); });
+    if (rc != FS_OK) return rc;
     CK(cudaEventRecord(s->xev[4], s->side));
-    float* dif_uv[2] = {dif[1], dif[2]};
-    if ((rc = enqueue_velocity_tail(s, dif_uv[0], dif_uv[1], dt, cnt)) != FS_OK) return rc;
     // the density download is issued after the velocity work so that a pageable
     // (host-blocking) copy still overlaps it
     CK(cudaStreamWaitEvent(down, s->xev[4], 0));
