@@ -518,15 +518,17 @@ int fs_batch_download(fs_batch* b, int index, float* d, float* u, float* v) {
     // Below 2^20 cells (the host call's line) one kernel writes the three grids over the link:
     // 24 grids of 64 to 512 a side in 570 us, 980 with a copy per field. Like a
     // copy's, pageable memory is complete on return.
-    if (b->direct_host && (long)b->rows[index] * b->cols[index] < (1L << 20)) {
-        HostGrids G{};
-        float* const host[3] = {d, u, v};
+    HostGrids G{};
+    float* const host[3] = {d, u, v};
+    for (int k = 0; k < 3; ++k) {
+        G.host[k] = host[k];
+        G.field[k] = b->fld(K_ST_D + k, index);
+    }
+    if (b->direct_host && G.aligned(3) && (long)b->rows[index] * b->cols[index] < (1L << 20)) {
         bool pageable = false;
-        for (int k = 0; k < 3; ++k) {
-            G.host[k] = host[k];
-            G.field[k] = b->fld(K_ST_D + k, index);
+        for (float* p : host) {
             cudaPointerAttributes a{};
-            FS_CK(cudaPointerGetAttributes(&a, host[k]));
+            FS_CK(cudaPointerGetAttributes(&a, p));
             pageable = pageable || a.type == cudaMemoryTypeUnregistered;
         }
         FS_CK(launch_host_grids(G, 3, false, b->rows[index], b->cols[index], b->pitch[index], b->stream));

@@ -185,6 +185,13 @@ __device__ __forceinline__ double half_warp_sum(int n, Get&& get) {
 struct HostGrids {
     float* host[6];
     float* field[6];
+    // Whether a kernel may take the host grids: floats at multiples of four bytes. (A caller's
+    // packed record or byte buffer may hold them anywhere; copies do not mind.)
+    bool aligned(int count) const {
+        uintptr_t bits = 0;
+        for (int k = 0; k < count; ++k) bits |= reinterpret_cast<uintptr_t>(host[k]);
+        return bits % sizeof(float) == 0;
+    }
 };
 cudaError_t launch_host_grids(const HostGrids& G, int count, bool up, int rows, int cols, int pitch, cudaStream_t st);
 

@@ -1657,17 +1657,18 @@ namespace {
 // One step on host grids without overlap (small grids). Where kernels can address any host
 // memory (GB300 beside a Grace CPU) one launch reads the six grids from the host and one
 // writes the three results back (800 x 800, pageable: 214 us per call against 333 with
-// copies). Elsewhere: stage the six inputs densely in scratch fields the step overwrites
-// anyway, spread them into the pitched fields with one kernel, step, copy the state out.
+// copies). Elsewhere, and for grids that do not lie on a multiple of four bytes: stage the six
+// inputs densely in scratch fields the step overwrites anyway, spread them into the pitched
+// fields with one kernel, step, copy the state out.
 int solve_host_serial(fs_solver* s, const float* const host[6], float* const out[3], float diff, float visc,
                       float dt) {
-    if (s->direct_host) {
-        float* const fields[6] = {s->st[F_D], s->st[F_U], s->st[F_V], s->src[F_D], s->src[F_U], s->src[F_V]};
-        HostGrids G{};
-        for (int k = 0; k < 6; ++k) {
-            G.host[k] = const_cast<float*>(host[k]);
-            G.field[k] = fields[k];
-        }
+    float* const fields[6] = {s->st[F_D], s->st[F_U], s->st[F_V], s->src[F_D], s->src[F_U], s->src[F_V]};
+    HostGrids G{};
+    for (int k = 0; k < 6; ++k) {
+        G.host[k] = const_cast<float*>(host[k]);
+        G.field[k] = fields[k];
+    }
+    if (s->direct_host && G.aligned(6)) {
         int rc;
         if ((rc = move_host_grids<true>(s, G, 6)) != FS_OK) return rc;
         if ((rc = run_steps(s, diff, visc, dt, 1)) != FS_OK) return rc;
@@ -1680,13 +1681,8 @@ int solve_host_serial(fs_solver* s, const float* const host[6], float* const out
     for (int k = 0; k < 6; ++k) {
         CK(cudaMemcpyAsync(stage[k], host[k], bytes, cudaMemcpyHostToDevice, s->stream));
         R.src[k] = stage[k];
+        R.dst[k] = fields[k];
     }
-    R.dst[0] = s->st[F_D];
-    R.dst[1] = s->st[F_U];
-    R.dst[2] = s->st[F_V];
-    R.dst[3] = s->src[F_D];
-    R.dst[4] = s->src[F_U];
-    R.dst[5] = s->src[F_V];
     repack_kernel<<<dim3(152 * 2, 6), 256, 0, s->stream>>>(R, s->rows, s->cols, s->pitch);
     CK(cudaGetLastError());
     s->stats.kernel_launches++;
