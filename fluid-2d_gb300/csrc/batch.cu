@@ -51,8 +51,8 @@ struct fs_batch {
     std::vector<size_t> off;  // per-grid offset (floats) inside each field-kind range
     size_t range_floats = 0;  // floats per field kind (all grids)
     float* slab = nullptr;
-    int* flags = nullptr;   // NonFinite
-    int* host_flag = nullptr;  // its copy in page-locked memory
+    int* flags = nullptr;             // StepFlags
+    HostFlags* host_flags = nullptr;  // their copy in page-locked memory
     cudaStream_t stream = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t gexec = nullptr;
@@ -138,6 +138,7 @@ fs_batch::Pass add_pass(fs_batch* b, const std::vector<StencilField>& fl, bool d
         b->h_wide.emplace_back();
         WideLaunch& W = b->h_wide.back();
         std::memset(&W, 0, sizeof(W));
+        W.flags = b->flags;
         W.nfields = cnt;
         int tiles = 0;
         for (int i = 0; i < cnt; ++i) {
@@ -430,11 +431,11 @@ int fs_batch_create(const fs_config* cfg, int count, const int* rows, const int*
         return rc;
     }
     b->flags = reinterpret_cast<int*>(b->slab + (size_t)K_COUNT * total);
-    NonFinite flag{0, 0, nullptr};
-    if ((e = cudaHostAlloc(&b->host_flag, sizeof(int), cudaHostAllocMapped)) != cudaSuccess ||
-        (*b->host_flag = 0, e = cudaHostGetDevicePointer(&flag.host, b->host_flag, 0)) != cudaSuccess ||
-        (e = cudaMemcpy(b->flags, &flag, sizeof(flag), cudaMemcpyHostToDevice)) != cudaSuccess) {
-        const int rc = cuda_error(e, "fs_batch_create: page-locked flag");
+    StepFlags flags{};
+    if ((e = cudaHostAlloc(&b->host_flags, sizeof(HostFlags), cudaHostAllocMapped)) != cudaSuccess ||
+        (*b->host_flags = {}, e = cudaHostGetDevicePointer(&flags.host, b->host_flags, 0)) != cudaSuccess ||
+        (e = cudaMemcpy(b->flags, &flags, sizeof(flags), cudaMemcpyHostToDevice)) != cudaSuccess) {
+        const int rc = cuda_error(e, "fs_batch_create: page-locked flags");
         fs_batch_destroy(b);
         return rc;
     }
@@ -481,7 +482,7 @@ int fs_batch_destroy(fs_batch* b) {
         if (b->lanes[l].done) cudaEventDestroy(b->lanes[l].done);
     }
     if (b->fork) cudaEventDestroy(b->fork);
-    if (b->host_flag) cudaFreeHost(b->host_flag);
+    if (b->host_flags) cudaFreeHost(b->host_flags);
     if (b->stream) cudaStreamDestroy(b->stream);
     cudaFree(b->slab);
     delete b;
@@ -592,8 +593,13 @@ int fs_batch_sync(fs_batch* b) {
     if (!b) return fail(FS_ERR_ARG, "fs_batch_sync: null handle");
     DeviceScope scope(b->device);
     FS_CK(cudaStreamSynchronize(b->stream));
-    if (b->cfg.check_finite && *reinterpret_cast<volatile int*>(b->host_flag)) {
-        *b->host_flag = 0;
+    if (*reinterpret_cast<volatile int*>(&b->host_flags->timed_out)) {
+        *b->host_flags = {};
+        FS_CK(cudaMemset(b->flags, 0, sizeof(int)));
+        return fail(FS_ERR_TIMEOUT, "a batched step's wait for a tile gave up: the states are not valid");
+    }
+    if (b->cfg.check_finite && *reinterpret_cast<volatile int*>(&b->host_flags->nonfinite)) {
+        b->host_flags->nonfinite = 0;
         FS_CK(cudaMemset(b->flags, 0, sizeof(int)));
         b->stats.nonfinite = 1;
         return fail(FS_ERR_NONFINITE, "a batched step produced a non-finite value");

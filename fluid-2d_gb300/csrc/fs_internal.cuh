@@ -58,7 +58,11 @@ struct StencilField {
 };
 
 constexpr int kMaxStencilFields = 4;
+// flags: where a wait that gives up is reported (StepFlags; may be null). polls: bound of the
+// waits for prefetched tiles, 0 the default (stage_wait).
 struct StencilLaunch {
+    int* flags;
+    unsigned polls;
     StencilField f[kMaxStencilFields];
     int nfields;
 };
@@ -143,18 +147,25 @@ inline void field_tiling(StencilField& f, int rows, int cols, int pitch, int reg
     f.tiles_y = 1 + (f.gy_last + f.tile_h - 1) / f.tile_h;
 }
 
-// The non-finite flag: a device word, followed two words later by the address of its copy in
-// page-locked host memory, which a synchronised host reads without a copy of its own. The
-// first report writes both.
-struct NonFinite {
-    int device;
-    unsigned poll_limit;  // polls before a wait between CTAs gives up (0 = default)
-    int* host;
+// What a step's launches report: a device word for the first non-finite value, and the address
+// of the words in host memory that a synchronised host reads without a copy of its own.
+struct HostFlags {
+    int nonfinite;
+    int timed_out;  // a wait for a prefetched tile gave up
 };
-__device__ __forceinline__ void report_nonfinite(int* flag) {
-    if (atomicOr(flag, 1) != 0) return;
-    int* const host = reinterpret_cast<const NonFinite*>(flag)->host;
-    if (host) *reinterpret_cast<volatile int*>(host) = 1;
+struct StepFlags {
+    int nonfinite;
+    unsigned poll_limit;  // polls before a wait between CTAs gives up (0 = default)
+    HostFlags* host;
+};
+__device__ __forceinline__ void report_nonfinite(int* flags) {
+    if (atomicOr(flags, 1) != 0) return;
+    HostFlags* const host = reinterpret_cast<const StepFlags*>(flags)->host;
+    if (host) *reinterpret_cast<volatile int*>(&host->nonfinite) = 1;
+}
+__device__ __forceinline__ void report_timeout(int* flags) {
+    HostFlags* const host = flags ? reinterpret_cast<const StepFlags*>(flags)->host : nullptr;
+    if (host) *reinterpret_cast<volatile int*>(&host->timed_out) = 1;
 }
 
 // Sets the calling thread's fs_last_error() message and returns code (solver.cu).
@@ -281,6 +292,7 @@ cudaError_t launch_advect_batch(int op, const AdvectJob* jobs, const int* prefix
 // architecture): field f owns the tiles [begin[f], begin[f + 1]) of the launch.
 constexpr int kMaxWideFields = 70;
 struct WideLaunch {
+    int* flags;  // as in StencilLaunch
     int nfields;
     int begin[kMaxWideFields + 1];
     StencilField f[kMaxWideFields];

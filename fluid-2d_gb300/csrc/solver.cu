@@ -107,19 +107,20 @@ struct fs_solver {
     float* p[2] = {};
     float* vel1[2] = {};
     float* pwarm[2] = {};
-    int* flags = nullptr;  // NonFinite, then (at [4]) the defect correction's two FP64 sums
-    // host memory the device writes: the non-finite flag's copy, and as of the last fs_sync
+    int* flags = nullptr;  // StepFlags, then (at [4]) the defect correction's two FP64 sums
+    // host memory the device writes: the flags' copy, and as of the last fs_sync
     // the network's error flag and the solves' control blocks. In the handle itself where the
     // device addresses any host memory and nothing is copied to it (page-locking takes longer
     // than the rest of fs_create), else page-locked.
     struct HostState {
-        int nonfinite;
+        HostFlags flags;
         int net_err;
         SolveCtrl ctrl[2];
     };
     HostState own_host{};
     HostState* host = nullptr;
-    bool direct_host = false;  // kernels can address pageable host memory
+    unsigned prefetch_polls = 0;  // StencilLaunch::polls
+    bool direct_host = false;     // kernels can address pageable host memory
     // residual-driven pressure solves: one control block per projection of a step,
     // and the per-CTA residual partial sums of the persistent kernel
     SolveCtrl* ctrl = nullptr;
@@ -255,6 +256,14 @@ std::vector<int> split_sweeps(int total, int k) {
     return out;
 }
 
+StencilLaunch new_launch(const fs_solver* s, int nfields) {
+    StencilLaunch L{};
+    L.flags = s->flags;
+    L.polls = s->prefetch_polls;
+    L.nfields = nfields;
+    return L;
+}
+
 void set_geometry(StencilField& f, const fs_solver* s, int halo) {
     field_tiling(f, s->rows, s->cols, s->pitch, s->tile_rows, halo);
 }
@@ -360,8 +369,7 @@ int enqueue_diffuse(fs_solver* s, const int* fields, int nf, const float* rates,
     const float* cur[3] = {};
     for (int q = 0; q < nf; ++q) cur[q] = s->st[fields[q]];
     for (size_t pass = 0; pass < plan.size(); ++pass) {
-        StencilLaunch L{};
-        L.nfields = nf;
+        StencilLaunch L = new_launch(s, nf);
         int begin = 0;
         for (int q = 0; q < nf; ++q) {
             const int fid = fields[q];
@@ -423,8 +431,7 @@ __nv_bfloat16* net_act(fs_solver* s, int k) {
 // Divergence of (u_in, v_in) into s->div: a pressure pass of zero sweeps.
 int enqueue_div_pass(fs_solver* s, const float* u_in, const float* v_in, Counter& cnt) {
     const float h = grid_h(s->rows, s->cols);
-    StencilLaunch L{};
-    L.nfields = 1;
+    StencilLaunch L = new_launch(s, 1);
     StencilField& f = L.f[0];
     set_geometry(f, s, 1);
     f.s_lr = f.s_tb = 1.f;
@@ -812,8 +819,7 @@ int enqueue_project(fs_solver* s, const float* u_in, const float* v_in, float* u
     float* pfinal = nullptr;
     for (int pass = 0; pass < m; ++pass) {
         const bool last = pass == m - 1;
-        StencilLaunch L{};
-        L.nfields = 1;
+        StencilLaunch L = new_launch(s, 1);
         StencilField& f = L.f[0];
         // a region's border columns have no divergence of their own
         set_geometry(f, s, std::max(plan[pass], pass == 0 ? 1 : 0));
@@ -1061,8 +1067,14 @@ int finish(fs_solver* s) {
         CK(cudaMemcpyAsync(s->host->ctrl, s->ctrl, 2 * sizeof(SolveCtrl), cudaMemcpyDeviceToHost, s->stream));
     if (net) CK(cudaMemcpyAsync(&s->host->net_err, s->net.err, sizeof(int), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
-    if (s->cfg.check_finite && *reinterpret_cast<volatile int*>(&s->host->nonfinite)) {
-        s->host->nonfinite = 0;
+    if (*reinterpret_cast<volatile int*>(&s->host->flags.timed_out)) {
+        s->host->flags = {};
+        if (solves) s->steps_reported = s->stats.steps;
+        CK(cudaMemsetAsync(s->flags, 0, sizeof(int), s->stream));
+        return fail(FS_ERR_TIMEOUT, "a pass's wait for a tile gave up: the state is not valid");
+    }
+    if (s->cfg.check_finite && *reinterpret_cast<volatile int*>(&s->host->flags.nonfinite)) {
+        s->host->flags.nonfinite = 0;
         CK(cudaMemsetAsync(s->flags, 0, sizeof(int), s->stream));
         s->stats.nonfinite = 1;
         return fail(FS_ERR_NONFINITE, "the step produced a non-finite value");
@@ -1437,15 +1449,15 @@ int fs_create(const fs_config* cfg, fs_solver** out) {
         if (cudaDeviceGetAttribute(&access, cudaDevAttrPageableMemoryAccess, dev) == cudaSuccess)
             s->direct_host = access != 0;
         const bool copies = learned || cfg->pressure_tolerance > 0.f || cfg->method == FS_METHOD_GAUSS_SEIDEL;
-        NonFinite f{0, 0, nullptr};
+        StepFlags f{};
         if (s->direct_host && !copies) {
             s->host = &s->own_host;
-            f.host = &s->host->nonfinite;
+            f.host = &s->host->flags;
         } else if ((e = cudaHostAlloc(&s->host, sizeof(*s->host), cudaHostAllocMapped)) != cudaSuccess) {
             rc = cuda_fail(e, "fs_create: pinned state block");
         } else {
             *s->host = {};
-            if ((e = cudaHostGetDevicePointer(&f.host, &s->host->nonfinite, 0)) != cudaSuccess)
+            if ((e = cudaHostGetDevicePointer(&f.host, &s->host->flags, 0)) != cudaSuccess)
                 rc = cuda_fail(e, "fs_create: pinned state block");
         }
         if (rc == FS_OK && (e = cudaMemcpy(s->flags, &f, sizeof(f), cudaMemcpyHostToDevice)) != cudaSuccess)
@@ -1546,6 +1558,11 @@ int fs_set_barrier_poll_limit(fs_solver* s, unsigned polls) {
     DeviceGuard g(s->device);
     // a device word read by every residual solve at launch, so captured step graphs see it too
     CK(cudaMemcpyAsync(s->flags + 1, &polls, sizeof(unsigned), cudaMemcpyHostToDevice, s->stream));
+    // the waits for prefetched tiles take it as a launch parameter
+    if (s->cfg.pressure_tolerance > 0.f && s->prefetch_polls != polls) {
+        s->prefetch_polls = polls;
+        destroy_graph(s);
+    }
     CK(cudaStreamSynchronize(s->stream));
     return FS_OK;
 }

@@ -440,30 +440,51 @@ __device__ __forceinline__ void prefetch_tile(const StencilField& F, int ty, int
         tma_load(dst + R * row, mk, gx, border ? gyb - 1 : gyb, bar);
     }
 }
-// Waits for the warp's prefetch; false when it gave up (a bound, and the same again).
+// Waits for the warp's prefetch, the same answer in every lane; false when the wait gave up:
+// after `polls` polls of about 120 ns, or without such a bound after 2^20 suspending tries
+// (1.3 us each).
 constexpr unsigned kStageWait = 1u << 20;
-__device__ __forceinline__ bool stage_wait(uint64_t* bar, unsigned parity) {
-    for (unsigned k = 0; k < 2 * kStageWait; ++k)
-        if (tc::mbar_try_wait(bar, parity)) return true;
-    return false;
+__device__ __forceinline__ bool stage_wait(uint64_t* bar, unsigned parity, unsigned polls) {
+    unsigned left = polls != 0 ? polls : kStageWait;
+    bool there;
+    while (!(there = polls != 0 ? tc::mbar_test_wait(bar, parity) : tc::mbar_try_wait(bar, parity)) && --left != 0)
+        if (polls != 0) __nanosleep(100);
+    return __all_sync(0xffffffffu, there);
+}
+// After a wait that gave up: the copy may still be on its way into the warp's rows, so one more
+// bounded wait, that it does not outlive the CTA, and NaN in the lane's columns of the rows.
+// Out of line: inlined, its registers cost the residual-driven solve 1 %.
+template <int ROWS>
+__device__ __noinline__ void stage_give_up(uint64_t* bar, unsigned parity, float4* rows) {
+    for (unsigned left = kStageWait; !tc::mbar_try_wait(bar, parity) && --left != 0;) {
+    }
+    const float nan = __int_as_float(0x7fffffff);
+    for (int k = 0; k < ROWS; ++k) rows[k * 32] = make_float4(nan, nan, nan, nan);
 }
 
-// What a warp carries from tile to tile: the parity of its prefetch, and the exchange buffer
-// that the next sweep uses (so that no barrier is needed between tiles).
+// What a warp carries from tile to tile: the parity of its prefetch and whether a wait for one
+// gave up, and the exchange buffer that the next sweep uses (so that no barrier is needed
+// between tiles).
+constexpr unsigned kPhase = 1, kGaveUp = 2;
 struct Carry {
-    unsigned phase = 0;
+    unsigned stage = 0;
     int buf = 0;
+    __device__ __forceinline__ unsigned phase() const { return stage & kPhase; }
+    __device__ __forceinline__ bool gave_up() const { return stage >= kGaveUp; }
 };
 
 // Tile (ty, tx) of one pass: load the region (fusing add_sources or the divergence into the
 // first pass), run n sweeps, store the output tile, then the optional residual
 // partial sums (for residual-driven pressure solves). xin/yout stand in for F.x/F.y so a persistent caller can ping-pong
-// buffers across passes. VEC: the block comes from the prefetch, and `next` starts the next
-// tile's once it has been read.
+// buffers across passes. VEC: the block comes from the prefetch (polls: the bound of the wait
+// for it), and `next` starts the next tile's once it has been read. A warp whose wait gave up
+// fills its staged rows with NaN and prefetches nothing more (its barrier's parity would no
+// longer tell one copy from another), so that this block and all that follow are NaN; the
+// kernel reports it at its end.
 template <int R, int NW, bool DIFF, bool VEC, bool RESID, class Next>
 __device__ __forceinline__ void process_tile(const StencilField& F, int n, int ty, int tx, const float* __restrict__ xin,
                                              float* __restrict__ yout, bool resid, float& rnum, float& rden,
-                                             Carry& carry, Next&& next) {
+                                             Carry& carry, unsigned polls, Next&& next) {
     constexpr int RW = kRegionW;
     constexpr unsigned FULL = 0xffffffffu;
     extern __shared__ float4 smem4[];
@@ -499,7 +520,7 @@ __device__ __forceinline__ void process_tile(const StencilField& F, int n, int t
     }
     const size_t o = (size_t)t.gyb * pitch + t.c0;
     const bool lane_in = t.ncol > 0;
-    const float4* const S = stage_ptr<R, NW>() + t.lane;
+    float4* const S = stage_ptr<R, NW>() + t.lane;
 
     float2 X[R][2], K[R][2];
     auto put = [](float2 (&x)[2], float4 v) {
@@ -521,10 +542,13 @@ __device__ __forceinline__ void process_tile(const StencilField& F, int n, int t
     // columns q of this block and rows i that are interior cells of the grid
     auto int_col = [&](int q) { return t.c0 + q >= 1 && q <= t.ncol - 2; };
     auto int_row = [&](int i) { return t.gyb + i >= 1 && i <= t.nrow - 2; };
-    bool arrived = true;
-    if (VEC) {
-        arrived = stage_wait(stage_bar<R, NW>(), carry.phase);
-        carry.phase ^= 1;
+    if (VEC && !carry.gave_up()) {
+        if (stage_wait(stage_bar<R, NW>(), carry.phase(), polls)) {
+            carry.stage ^= kPhase;
+        } else {
+            carry.stage |= kGaveUp;
+            stage_give_up<stage_rows<R>()>(stage_bar<R, NW>(), carry.phase(), S);
+        }
     }
 
     // ------------------------------------------------------------------ load
@@ -589,8 +613,7 @@ __device__ __forceinline__ void process_tile(const StencilField& F, int n, int t
     }
     if (VEC) {
         __syncwarp();  // the block has been read
-        next();
-        if (!arrived) X[0][0].x = __int_as_float(0x7fffffff);  // reported as a non-finite step
+        if (!carry.gave_up()) next();
     }
     if ((DIFF ? F.kind == PASS_DIFFUSE_FIRST : F.kind == PASS_PRESSURE_FIRST) && F.cst_out != nullptr && t.ocol) {
         const int hi = min(t.r_hi, t.nrow);
@@ -816,12 +839,13 @@ __global__ void __launch_bounds__(32 * NW, (NW <= 8 ? 2 : 1))
         else
             walk.start(L.f[nf], nb - L.f[nf].tile_begin, gridDim.x);
         const StencilField& F = L.f[f];
-        process_tile<kR, NW, DIFF, VEC, false>(F, F.sweeps, ty, tx, F.x, F.y, false, rn, rd, carry, [&] {
+        process_tile<kR, NW, DIFF, VEC, false>(F, F.sweeps, ty, tx, F.x, F.y, false, rn, rd, carry, L.polls, [&] {
             if (nb < total) prefetch_tile<kR, NW, DIFF>(L.f[nf], walk.ty, walk.col(), &L.f[nf].mx, &L.f[nf].mk);
         });
         b = nb;
         f = nf;
     }
+    if (carry.gave_up()) report_timeout(L.flags);
 }
 
 // One pass over the fields of a batch of grids of uneven size, up to kMaxWideFields
@@ -858,12 +882,13 @@ __global__ void __launch_bounds__(32 * NW, (NW <= 8 ? 2 : 1)) stencil_wide_kerne
         else
             walk.start(L.f[nf], nb - L.begin[nf], gridDim.x);
         const StencilField& F = L.f[f];
-        process_tile<kR, NW, DIFF, true, false>(F, F.sweeps, ty, tx, F.x, F.y, false, rn, rd, carry, [&] {
+        process_tile<kR, NW, DIFF, true, false>(F, F.sweeps, ty, tx, F.x, F.y, false, rn, rd, carry, 0, [&] {
             if (nb < total) prefetch_tile<kR, NW, DIFF>(L.f[nf], walk.ty, walk.col(), &L.f[nf].mx, &L.f[nf].mk);
         });
         b = nb;
         f = nf;
     }
+    if (carry.gave_up()) report_timeout(L.flags);
 }
 
 // ---------------------------------------------------------------------------
@@ -948,12 +973,13 @@ __global__ void __launch_bounds__(32 * NW, (NW <= 8 ? 2 : 1))
         walk.start(F, blockIdx.x, G);
         // the previous pass's stores, ordered by the grid barrier, before the TMA engine reads
         asm volatile("fence.proxy.async;" ::: "memory");
-        if (blockIdx.x < ntiles) prefetch_tile<kR, NW, false>(F, walk.ty, walk.col(), mx, &F.mk);
+        if (blockIdx.x < ntiles && !carry.gave_up())
+            prefetch_tile<kR, NW, false>(F, walk.ty, walk.col(), mx, &F.mk);
 #pragma unroll 1
         for (unsigned t = blockIdx.x; t < ntiles; t += G) {
             const int ty = walk.ty, tx = walk.col();
             walk.next();
-            process_tile<kR, NW, false, true, true>(F, take * F.sweeps, ty, tx, x, P.p[dst], check, rn, rd, carry, [&] {
+            process_tile<kR, NW, false, true, true>(F, take * F.sweeps, ty, tx, x, P.p[dst], check, rn, rd, carry, 0, [&] {
                 if (t + G < ntiles) prefetch_tile<kR, NW, false>(F, walk.ty, walk.col(), mx, &F.mk);
             });
         }
@@ -1004,6 +1030,7 @@ __global__ void __launch_bounds__(32 * NW, (NW <= 8 ? 2 : 1))
             }
         }
     }
+    if (carry.gave_up()) atomicExch(&P.ctrl->error, 1);
     if (blockIdx.x == 0 && tid == 0) {
         P.ctrl->passes = (P.segment ? P.ctrl->passes : 0) + passes;
         P.ctrl->residual = ratio;

@@ -42,7 +42,7 @@ extern "C" {
 #define FS_ERR_CUDA 2         /* a CUDA runtime call failed; see fs_last_error() */
 #define FS_ERR_NONFINITE 3    /* the step produced a NaN or Inf (state is still updated) */
 #define FS_ERR_NOT_CONVERGED 4/* residual-driven pressure solve hit its iteration cap */
-#define FS_ERR_TIMEOUT 5      /* a bounded host wait ran out */
+#define FS_ERR_TIMEOUT 5      /* a bounded wait ran out */
 #define FS_ERR_NOMEM 6        /* device or pinned host allocation failed */
 #define FS_ERR_STATE 7        /* call not valid in the handle's current state */
 
@@ -197,6 +197,11 @@ FS_API int fs_sync(fs_solver* s);
  * (pressure_tolerance > 0), in polls of about 120 ns; 0 restores the default (2^24 polls,
  * about 2 s). When a wait runs out the solve stops, the step's velocity is left
  * unprojected and fs_sync / fs_step return FS_ERR_TIMEOUT; the handle stays usable.
+ * On such a handle it also bounds the waits for the tiles that a diffusion pass has under way
+ * (default, and for every other pass and handle: about 1.4 s). When such a wait runs out, the
+ * cells that needed the tile become NaN and the next fs_sync / fs_step / fs_batch_sync returns
+ * FS_ERR_TIMEOUT, whatever check_finite is; upload a state before going on.
+ * fs_project_noalloc has no call that could report it: there the NaN is all there is.
  * The reference has no bounded waits (it has no grid-wide synchronisation at all). */
 FS_API int fs_set_barrier_poll_limit(fs_solver* s, unsigned polls);
 
