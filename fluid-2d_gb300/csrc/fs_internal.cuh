@@ -37,9 +37,10 @@ struct StencilField {
     // tensor maps of x and of the second array (x2 or cst), set by the launchers
     CUtensorMap mx, mk;
     // inputs
-    const float* x;     // state in: x (diffuse), p (pressure; may be null = zero start), u (pressure first)
+    const float* x;     // state in: x (diffuse), p (pressure), u (pressure first)
     const float* x2;    // sources s (diffuse first) or v (pressure first)
-    const float* cst;   // x0 (diffuse) or div (pressure) for non-first passes
+    const float* cst;   // non-first passes: x0 (diffuse) or div (pressure); pressure first: the
+                        // start (null: zero)
     // outputs
     float* y;           // state out (x or p); null: none (a pass of no sweeps)
     float* cst_out;     // first pass: x0 or div out

@@ -1064,10 +1064,16 @@ template <int NW> cudaError_t prepare_variant() {
     return e;
 }
 
+// Whether the two arrays that a pass reads are there: a launch without one is refused, since the
+// kernels read both whatever they are.
+const float* second_array(const StencilField& f) {
+    return f.kind == PASS_DIFFUSE_FIRST || f.kind == PASS_PRESSURE_FIRST ? f.x2 : f.cst;
+}
+bool complete(const StencilField& f) { return f.x != nullptr && second_array(f) != nullptr; }
+
 // Tensor map of a field's rows in boxes of `box` rows x 128 columns (base and pitch 16-byte
-// aligned); a null base leaves the map zero.
+// aligned).
 cudaError_t encode_map(CUtensorMap* map, const float* base, int rows, int cols, int pitch, int box) {
-    if (!base) return cudaSuccess;
     using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                 const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -1087,12 +1093,12 @@ cudaError_t encode_map(CUtensorMap* map, const float* base, int rows, int cols, 
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
 }
 
+cudaError_t encode_second(StencilField& f) {
+    return encode_map(&f.mk, second_array(f), f.rows, f.cols, f.pitch, f.kind == PASS_PRESSURE_FIRST ? kR + 2 : kR);
+}
 cudaError_t encode_field(StencilField& f) {
-    const bool first = f.kind == PASS_DIFFUSE_FIRST || f.kind == PASS_PRESSURE_FIRST;
-    cudaError_t e = encode_map(&f.mx, f.x, f.rows, f.cols, f.pitch, kR);
-    if (e == cudaSuccess)
-        e = encode_map(&f.mk, first ? f.x2 : f.cst, f.rows, f.cols, f.pitch, f.kind == PASS_PRESSURE_FIRST ? kR + 2 : kR);
-    return e;
+    const cudaError_t e = encode_map(&f.mx, f.x, f.rows, f.cols, f.pitch, kR);
+    return e == cudaSuccess ? encode_second(f) : e;
 }
 
 template <int NW>
@@ -1151,6 +1157,7 @@ cudaError_t launch_variant(StencilLaunch& L, cudaStream_t st) {
     int blocks = 0;
     bool vec = true;
     for (int i = 0; i < L.nfields; ++i) {
+        if (!complete(L.f[i])) return cudaErrorInvalidValue;
         blocks += L.f[i].tiles_x * L.f[i].tiles_y;
         vec = vec && vector_rows(L.f[i]);
     }
@@ -1227,9 +1234,9 @@ cudaError_t pressure_solve_max_blocks(int tile_rows, int* blocks) {
 }
 
 cudaError_t launch_pressure_solve(PressureSolve& P, int tile_rows, int blocks, cudaStream_t st) {
-    if (blocks <= 0) return cudaErrorInvalidValue;
+    if (blocks <= 0 || !complete(P.first) || !P.mid.cst || !P.p[0] || !P.p[1]) return cudaErrorInvalidValue;
     cudaError_t e = encode_field(P.first);
-    if (e == cudaSuccess) e = encode_field(P.mid);
+    if (e == cudaSuccess) e = encode_second(P.mid);  // its field is p[0] or p[1]
     for (int k = 0; k < 2 && e == cudaSuccess; ++k)
         e = encode_map(&P.mp[k], P.p[k], P.mid.rows, P.mid.cols, P.mid.pitch, kR);
     if (e != cudaSuccess) return e;
@@ -1239,7 +1246,8 @@ cudaError_t launch_pressure_solve(PressureSolve& P, int tile_rows, int blocks, c
 
 cudaError_t prepare_stencil_wide(WideLaunch& L) {
     cudaError_t e = cudaSuccess;
-    for (int i = 0; i < L.nfields && e == cudaSuccess; ++i) e = encode_field(L.f[i]);
+    for (int i = 0; i < L.nfields && e == cudaSuccess; ++i)
+        e = complete(L.f[i]) ? encode_field(L.f[i]) : cudaErrorInvalidValue;
     return e;
 }
 
