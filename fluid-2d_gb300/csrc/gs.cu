@@ -292,7 +292,7 @@ __device__ __forceinline__ void gs_chunk(const GsBand<DIFF, PLACE>& B, bool firs
 // (ONE) between bands.
 template <bool DIFF, int PLACE, bool ONE>
 __global__ void __launch_bounds__(32 * kMaxWarps) gs_solve_kernel(const __grid_constant__ GsSolve S) {
-    __shared__ int s_stop;
+    __shared__ int s_stop[2];  // a warp gave up in an even, an odd chunk
     __shared__ __align__(16) float s_mail[kMaxWarps][2 * kChunk];
     const int m = S.n - 2, lines = gs_lines(m);
     const int array = (lines + 1) * kLine;
@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps) gs_solve_kernel(const __grid_c
     const int in_flight = ONE ? (int)(blockDim.x >> 5) / S.bands : S.sweeps;
     const unsigned lim_set = S.poll_limit ? __ldcg(S.poll_limit) : 0u;
     const unsigned limit = lim_set ? lim_set : kGsPolls;
-    if (threadIdx.x == 0) s_stop = 0;
+    if (threadIdx.x == 0) s_stop[0] = s_stop[1] = 0;
     for (int item = blockIdx.x; item < (ONE ? S.nf : S.nf * S.bands); item += gridDim.x) {
         const int fi = ONE ? item : item / S.bands;
         const GsField& F = S.f[fi];
@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps) gs_solve_kernel(const __grid_c
         const int total = lines + S.lag * (S.sweeps - 1) + (ONE ? S.band_lag * (S.bands - 1) : 0);
         // chunk q; word, xr, cc: its import, loaded two chunks before, and its lines, loaded one
         // before; next, xn, cn: the next chunk's
-        auto chunk = [&](int q, unsigned long long& word, unsigned long long& next, float (&xr)[kChunk],
+        auto chunk = [&](int q, int& stop, unsigned long long& word, unsigned long long& next, float (&xr)[kChunk],
                          float (&cc)[kChunk], float (&xn)[kChunk], float (&cn)[kChunk]) {
             if (ONE && q * kChunk - s * S.lag - start >= lines) s += in_flight;
             const int t0 = q * kChunk - s * S.lag - start;
@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(32 * kMaxWarps) gs_solve_kernel(const __grid_c
                         if (++polls > limit || ((polls & 63u) == 0 && *(volatile int*)&S.ctrl->error != 0)) {
                             if (lane == 0) {
                                 atomicExch(&S.ctrl->error, 1);
-                                *(volatile int*)&s_stop = 1;
+                                *(volatile int*)&stop = 1;
                             }
                             break;
                         }
@@ -430,13 +430,15 @@ __global__ void __launch_bounds__(32 * kMaxWarps) gs_solve_kernel(const __grid_c
                 }
             }
             __syncthreads();
-            return ONE || *(volatile int*)&s_stop == 0;  // the same for every thread after the barrier
+            // the same for every thread: a faster warp may write the next chunk's word already,
+            // but this one not before the next barrier
+            return ONE || *(volatile int*)&stop == 0;
         };
         unsigned long long wa = 0, wb = 0;
 #pragma unroll 1
         for (int q = 0; q * kChunk < total; q += 2) {
-            if (!chunk(q, wa, wb, xa, ca, xb, cb)) return;
-            if (!chunk(q + 1, wb, wa, xb, cb, xa, ca)) return;
+            if (!chunk(q, s_stop[0], wa, wb, xa, ca, xb, cb)) return;
+            if (!chunk(q + 1, s_stop[1], wb, wa, xb, cb, xa, ca)) return;
         }
         B.store(part, parts);
     }
