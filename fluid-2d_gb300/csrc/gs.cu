@@ -24,8 +24,10 @@
 // chunks before their use (a load of another SM's store takes longer than a chunk).
 // Waits are bounded: a warp that gives up sets ctrl->error and the solve ends
 // (FS_ERR_TIMEOUT on the host). All CTAs are co-resident (cooperative launch); a CTA with
-// several bands takes every gridDim.x-th in turn, which cannot deadlock because a band's
-// sweeps reach at most as many bands ahead as a launch has sweeps.
+// several bands takes every gridDim.x-th in turn, which cannot deadlock: a band's last sweep
+// needs one sweep less of the band below, two less of the next, so at most as many bands as a
+// launch has sweeps, and the lowest unfinished band and the gridDim.x - 1 after it are all
+// under way (solve() keeps a launch's sweeps at or below the SMs, and so the CTAs).
 //
 // Grids whose bands all fit one SM's shared memory (up to 141 x 141) run in one CTA per
 // field instead, bands side by side, so that nothing leaves the SM.
@@ -722,7 +724,11 @@ cudaError_t launch_placed(GsSolve& S, cudaStream_t st) {
 
 // All sweeps of a solve, kMaxWarps to a launch where a warp runs one sweep.
 cudaError_t solve(GsSolve S, bool diff, int sweeps, unsigned& epoch, cudaStream_t st, int* launches) {
-    const int most = one_cta(S.n) ? sweeps : kMaxWarps;
+    int dev = 0, sms = 0;
+    cudaError_t q = cudaGetDevice(&dev);
+    if (q == cudaSuccess) q = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (q != cudaSuccess) return q;
+    const int most = one_cta(S.n) ? sweeps : std::min(kMaxWarps, sms);
     for (int done = 0; done < sweeps;) {
         S.sweeps = std::min(most, sweeps - done);
         S.epoch = ++epoch;
