@@ -289,7 +289,9 @@ __global__ void __launch_bounds__(256) conv3x3_ref_kernel(const ConvArgs P, cons
 // range of slots in chunks of 128 (eight K = 16 MMAs per tile), double-buffered: the copies
 // of chunk s + 1 run while chunk s is multiplied. The CTA writes its 289 x 32 partial sums
 // to a workspace and wgrad_reduce_kernel adds the CTAs' partials in a fixed order, so the
-// gradient is deterministic.
+// gradient is deterministic. The product of a border slot's zero gradient with the pixel next
+// to it is zero unless that pixel is not finite; NaN in a row that has such products (dx = 0
+// and 2) is therefore summed again over the pixels alone (wgrad_row_again).
 // 65,536 pixels: 13.3 us (ncu, cold caches; 25 us where the threads loaded the nine taps of 64 pixels at a
 // time and transposed them), bound by the latency of a CTA's two to four chunks.
 constexpr int kWgK = kTileM;               // slots per chunk
@@ -307,6 +309,27 @@ struct WgradArgs {
     int per;                  // slots per CTA (a multiple of kWgK)
     int* err;
 };
+
+// The NaN of one row (tap dy, dx and channel ci) of a CTA's partial result, summed once more
+// over the pixels of slots [pbeg, pend) in order.
+__device__ __noinline__ void wgrad_row_again(const WgradArgs& P, float* out, int dy, int dx, int ci, long pbeg,
+                                             long pend) {
+    for (int c = 0; c < kC; ++c) {
+        if (!isnan(out[c])) continue;
+        float acc = 0.f;
+        for (long s = pbeg; s < pend; ++s) {
+            const long y = s / (P.W + 2);
+            const int xx = (int)(s - y * (P.W + 2)) - 1;
+            if (xx < 0 || xx >= P.W) continue;
+            const int ly = (int)(y % P.img_h) + dy - 1, ix = xx + dx - 1;
+            const long iy = y + dy - 1, src = P.up ? (iy >> 1) * (P.W >> 1) + (ix >> 1) : iy * P.W + ix;
+            const bool in = ly >= 0 && ly < P.img_h && ix >= 0 && ix < P.W;
+            const float x = in ? __bfloat162float(P.x[src * kC + ci]) : 0.f;
+            acc = fmaf(x, __bfloat162float(P.dz[(y * P.W + xx) * kC + c]), acc);
+        }
+        out[c] = acc;
+    }
+}
 
 __global__ void __launch_bounds__(kWgThreads) wgrad_tc_kernel(const WgradArgs P) {
     extern __shared__ __align__(1024) uint8_t sm[];
@@ -426,6 +449,10 @@ __global__ void __launch_bounds__(kWgThreads) wgrad_tc_kernel(const WgradArgs P)
 #pragma unroll
                 for (int q = 0; q < 8; ++q) o[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
             }
+            bool nan = false;
+#pragma unroll
+            for (int c = 0; c < 32; ++c) nan |= isnan(v[c]);
+            if (nan && dx != 1 && f < kK) wgrad_row_again(P, out + (size_t)f * kC, dy, dx, lane, pbeg, pend);
         }
     }
     tc::fence_before_sync();
