@@ -315,7 +315,7 @@ struct GsFields {
     float* dif[3];
     float* vel[2];
     float* p;
-    int *head, *next;
+    int *head, *next, *cells;
     void* words;
     SolveCtrl* ctrl;            // error flag of the waits between SMs
     const unsigned* poll_limit; // device word: polls before such a wait gives up (0 = default)

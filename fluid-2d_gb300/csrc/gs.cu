@@ -39,8 +39,8 @@
 //
 // The splat keeps the host solver's order of additions to every cell: a cell receives
 // its contributions in the raster order of their source cells. Source cells are linked
-// into one list per target, and each cell sorts the few it receives; cells that receive
-// very many fall back to one thread that applies all sources in order.
+// into one list per target, and a thread sorts the few that its cell receives; a cell that
+// receives more gets a warp, or a CTA.
 //
 // Every operation uses explicitly rounded single-precision intrinsics so that no
 // contraction changes a result; the outputs are bit-identical to the host solver's.
@@ -525,14 +525,17 @@ __global__ void __launch_bounds__(256) gs_gather_kernel(const GsVel A) {
 struct GsSplat {
     const float *d, *u, *v;  // diffused density, the step's initial velocity
     float* out;
-    int* head;  // per target cell: the last source linked to it (-1: none)
-    int* next;  // per source cell: the source linked before it
-    int* many;  // set when a cell receives more sources than kGsMost
+    int* head;   // per target cell: the last source linked to it (-1: none)
+    int* next;   // per source cell: the source linked before it
+    int* crowd;    // [0], [1]: cells on the lists below so far, [2]: the farthest a source moves
+    int* cells;    // the cells that receive more than kGsSorted sources
+    int* crowded;  // those of them that receive more than kGsBunch
     int n, P;
     float dt0;
 };
-constexpr int kGsSorted = 24;  // sources a thread sorts in its own array
-constexpr int kGsMost = 256;   // more go to the in-order form
+constexpr int kGsSorted = 24;  // sources that a thread sorts in its own array
+constexpr int kGsBunch = 128;  // sources that a warp sorts in shared memory
+constexpr int kGsCrowdThreads = 1024, kGsListed = kGsCrowdThreads;  // sources that a CTA sorts
 
 // Target cell and offsets of source (i, j) (fluid_solver_cpu.cpp:132-139); false when the
 // source leaves the grid (a NaN position too).
@@ -551,110 +554,195 @@ __device__ __forceinline__ bool gs_target(const GsSplat& A, int i, int j, int& i
 
 __global__ void __launch_bounds__(256) gs_link_kernel(const GsSplat A) {
     const int j = 1 + blockIdx.x * 32 + threadIdx.x, i = 1 + blockIdx.y * 8 + threadIdx.y;
-    if (i > A.n - 2 || j > A.n - 2) return;
-    int i0, j0;
+    int i0, j0, far = 0;
     float s0, s2;
-    if (!gs_target(A, i, j, i0, j0, s0, s2)) return;
-    const int o = i * A.P + j;
-    A.next[o] = atomicExch(A.head + (i0 * A.P + j0), o);
+    if (i <= A.n - 2 && j <= A.n - 2 && gs_target(A, i, j, i0, j0, s0, s2)) {
+        const int o = i * A.P + j;
+        A.next[o] = atomicExch(A.head + (i0 * A.P + j0), o);
+        far = max(abs(i0 - i), abs(j0 - j));
+    }
+    far = __reduce_max_sync(0xffffffffu, far);
+    if (threadIdx.x == 0 && far > __ldcg(A.crowd + 2)) atomicMax(A.crowd + 2, far);
 }
 
-// Contribution of source o to the cell at offset (di, dj) from its target.
-__device__ __forceinline__ float gs_share(const GsSplat& A, int o, int di, int dj) {
-    const int i = o / A.P, j = o - i * A.P;
+// What a source adds to the cell at offset (di, dj) from its target.
+__device__ __forceinline__ float gs_weighted(float s0, float s2, int di, int dj, float d) {
+    const float wx = dj ? s0 : __fsub_rn(1.f, s0), wy = di ? s2 : __fsub_rn(1.f, s2);
+    return __fmul_rn(__fmul_rn(wx, wy), d);
+}
+// The same of source o (source * 4 + corner).
+__device__ __forceinline__ float gs_share(const GsSplat& A, int source) {
+    const int o = source >> 2, i = o / A.P, j = o - i * A.P;
     int i0, j0;
     float s0, s2;
     gs_target(A, i, j, i0, j0, s0, s2);
-    const float wx = dj ? s0 : __fsub_rn(1.f, s0), wy = di ? s2 : __fsub_rn(1.f, s2);
-    return __fmul_rn(__fmul_rn(wx, wy), __ldg(A.d + o));
+    return gs_weighted(s0, s2, (source >> 1) & 1, source & 1, __ldg(A.d + o));
 }
 
 // Sum of the contributions to interior cell (i, j) in the raster order of their sources
-// (advect(trace=true), fluid_solver_cpu.cpp:127-152).
-__device__ float gs_collect(const GsSplat& A, int i, int j) {
+// (advect(trace=true), fluid_solver_cpu.cpp:127-152); false when there are too many.
+__device__ bool gs_collect(const GsSplat& A, int i, int j, float& acc) {
     int src[kGsSorted];  // source * 4 + corner; a source reaches a cell through one corner
     int cnt = 0;
     for (int c = 0; c < 4; ++c) {
         const int di = c >> 1, dj = c & 1;
         for (int o = __ldcg(A.head + ((i - di) * A.P + j - dj)); o >= 0; o = __ldcg(A.next + o)) {
-            if (cnt < kGsSorted) {
-                int k = cnt;
-                for (; k > 0 && (src[k - 1] >> 2) > o; --k) src[k] = src[k - 1];
-                src[k] = o * 4 + c;
-            }
-            if (++cnt > kGsMost) {
-                atomicExch(A.many, 1);
-                return 0.f;
-            }
+            if (cnt == kGsSorted) return false;
+            int k = cnt++;
+            for (; k > 0 && (src[k - 1] >> 2) > o; --k) src[k] = src[k - 1];
+            src[k] = o * 4 + c;
         }
     }
-    float acc = 0.f;
-    if (cnt <= kGsSorted) {
-        for (int k = 0; k < cnt; ++k) acc = __fadd_rn(acc, gs_share(A, src[k] >> 2, (src[k] >> 1) & 1, src[k] & 1));
-        return acc;
-    }
-    // more than the array holds: the lists once per contribution, next larger source each time
-    int last = -1;
-    for (int k = 0; k < cnt; ++k) {
-        int best = 0x7fffffff, bc = 0;
-        for (int c = 0; c < 4; ++c)
-            for (int o = __ldcg(A.head + ((i - (c >> 1)) * A.P + j - (c & 1))); o >= 0; o = __ldcg(A.next + o))
-                if (o > last && o < best) {
-                    best = o;
-                    bc = c;
-                }
-        acc = __fadd_rn(acc, gs_share(A, best, bc >> 1, bc & 1));
-        last = best;
-    }
-    return acc;
+    acc = 0.f;
+    for (int k = 0; k < cnt; ++k) acc = __fadd_rn(acc, gs_share(A, src[k]));
+    return true;
 }
 
 // One thread per cell; edges and corners repeat or average (their two edge neighbours hold
-// the same value) the inner cell's sum.
+// the same value) the inner cell's sum. Cells with more sources than a thread sorts are left
+// to the kernels below.
+__device__ __forceinline__ float gs_edge(float x, bool corner) { return corner ? __fmul_rn(0.5f, __fadd_rn(x, x)) : x; }
 __global__ void __launch_bounds__(256) gs_splat_kernel(const GsSplat A) {
     const int gj = blockIdx.x * 32 + threadIdx.x, gi = blockIdx.y * 8 + threadIdx.y;
     if (gi >= A.n || gj >= A.n) return;
     const int i = min(max(gi, 1), A.n - 2), j = min(max(gj, 1), A.n - 2);
-    const float x = gs_collect(A, i, j);
-    A.out[(size_t)gi * A.P + gj] = gi != i && gj != j ? __fmul_rn(0.5f, __fadd_rn(x, x)) : x;
+    float x;
+    if (gs_collect(A, i, j, x))
+        A.out[(size_t)gi * A.P + gj] = gs_edge(x, gi != i && gj != j);
+    else if (gi == i && gj == j)
+        A.cells[atomicAdd(A.crowd, 1)] = i * A.P + j;
 }
 
-// Every source in order by one thread, when some cell received more than kGsMost.
-__global__ void __launch_bounds__(1024) gs_splat_in_order_kernel(const GsSplat A) {
-    if (*A.many == 0) return;
-    const int n = A.n, P = A.P;
-    float* g = A.out;
-    for (int e = threadIdx.x; e < n * n; e += blockDim.x) g[(size_t)(e / n) * P + e % n] = 0.f;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int i = 1; i < n - 1; ++i)
-            for (int j = 1; j < n - 1; ++j) {
-                int i0, j0;
-                float s0, s2;
-                if (!gs_target(A, i, j, i0, j0, s0, s2)) continue;
-                const float s1 = __fsub_rn(1.f, s0), s3 = __fsub_rn(1.f, s2);
-                const float w = A.d[(size_t)i * P + j];
-                // edge cells that this adds to are filled below
-                float* t = g + (size_t)i0 * P + j0;
-                t[0] = __fadd_rn(t[0], __fmul_rn(__fmul_rn(s1, s3), w));
-                t[P] = __fadd_rn(t[P], __fmul_rn(__fmul_rn(s1, s2), w));
-                t[1] = __fadd_rn(t[1], __fmul_rn(__fmul_rn(s0, s3), w));
-                t[P + 1] = __fadd_rn(t[P + 1], __fmul_rn(__fmul_rn(s0, s2), w));
-            }
+// acc and the first cnt of v (16-byte aligned) one after another, by one thread.
+__device__ float gs_add_up(float acc, const float* v, int cnt) {
+    int k = 0;
+#pragma unroll 1
+    for (; k + 8 <= cnt; k += 8) {
+        const float4 a = *reinterpret_cast<const float4*>(v + k), b = *reinterpret_cast<const float4*>(v + k + 4);
+        const float t[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc = __fadd_rn(acc, t[e]);
     }
-    __syncthreads();
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        const int c = min(max(k, 1), n - 2);
-        const float w = g[(size_t)c * P + 1], e = g[(size_t)c * P + n - 2], t = g[P + c], b = g[(size_t)(n - 2) * P + c];
-        if (k == c) {
-            g[(size_t)k * P] = w;
-            g[(size_t)k * P + n - 1] = e;
-            g[k] = t;
-            g[(size_t)(n - 1) * P + k] = b;
-        } else {  // corners: (0, 0) and (0, n-1), or (n-1, 0) and (n-1, n-1)
-            g[(size_t)k * P] = __fmul_rn(0.5f, __fadd_rn(w, w));
-            g[(size_t)k * P + n - 1] = __fmul_rn(0.5f, __fadd_rn(e, e));
+    for (; k < cnt; ++k) acc = __fadd_rn(acc, v[k]);
+    return acc;
+}
+// A cell's sum to the cell, and to the edges and the corner that repeat it, by one thread.
+__device__ void gs_put_sum(const GsSplat& A, int i, int j, float x) {
+    for (int gi : {i, i == 1 ? 0 : -1, i == A.n - 2 ? A.n - 1 : -1})
+        for (int gj : {j, j == 1 ? 0 : -1, j == A.n - 2 ? A.n - 1 : -1})
+            if (gi >= 0 && gj >= 0) A.out[(size_t)gi * A.P + gj] = gs_edge(x, gi != i && gj != j);
+}
+
+// Cells of up to kGsBunch sources, a warp each in turn: four lanes walk the four lists (0.35 us
+// a link), the warp sorts what they find by rank and one lane adds. Others go on to
+// gs_crowd_kernel.
+constexpr int kGsBunchWarps = 8;
+__global__ void __launch_bounds__(32 * kGsBunchWarps) gs_bunch_kernel(const GsSplat A) {
+    __shared__ int lists[kGsBunchWarps][kGsBunch];
+    __shared__ __align__(16) float shares[kGsBunchWarps][kGsBunch];
+    constexpr unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, cells = __ldcg(A.crowd);
+    int* const list = lists[w];
+    float* const share = shares[w];
+    for (int q = blockIdx.x * kGsBunchWarps + w; q < cells; q += gridDim.x * kGsBunchWarps) {
+        const int cell = __ldcg(A.cells + q), i = cell / A.P, j = cell - i * A.P;
+        int o = lane < 4 ? __ldcg(A.head + ((i - (lane >> 1)) * A.P + j - (lane & 1))) : -1, cnt = 0;
+        for (unsigned m; cnt <= kGsBunch && (m = __ballot_sync(FULL, o >= 0)) != 0;) {
+            const int k = cnt + __popc(m & ((1u << lane) - 1));
+            cnt += __popc(m);
+            if (o >= 0) {
+                if (k < kGsBunch) list[k] = o * 4 + lane;
+                o = __ldcg(A.next + o);
+            }
         }
+        __syncwarp();
+        if (cnt > kGsBunch) {
+            if (lane == 0) A.crowded[atomicAdd(A.crowd + 1, 1)] = cell;
+            continue;
+        }
+        for (int e = lane; e < cnt; e += 32) {
+            const int mine = list[e];
+            int place = 0;  // the sources before it
+#pragma unroll 8
+            for (int k = 0; k < cnt; ++k) place += list[k] < mine;
+            share[place] = gs_share(A, mine);
+        }
+        __syncwarp();
+        if (lane == 0) gs_put_sum(A, i, j, gs_add_up(0.f, share, cnt));
+        __syncwarp();
+    }
+}
+
+// Cells of more sources, a CTA each in turn. Every source that could reach the cell, those
+// within the farthest move of any source, is looked at in raster order, a thousand at a time
+// (about 1 us); those that do reach it are packed, and one thread adds them while the others
+// look on. Where the cell's lists are shorter than that takes (0.35 us a link), they are walked
+// and sorted instead. A step at 800 x 800 (1.6 ms, 1.8 with the flow that makes the crowd), ms
+// with n sources in a cell, and where a thread walked its cell's lists once per source up to
+// 256 and one thread applied all sources beyond: 149 1.84 and 7.7, 253 1.85 and 20.7, 11289
+// 1.91 and 144, all 640,000 4.7 and 130.
+__global__ void __launch_bounds__(kGsCrowdThreads) gs_crowd_kernel(const GsSplat A) {
+    constexpr int T = kGsCrowdThreads;
+    __shared__ int list[kGsListed];
+    __shared__ __align__(16) float share[T];
+    __shared__ int hits[T / 32];
+    __shared__ int s_count;
+    static_assert(T / 32 == 32, "a warp's lanes hold the warps' counts");
+    const int crowded = __ldcg(A.crowd + 1), reach = __ldcg(A.crowd + 2) + 1;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, n = A.n, P = A.P;
+    for (int q = blockIdx.x; q < crowded; q += gridDim.x) {
+        const int cell = __ldcg(A.crowded + q), i = cell / P, j = cell - i * P;
+        const int top = max(1, i - reach), left = max(1, j - reach);
+        const int cols = min(n - 2, j + reach) - left + 1, box = (min(n - 2, i + reach) - top + 1) * cols;
+        const int most = min(kGsListed, 3 * (box / T));  // links worth walking
+        float acc = 0.f;
+        int cnt = kGsListed + 1;
+        if (most > kGsBunch) {
+            if (tid == 0) s_count = 0;
+            __syncthreads();
+            if (lane == 0 && w < 4)
+                for (int o = __ldcg(A.head + ((i - (w >> 1)) * P + j - (w & 1))); o >= 0; o = __ldcg(A.next + o)) {
+                    const int k = atomicAdd(&s_count, 1);
+                    if (k >= most) break;
+                    list[k] = o * 4 + w;
+                }
+            __syncthreads();
+            cnt = s_count;
+        }
+        if (cnt <= most) {
+            if (tid < cnt) {
+                const int mine = list[tid];
+                int place = 0;
+#pragma unroll 8
+                for (int k = 0; k < cnt; ++k) place += list[k] < mine;
+                share[place] = gs_share(A, mine);
+            }
+            __syncthreads();
+            if (tid == 0) acc = gs_add_up(acc, share, cnt);
+        } else {
+            for (int e0 = 0; e0 < box; e0 += T) {
+                const int e = e0 + tid, r = e / cols, si = top + r, sj = left + e - r * cols;
+                int i0, j0;
+                float s0, s2, mine = 0.f;
+                bool hit = e < box && gs_target(A, si, sj, i0, j0, s0, s2);
+                if (hit) {
+                    const int di = i - i0, dj = j - j0;
+                    hit = (unsigned)(di | dj) <= 1u;
+                    if (hit) mine = gs_weighted(s0, s2, di, dj, __ldg(A.d + (size_t)si * P + sj));
+                }
+                const unsigned m = __ballot_sync(0xffffffffu, hit);
+                if (lane == 0) hits[w] = __popc(m);
+                __syncthreads();
+                const int h = hits[lane];
+                const int before = __reduce_add_sync(0xffffffffu, lane < w ? h : 0);
+                cnt = __reduce_add_sync(0xffffffffu, h);
+                if (hit) share[before + __popc(m & ((1u << lane) - 1))] = mine;
+                __syncthreads();
+                if (tid == 0) acc = gs_add_up(acc, share, cnt);
+            }
+        }
+        if (tid == 0) gs_put_sum(A, i, j, acc);
+        __syncthreads();
     }
 }
 
@@ -784,8 +872,8 @@ cudaError_t gs_step(const GsFields& G, int n, int pitch, int kd, int kp, float d
     S.cdiv = -0.5f * h;
     S.ctrl = G.ctrl;
     S.poll_limit = G.poll_limit;
-    // the words' tags and the splat's overflow flag start at zero, the lists empty
-    int* many = reinterpret_cast<int*>(G.words);
+    // the words' tags and the splat's counts start at zero, the lists empty
+    int* crowd = reinterpret_cast<int*>(G.words);
     S.words = reinterpret_cast<unsigned long long*>(G.words) + 32;
     const int max_bands = (n - 2 + 31) / 32;
     GS_CK(cudaMemsetAsync(G.words, 0, 256 + (size_t)3 * max_bands * 2 * (n - 2) * 8, st));
@@ -825,13 +913,18 @@ cudaError_t gs_step(const GsFields& G, int n, int pitch, int kd, int kp, float d
     // density on the side stream
     GS_CK(cudaEventRecord(G.fork, st));
     GS_CK(cudaStreamWaitEvent(G.side, G.fork, 0));
-    const GsSplat A{G.dif[0], G.state[1], G.state[2], G.state[0], G.head, G.next, many, n, pitch, dt0};
+    const GsSplat A{G.dif[0], G.state[1], G.state[2], G.state[0], G.head, G.next, crowd, G.cells,
+                    G.cells + (size_t)n * pitch / 2, n, pitch, dt0};
     GS_CK(cudaMemsetAsync(G.head, 0xff, (size_t)n * pitch * sizeof(int), G.side));
     gs_link_kernel<<<cells2, threads, 0, G.side>>>(A);
     gs_splat_kernel<<<cells2, threads, 0, G.side>>>(A);
-    gs_splat_in_order_kernel<<<1, 1024, 0, G.side>>>(A);
+    int dev = 0, sms = 0;
+    GS_CK(cudaGetDevice(&dev));
+    GS_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    gs_bunch_kernel<<<4 * sms, 32 * kGsBunchWarps, 0, G.side>>>(A);
+    gs_crowd_kernel<<<sms, kGsCrowdThreads, 0, G.side>>>(A);
     GS_CK(cudaGetLastError());
-    *launches += 3;
+    *launches += 4;
     GS_CK(cudaEventRecord(G.join, G.side));
     // velocity
     auto project = [&](const float* u, const float* v, float* uo, float* vo) -> cudaError_t {

@@ -949,7 +949,8 @@ int enqueue_step(fs_solver* s, float diff, float visc, float dt, Counter& cnt) {
         F.p = scratch(11);
         F.head = reinterpret_cast<int*>(scratch(12));
         F.next = reinterpret_cast<int*>(scratch(13));
-        F.words = scratch(14);
+        F.cells = reinterpret_cast<int*>(scratch(14));
+        F.words = scratch(15);
         F.ctrl = s->ctrl;
         F.poll_limit = reinterpret_cast<const unsigned*>(s->flags + 1);
         F.side = s->side;
