@@ -322,7 +322,7 @@ struct GsFields {
     cudaStream_t side;          // the splat's stream, forked and joined by the events
     cudaEvent_t fork, join;
 };
-int gs_one_cta_size();            // largest n without waits between CTAs
+bool gs_one_cta(int n);            // whether solves of size n need no waits between CTAs
 int gs_tiled_max_size();           // largest n the method accepts (0: no device)
 cudaError_t gs_prepare();          // shared-memory opt-in on the current device, outside capture
 cudaError_t gs_step(const GsFields& F, int n, int pitch, int kd, int kp, float diff, float visc, float dt,

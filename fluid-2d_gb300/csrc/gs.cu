@@ -831,11 +831,7 @@ cudaError_t solve(GsSolve S, bool diff, int sweeps, unsigned& epoch, cudaStream_
 
 }  // namespace
 
-int gs_one_cta_size() {
-    int n = 3;
-    while (one_cta(n + 1)) ++n;
-    return n;
-}
+bool gs_one_cta(int n) { return one_cta(n); }
 
 int gs_tiled_max_size() { return smem_limit() > 0 ? 16384 : 0; }
 

@@ -119,6 +119,7 @@ struct fs_solver {
     };
     HostState own_host{};
     HostState* host = nullptr;
+    bool gs_waits = false;        // Gauss-Seidel solves with waits between CTAs
     unsigned prefetch_polls = 0;  // StencilLaunch::polls
     bool direct_host = false;     // kernels can address pageable host memory
     // residual-driven pressure solves: one control block per projection of a step,
@@ -1054,8 +1055,7 @@ int read_solve_ctrl(const fs_solver* s, SolveCtrl* out) {
 // Whether a step's solves have an outcome that no sync has reported yet: residual solves,
 // and Gauss-Seidel solves with waits between CTAs.
 bool unreported_solves(const fs_solver* s) {
-    const bool gs = s->cfg.method == FS_METHOD_GAUSS_SEIDEL;
-    return (gs ? s->rows > gs_one_cta_size() : s->cfg.pressure_tolerance > 0.f) && s->stats.steps > 0 &&
+    return (s->gs_waits || s->cfg.pressure_tolerance > 0.f) && s->stats.steps > 0 &&
            s->steps_reported != s->stats.steps;
 }
 
@@ -1336,7 +1336,10 @@ int fs_create(const fs_config* cfg, fs_solver** out) {
     cudaError_t e = stencil_prepare();
     if (e == cudaSuccess) e = pressure_solve_max_blocks(s->tile_rows, &s->solve_blocks);
     if (e == cudaSuccess && cfg->pressure_tolerance > 0.f) e = pressure_solve_max_blocks(128, &s->solve_blocks_tall);
-    if (e == cudaSuccess && cfg->method == FS_METHOD_GAUSS_SEIDEL) e = gs_prepare();
+    if (e == cudaSuccess && cfg->method == FS_METHOD_GAUSS_SEIDEL) {
+        e = gs_prepare();
+        s->gs_waits = !gs_one_cta(cfg->rows);
+    }
     if (e != cudaSuccess) {
         delete s;
         return cuda_fail(e, "fs_create: stencil kernel set-up");
