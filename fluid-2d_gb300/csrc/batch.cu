@@ -402,8 +402,7 @@ int fs_batch_create(const fs_config* cfg, int count, const int* rows, const int*
         return fail(FS_ERR_CUDA, "fs_batch_create: no CUDA device");
     }
     b->device = dev;
-    int access = 0;
-    if (cudaDeviceGetAttribute(&access, cudaDevAttrPageableMemoryAccess, dev) == cudaSuccess) b->direct_host = access != 0;
+    b->direct_host = addresses_host(dev);
     DeviceScope scope(dev);
     b->count = count;
     b->tile_rows = cfg->tile_rows ? cfg->tile_rows : 64;

@@ -47,6 +47,17 @@ inline std::vector<int> plan_passes(int total, int k) {
     return out;
 }
 
+// Whether kernels on the device read and write the host's pageable memory in place, through the
+// host's page tables (a GB300 beside its Grace CPU). Pageable access alone is not enough: where
+// software provides it, each page that a kernel touches moves to the device and back.
+inline bool addresses_host(int dev) {
+    for (cudaDeviceAttr a : {cudaDevAttrPageableMemoryAccess, cudaDevAttrPageableMemoryAccessUsesHostPageTables}) {
+        int has = 0;
+        if (cudaDeviceGetAttribute(&has, a, dev) != cudaSuccess || has == 0) return false;
+    }
+    return true;
+}
+
 // a = dt * float(rows*cols) * rate (fluid_solver_gpu.cu:79) and the FP32 pair whose sum is
 // the reciprocal of the reference's double divisor 1 + 4a.
 inline void field_diffusion(StencilField& f, int rows, int cols, float rate, float dt) {

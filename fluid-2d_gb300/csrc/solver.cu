@@ -1449,9 +1449,7 @@ int fs_create(const fs_config* cfg, fs_solver** out) {
     if (rc == FS_OK && learned && (e = cudaMallocHost(&s->host_ctrl, 2 * sizeof(SolveCtrl))) != cudaSuccess)
         rc = cuda_fail(e, "fs_create: pinned control block");
     if (rc == FS_OK) {
-        int access = 0;
-        if (cudaDeviceGetAttribute(&access, cudaDevAttrPageableMemoryAccess, dev) == cudaSuccess)
-            s->direct_host = access != 0;
+        s->direct_host = addresses_host(dev);
         const bool copies = learned || cfg->pressure_tolerance > 0.f || cfg->method == FS_METHOD_GAUSS_SEIDEL;
         StepFlags f{};
         if (s->direct_host && !copies) {
