@@ -18,11 +18,14 @@
 // one (add_sources x + dt*s and the diffusion numerator x0 + a*sum). The reference divides
 // by D = 1.0 + 4.0*a in double; FP64 is slow on GB300, so the quotient is formed as
 //   q = fma(num, rh, num*rl),   rh + rl = 1/D split into two floats:
-// the error before the last rounding is below 2^-47 of the quotient (the split's and the
-// small product's), so q differs from the correctly rounded quotient only where that lies
-// within such a distance of a rounding boundary: 0 of 2^28 random quotients (a from 1e-4 to
-// 1e4) differed from (float)((double)num / D), against 1 for the Newton-corrected quotient
-// of two more operations that this replaced.
+// the error before the last rounding is below 2^-47 of the quotient (the split's and the small
+// product's) while num*rl is a normal number, and at most 2^-150 more below, so q is the
+// correctly rounded quotient or, where that lies so close to a rounding boundary, the float
+// next to it. 0 of 2^28 random quotients of numerators near one (a from 1e-4 to 1e4) differed
+// from (float)((double)num / D), against 1 for the Newton-corrected quotient of two more
+// operations that this replaced. Of 2^24 at each smaller magnitude, this and Newton: none down
+// to 2^-92; 133 and 0 at 2^-100, 3 % and 0.3 % at 2^-120, 0.6 % and 4.6 % at 2^-130, none by
+// more than one unit in the last place.
 
 #include <algorithm>
 
