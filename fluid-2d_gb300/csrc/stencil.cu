@@ -465,6 +465,23 @@ __device__ __noinline__ void stage_give_up(uint64_t* bar, unsigned parity, float
     for (int k = 0; k < ROWS; ++k) rows[k * 32] = make_float4(nan, nan, nan, nan);
 }
 
+// The wait of a residual-driven solve on 64-row regions, without a result to carry: it reports
+// a wait that gave up by itself (*error = 1) and waits once more as long, so that the barrier
+// is armed again behind its copy; the solve's outcome is an error then whatever it computes.
+// One statement, since what the compiler makes of the loop above costs that kernel 1 % (steps
+// of two solves of 512 sweeps, 514 x 514 and 2050 x 2050: 926 and 3270 us against 938 and 3310;
+// with 128-row regions, 1026 x 1026, it is the other way round: 1308 us against 1319).
+__device__ __forceinline__ void stage_wait_or_report(uint64_t* bar, unsigned parity, int* error) {
+    asm volatile(
+        "{\n .reg .pred p;\n .reg .u32 left;\n mov.u32 left, %3;\n"
+        "W%=:\n mbarrier.try_wait.parity.shared::cta.b64 p, [%0], %1;\n @p bra D%=;\n"
+        " sub.u32 left, left, 1;\n setp.ne.u32 p, left, %4;\n @p bra N%=;\n st.volatile.global.u32 [%2], 1;\n"
+        "N%=:\n setp.ne.u32 p, left, 0;\n @p bra W%=;\n"
+        "D%=:\n}\n" ::"r"(tc::smem_u32(bar)),
+        "r"(parity), "l"(error), "n"(2 * kStageWait), "n"(kStageWait)
+        : "memory");
+}
+
 // What a warp carries from tile to tile: the parity of its prefetch and whether a wait for one
 // gave up, and the exchange buffer that the next sweep uses (so that no barrier is needed
 // between tiles).
@@ -483,11 +500,11 @@ struct Carry {
 // for it), and `next` starts the next tile's once it has been read. A warp whose wait gave up
 // fills its staged rows with NaN and prefetches nothing more (its barrier's parity would no
 // longer tell one copy from another), so that this block and all that follow are NaN; the
-// kernel reports it at its end.
+// kernel reports it at its end. error: a residual-driven solve's error word.
 template <int R, int NW, bool DIFF, bool VEC, bool RESID, class Next>
 __device__ __forceinline__ void process_tile(const StencilField& F, int n, int ty, int tx, const float* __restrict__ xin,
                                              float* __restrict__ yout, bool resid, float& rnum, float& rden,
-                                             Carry& carry, unsigned polls, Next&& next) {
+                                             Carry& carry, unsigned polls, int* error, Next&& next) {
     constexpr int RW = kRegionW;
     constexpr unsigned FULL = 0xffffffffu;
     extern __shared__ float4 smem4[];
@@ -545,7 +562,10 @@ __device__ __forceinline__ void process_tile(const StencilField& F, int n, int t
     // columns q of this block and rows i that are interior cells of the grid
     auto int_col = [&](int q) { return t.c0 + q >= 1 && q <= t.ncol - 2; };
     auto int_row = [&](int i) { return t.gyb + i >= 1 && i <= t.nrow - 2; };
-    if (VEC && !carry.gave_up()) {
+    if (RESID && NW <= 8) {
+        stage_wait_or_report(stage_bar<R, NW>(), carry.phase(), error);
+        carry.stage ^= kPhase;
+    } else if (VEC && !carry.gave_up()) {
         if (stage_wait(stage_bar<R, NW>(), carry.phase(), polls)) {
             carry.stage ^= kPhase;
         } else {
@@ -842,7 +862,7 @@ __global__ void __launch_bounds__(32 * NW, (NW <= 8 ? 2 : 1))
         else
             walk.start(L.f[nf], nb - L.f[nf].tile_begin, gridDim.x);
         const StencilField& F = L.f[f];
-        process_tile<kR, NW, DIFF, VEC, false>(F, F.sweeps, ty, tx, F.x, F.y, false, rn, rd, carry, L.polls, [&] {
+        process_tile<kR, NW, DIFF, VEC, false>(F, F.sweeps, ty, tx, F.x, F.y, false, rn, rd, carry, L.polls, nullptr, [&] {
             if (nb < total) prefetch_tile<kR, NW, DIFF>(L.f[nf], walk.ty, walk.col(), &L.f[nf].mx, &L.f[nf].mk);
         });
         b = nb;
@@ -885,7 +905,7 @@ __global__ void __launch_bounds__(32 * NW, (NW <= 8 ? 2 : 1)) stencil_wide_kerne
         else
             walk.start(L.f[nf], nb - L.begin[nf], gridDim.x);
         const StencilField& F = L.f[f];
-        process_tile<kR, NW, DIFF, true, false>(F, F.sweeps, ty, tx, F.x, F.y, false, rn, rd, carry, 0, [&] {
+        process_tile<kR, NW, DIFF, true, false>(F, F.sweeps, ty, tx, F.x, F.y, false, rn, rd, carry, 0, nullptr, [&] {
             if (nb < total) prefetch_tile<kR, NW, DIFF>(L.f[nf], walk.ty, walk.col(), &L.f[nf].mx, &L.f[nf].mk);
         });
         b = nb;
@@ -982,7 +1002,8 @@ __global__ void __launch_bounds__(32 * NW, (NW <= 8 ? 2 : 1))
         for (unsigned t = blockIdx.x; t < ntiles; t += G) {
             const int ty = walk.ty, tx = walk.col();
             walk.next();
-            process_tile<kR, NW, false, true, true>(F, take * F.sweeps, ty, tx, x, P.p[dst], check, rn, rd, carry, 0, [&] {
+            process_tile<kR, NW, false, true, true>(F, take * F.sweeps, ty, tx, x, P.p[dst], check, rn, rd, carry, 0,
+                                                    &P.ctrl->error, [&] {
                 if (t + G < ntiles) prefetch_tile<kR, NW, false>(F, walk.ty, walk.col(), mx, &F.mk);
             });
         }
