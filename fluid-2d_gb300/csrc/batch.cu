@@ -7,7 +7,8 @@
 // all grids: a stencil pass carries the grids' field descriptors in its launch
 // parameters (tiles of all grids concatenated, walked by persistent CTAs; a pass of more
 // fields than the parameter space holds, 70 with their tensor maps, is split into launches of
-// equal field counts), and the advection and gradient stages walk a device table of per-grid jobs (a block -> job map).
+// equal field counts), and the advection and gradient stages walk a device table of per-grid
+// jobs (a block -> job map).
 // The grids are dealt to a few lanes (longest-processing-time first, by cells) and each
 // lane runs its own sequence of launches on its own stream, so one lane's small final
 // wave overlaps another lane's work instead of idling the GPU between sub-steps. The
@@ -53,6 +54,7 @@ struct fs_batch {
     float* slab = nullptr;
     int* flags = nullptr;             // StepFlags
     HostFlags* host_flags = nullptr;  // their copy in page-locked memory
+    int* timed_out = nullptr;         // its word for a wait that gave up, as the device sees it
     cudaStream_t stream = nullptr;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t gexec = nullptr;
@@ -138,7 +140,7 @@ fs_batch::Pass add_pass(fs_batch* b, const std::vector<StencilField>& fl, bool d
         b->h_wide.emplace_back();
         WideLaunch& W = b->h_wide.back();
         std::memset(&W, 0, sizeof(W));
-        W.flags = b->flags;
+        W.timed_out = b->timed_out;
         W.nfields = cnt;
         int tiles = 0;
         for (int i = 0; i < cnt; ++i) {
@@ -438,6 +440,7 @@ int fs_batch_create(const fs_config* cfg, int count, const int* rows, const int*
         fs_batch_destroy(b);
         return rc;
     }
+    b->timed_out = &flags.host->timed_out;
     // lanes: grids dealt longest-first to the lane with the fewest cells so far
     const int nlanes = std::min(kBatchLanes, count);
     b->lanes.resize(nlanes);

@@ -293,7 +293,7 @@ cudaError_t launch_advect_batch(int op, const AdvectJob* jobs, const int* prefix
 // architecture): field f owns the tiles [begin[f], begin[f + 1]) of the launch.
 constexpr int kMaxWideFields = 70;
 struct WideLaunch {
-    int* flags;  // as in StencilLaunch
+    int* timed_out;  // the host's word for a wait that gave up (HostFlags)
     int nfields;
     int begin[kMaxWideFields + 1];
     StencilField f[kMaxWideFields];

@@ -130,7 +130,7 @@ __device__ __forceinline__ float div_by(float x, float b, float y) {
         const float r = __fmaf_rn(-q0, b, x);
         return __fmaf_rn(r, y, q0);
     }
-    return ax == 0.f ? x : ieee_div(x, b);  // out of line: rare, and keeps the epilogue small
+    return ax == 0.f ? x : ieee_div(x, b);  // out of line: rare, and keeps the kernel small
 }
 
 // Where a thread's block meets the domain edge.
@@ -465,12 +465,13 @@ __device__ __noinline__ void stage_give_up(uint64_t* bar, unsigned parity, float
     for (int k = 0; k < ROWS; ++k) rows[k * 32] = make_float4(nan, nan, nan, nan);
 }
 
-// The wait of a residual-driven solve on 64-row regions, without a result to carry: it reports
-// a wait that gave up by itself (*error = 1) and waits once more as long, so that the barrier
-// is armed again behind its copy; the solve's outcome is an error then whatever it computes.
-// One statement, since what the compiler makes of the loop above costs that kernel 1 % (steps
-// of two solves of 512 sweeps, 514 x 514 and 2050 x 2050: 926 and 3270 us against 938 and 3310;
-// with 128-row regions, 1026 x 1026, it is the other way round: 1308 us against 1319).
+// The same wait without a result to carry: it reports a wait that gave up by itself (*error = 1)
+// and waits once more as long, so that the barrier is armed again behind its copy. For kernels
+// whose every result is void once the word is set, batches and solves on 64-row regions. One
+// statement, since the compiler's registers and schedule around the loop above cost those
+// kernels 1 to 2 % (batch of 24 grids of 64 to 512 a side 278 against 275 us a step; steps of
+// two solves of 512 sweeps, 514 x 514 and 2050 x 2050, 938 and 3310 against 926 and 3270;
+// 128-row regions, 1026 x 1026, are the other way round: 1308 against 1319).
 __device__ __forceinline__ void stage_wait_or_report(uint64_t* bar, unsigned parity, int* error) {
     asm volatile(
         "{\n .reg .pred p;\n .reg .u32 left;\n mov.u32 left, %3;\n"
@@ -494,14 +495,14 @@ struct Carry {
 };
 
 // Tile (ty, tx) of one pass: load the region (fusing add_sources or the divergence into the
-// first pass), run n sweeps, store the output tile, then the optional residual
-// partial sums (for residual-driven pressure solves). xin/yout stand in for F.x/F.y so a persistent caller can ping-pong
-// buffers across passes. VEC: the block comes from the prefetch (polls: the bound of the wait
+// first pass), run n sweeps, store the output tile, then the optional residual partial sums (for
+// residual-driven pressure solves). xin/yout stand in for F.x/F.y so a persistent caller can
+// ping-pong buffers across passes. VEC: the block comes from the prefetch (polls: the bound of the wait
 // for it), and `next` starts the next tile's once it has been read. A warp whose wait gave up
 // fills its staged rows with NaN and prefetches nothing more (its barrier's parity would no
 // longer tell one copy from another), so that this block and all that follow are NaN; the
-// kernel reports it at its end. error: a residual-driven solve's error word.
-template <int R, int NW, bool DIFF, bool VEC, bool RESID, class Next>
+// kernel reports it at its end. SELF: the wait reports to `error` by itself instead.
+template <int R, int NW, bool DIFF, bool VEC, bool RESID, bool SELF, class Next>
 __device__ __forceinline__ void process_tile(const StencilField& F, int n, int ty, int tx, const float* __restrict__ xin,
                                              float* __restrict__ yout, bool resid, float& rnum, float& rden,
                                              Carry& carry, unsigned polls, int* error, Next&& next) {
@@ -562,7 +563,7 @@ __device__ __forceinline__ void process_tile(const StencilField& F, int n, int t
     // columns q of this block and rows i that are interior cells of the grid
     auto int_col = [&](int q) { return t.c0 + q >= 1 && q <= t.ncol - 2; };
     auto int_row = [&](int i) { return t.gyb + i >= 1 && i <= t.nrow - 2; };
-    if (RESID && NW <= 8) {
+    if (SELF) {
         stage_wait_or_report(stage_bar<R, NW>(), carry.phase(), error);
         carry.stage ^= kPhase;
     } else if (VEC && !carry.gave_up()) {
@@ -862,7 +863,7 @@ __global__ void __launch_bounds__(32 * NW, (NW <= 8 ? 2 : 1))
         else
             walk.start(L.f[nf], nb - L.f[nf].tile_begin, gridDim.x);
         const StencilField& F = L.f[f];
-        process_tile<kR, NW, DIFF, VEC, false>(F, F.sweeps, ty, tx, F.x, F.y, false, rn, rd, carry, L.polls, nullptr, [&] {
+        process_tile<kR, NW, DIFF, VEC, false, false>(F, F.sweeps, ty, tx, F.x, F.y, false, rn, rd, carry, L.polls, nullptr, [&] {
             if (nb < total) prefetch_tile<kR, NW, DIFF>(L.f[nf], walk.ty, walk.col(), &L.f[nf].mx, &L.f[nf].mk);
         });
         b = nb;
@@ -905,13 +906,12 @@ __global__ void __launch_bounds__(32 * NW, (NW <= 8 ? 2 : 1)) stencil_wide_kerne
         else
             walk.start(L.f[nf], nb - L.begin[nf], gridDim.x);
         const StencilField& F = L.f[f];
-        process_tile<kR, NW, DIFF, true, false>(F, F.sweeps, ty, tx, F.x, F.y, false, rn, rd, carry, 0, nullptr, [&] {
+        process_tile<kR, NW, DIFF, true, false, true>(F, F.sweeps, ty, tx, F.x, F.y, false, rn, rd, carry, 0, L.timed_out, [&] {
             if (nb < total) prefetch_tile<kR, NW, DIFF>(L.f[nf], walk.ty, walk.col(), &L.f[nf].mx, &L.f[nf].mk);
         });
         b = nb;
         f = nf;
     }
-    if (carry.gave_up()) report_timeout(L.flags);
 }
 
 // ---------------------------------------------------------------------------
@@ -920,7 +920,9 @@ __global__ void __launch_bounds__(32 * NW, (NW <= 8 ? 2 : 1)) stencil_wide_kerne
 // at 514 x 514 before the sums, the outcome and the barrier took their present form: sweeps
 // 8,900 (13,900 in an edge tile), load 1,000, store 600-2,400, residual sums 3,300, barrier
 // 6,200, outcome 6,300. 256 sweeps there: 385 us in single passes, 289 in pairs, 230 with
-// short sums and the one-word barrier (1026 x 1026: 472 and 317 us, 2050 x 2050: 874 and 787).
+// short sums and the one-word barrier (1026 x 1026: 472 and 319 us, 2050 x 2050: 874 and 790).
+// What is left there (ncu): the barriers of the sweeps (3.1 of 7.9 cycles a warp spends per
+// instruction at 514 x 514, 4.4 of 11.5 at 1026 x 1026) with issue 25 and 35 % busy.
 
 constexpr unsigned kBarrierSpinLimit = 1u << 24;  // default: ~2 s of polling, then give up
 
@@ -1002,7 +1004,7 @@ __global__ void __launch_bounds__(32 * NW, (NW <= 8 ? 2 : 1))
         for (unsigned t = blockIdx.x; t < ntiles; t += G) {
             const int ty = walk.ty, tx = walk.col();
             walk.next();
-            process_tile<kR, NW, false, true, true>(F, take * F.sweeps, ty, tx, x, P.p[dst], check, rn, rd, carry, 0,
+            process_tile<kR, NW, false, true, true, NW <= 8>(F, take * F.sweeps, ty, tx, x, P.p[dst], check, rn, rd, carry, 0,
                                                     &P.ctrl->error, [&] {
                 if (t + G < ntiles) prefetch_tile<kR, NW, false>(F, walk.ty, walk.col(), mx, &F.mk);
             });

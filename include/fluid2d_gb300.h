@@ -199,8 +199,9 @@ FS_API int fs_sync(fs_solver* s);
  * unprojected and fs_sync / fs_step return FS_ERR_TIMEOUT; the handle stays usable.
  * On such a handle it also bounds the waits for the tiles that a diffusion pass has under way
  * (default, and for every other pass and handle: about 1.4 s). When such a wait runs out, the
- * cells that needed the tile become NaN and the next fs_sync / fs_step / fs_batch_sync returns
- * FS_ERR_TIMEOUT, whatever check_finite is; upload a state before going on.
+ * cells that needed the tile are NaN (in a batch or a solve, any value) and the next fs_sync /
+ * fs_step / fs_batch_sync returns FS_ERR_TIMEOUT, whatever check_finite is; upload a state
+ * before going on.
  * fs_project_noalloc has no call that could report it: there the NaN is all there is.
  * The reference has no bounded waits (it has no grid-wide synchronisation at all). */
 FS_API int fs_set_barrier_poll_limit(fs_solver* s, unsigned polls);
