@@ -291,7 +291,9 @@ dim3 grid_for(int rows, int cols, int per_x, int per_y) {
 // Cells of a column per thread: four give a warp the reads to keep in flight and the splat
 // its sums along the column; small grids then have too few warps to hide a read's latency.
 // Whole steps (15 diffusion, 20 pressure sweeps), us with 1 and with 4: 130 x 130 41.0 and
-// 43.1, 771 x 1283 87.1 and 88.1, 2050 x 2050 259 and 252, 8194 x 8194 3569 and 3436.
+// 43.1, 771 x 1283 87.1 and 88.1, 1154 x 1154 100.7 and 100.2, 1400 x 1400 144.5 and 143.5,
+// 1540 x 1540 160.2 and 159.3, 1700 x 1700 186.4 and 183.7, 2050 x 2050 259 and 252,
+// 8194 x 8194 3569 and 3436.
 bool four_rows(int rows, int cols) { return (long)rows * cols >= 2L << 20; }
 
 }  // namespace

@@ -668,7 +668,7 @@ __global__ void __launch_bounds__(kInfThreads) net_infer32_kernel(const InferArg
         tc::fence_after_sync();
         if (!ok) return;
         const float* bias = A.params + (size_t)li * (kC * kK + kC) + kC * kK;
-        // warp w reads tensor-memory lanes 32*(w%4).. of the tiles T = w/4, w/4 + 2, ...
+        // warp w reads tensor-memory lanes 32*(w%4).. of the tiles T = w/4, w/4 + 4, ...
         for (int T = warp >> 2; T < L.tiles; T += kInfThreads / 128) {
             float v[32];
             tc::tmem_ld_32x32(taddr + ((uint32_t)((warp & 3) * 32) << 16) + T * 32, v);

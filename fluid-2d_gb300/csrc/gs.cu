@@ -32,10 +32,13 @@
 // Grids whose bands all fit one SM's shared memory (up to 141 x 141) run in one CTA per
 // field instead, bands side by side, so that nothing leaves the SM.
 //
-// What bounds it: the latency of a chunk's instructions on the chain of bands, columns and
-// sweeps, and the trips between SMs (2-3 us per band with a CTA per band). At 20/20 sweeps a
-// step takes 0.43 ms at 130 x 130 (1.12 ms with a block barrier per anti-diagonal of one CTA)
-// and 1.61 ms at 800 x 800 (21.0 ms with a grid barrier per diagonal of 64 x 64 tiles).
+// What bounds it: the chain of bands, columns and sweeps, a chunk of eight columns after another,
+// each as long as its slowest warp's instructions (ncu: the largest stall is the barrier behind
+// a chunk, then waits for the own instructions before; schedulers issue in 51 % of the cycles
+// with 24 warps in one CTA, in 27 % with 20), and from band to band the 32 columns of skew and
+// a trip between SMs, 7 us in all. At 20/20 sweeps a step takes 0.41 ms at 130 x 130 (1.12 ms
+// with a block barrier per anti-diagonal of one CTA) and 1.58 ms at 800 x 800 (21.0 ms with a
+// grid barrier per diagonal of 64 x 64 tiles).
 //
 // The splat keeps the host solver's order of additions to every cell: a cell receives
 // its contributions in the raster order of their source cells. Source cells are linked
@@ -62,7 +65,7 @@ constexpr unsigned kGsPolls = 1u << 21;  // default bound of a wait, about 2 s
 
 // One field of a solve. Diffusion: x + dt*src is both the start and the constant term;
 // pressure: the constant term is the divergence of (u, v), the start zero. A later launch
-// of the same solve (more than kMaxSweeps sweeps) starts from `start`.
+// of the same solve (more than kMaxWarps sweeps) starts from `start`.
 struct GsField {
     const float* x;
     const float* src;

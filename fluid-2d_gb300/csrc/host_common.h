@@ -1,4 +1,5 @@
-// Host-side helpers shared by the single-grid and batched drivers: pass planning, the reference's step constants, and CUDA error reporting.
+// Host-side helpers shared by the single-grid and batched drivers: pass planning, the reference's
+// step constants, and CUDA error reporting.
 #pragma once
 
 #include <cuda_runtime.h>

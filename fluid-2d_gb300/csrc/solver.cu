@@ -4,8 +4,9 @@
 // fluid_solver_gpu::solve (mworchel/fluid-2d src/fluid_solver_gpu.cu:222-258) in the
 // same stage order, planned as a short fixed sequence of fused kernels:
 //
-//   diffuse d,u,v  : ceil(Kd/K) stencil passes, all three fields in each launch
-//                    (add_sources fused into the first pass)
+//   diffuse d,u,v  : ceil(Kd/K) stencil passes, all three fields in each launch, or u and v
+//                    with d beside them on the side stream (density_branch_pays); add_sources
+//                    fused into the first pass
 //   advect d       : memset + forward splat + finish (Neumann fill + smoothing)
 //   project        : ceil(Kp/K) stencil passes (divergence fused into the first), then the
 //                    gradient subtract + reflecting fills
@@ -1571,7 +1572,11 @@ int fs_set_barrier_poll_limit(fs_solver* s, unsigned polls) {
 
 // Grids of at least this many cells take the overlapped host step below. On smaller
 // grids the copies are shorter than what the overlap costs (an eager step in place of one
-// graph launch, and the diffusion split into two launches).
+// graph launch, and the diffusion split into two launches). Page-locked grids, 15/20 sweeps, us
+// a call in one piece and overlapped: 1000 x 1000 292 and 294, 1026 x 1026 307 and 303,
+// 1400 x 1400 518 and 492, 2050 x 2050 1017 and 961. Pageable ones, which the copy engine moves
+// more slowly than a kernel does, would do better in one piece for longer: 1026 x 1026 307 and
+// 392, 1400 x 1900 671 and 730, 2050 x 2050 1023 and 1035 (1230 and 1191 at 40/40 sweeps).
 #ifndef FS_OVERLAP_MIN_CELLS
 #define FS_OVERLAP_MIN_CELLS (1L << 20)
 #endif
