@@ -311,13 +311,13 @@ struct WgradArgs {
 };
 
 // The NaN of one row (tap dy, dx and channel ci) of a CTA's partial result, summed once more
-// over the pixels of slots [pbeg, pend) in order.
+// over the pixels of slots [pbeg, pend) in order, until the sum is NaN for good.
 __device__ __noinline__ void wgrad_row_again(const WgradArgs& P, float* out, int dy, int dx, int ci, long pbeg,
                                              long pend) {
     for (int c = 0; c < kC; ++c) {
         if (!isnan(out[c])) continue;
         float acc = 0.f;
-        for (long s = pbeg; s < pend; ++s) {
+        for (long s = pbeg; s < pend && !isnan(acc); ++s) {
             const long y = s / (P.W + 2);
             const int xx = (int)(s - y * (P.W + 2)) - 1;
             if (xx < 0 || xx >= P.W) continue;

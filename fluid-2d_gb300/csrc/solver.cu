@@ -1561,12 +1561,12 @@ int fs_set_barrier_poll_limit(fs_solver* s, unsigned polls) {
     DeviceGuard g(s->device);
     // a device word read by every residual solve at launch, so captured step graphs see it too
     CK(cudaMemcpyAsync(s->flags + 1, &polls, sizeof(unsigned), cudaMemcpyHostToDevice, s->stream));
+    CK(cudaStreamSynchronize(s->stream));
     // the waits for prefetched tiles take it as a launch parameter
     if (s->cfg.pressure_tolerance > 0.f && s->prefetch_polls != polls) {
         s->prefetch_polls = polls;
         destroy_graph(s);
     }
-    CK(cudaStreamSynchronize(s->stream));
     return FS_OK;
 }
 
